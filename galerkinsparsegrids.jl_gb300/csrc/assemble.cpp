@@ -15,6 +15,7 @@
 // cancel exactly.  The 1D operator is built by the reference's route
 // (dlf1d.cpp), so the same sums cancel here.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "sgdg_core.h"
@@ -228,13 +229,19 @@ CSR add_scaled(const std::vector<const CSR*>& As, const std::vector<double>& s) 
     return out;
 }
 
-LineTables line_tables(const DLF1D& op, int levels, bool square) {
+LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune) {
     const int k = op.k;
+    double least = -1.0;  // entries of at most this magnitude are left out
+    if (prune) {
+        double top = 0.0;
+        for (double v : op.val) top = std::max(top, std::fabs(v));
+        least = kPruneRel * top;
+    }
     LineTables T;
     T.k = k;
     T.levels = levels;
     std::vector<int64_t> marker;
-    std::vector<double> acc;
+    std::vector<double> acc, mag;
     std::vector<int32_t> cols;
     for (int lm = 1; lm <= levels; lm++) {
         const int nrb = 1 << (lm - 1), m = nrb * k;
@@ -249,8 +256,10 @@ LineTables line_tables(const DLF1D& op, int levels, bool square) {
                     const int cb = op.colblk[p];
                     if (cb >= nrb) continue;
                     for (int mj = 0; mj < k; mj++) {
+                        const double v = op.val[(size_t)p * k * k + (size_t)md * k + mj];
+                        if (prune && !(std::fabs(v) > least)) continue;
                         lc.push_back(cb * k + mj);
-                        lv.push_back(op.val[(size_t)p * k * k + (size_t)md * k + mj]);
+                        lv.push_back(v);
                     }
                 }
                 lp[rb * k + md + 1] = (int64_t)lc.size();
@@ -266,6 +275,7 @@ LineTables line_tables(const DLF1D& op, int levels, bool square) {
         // row's entries ascending, each times the entries of that row)
         marker.assign(m, -1);
         acc.assign(m, 0.0);
+        mag.assign(m, 0.0);
         const int64_t base = (int64_t)T.col.size();
         T.rowptr.push_back(base);
         for (int r = 0; r < m; r++) {
@@ -278,14 +288,17 @@ LineTables line_tables(const DLF1D& op, int levels, bool square) {
                     if (marker[c] != r) {
                         marker[c] = r;
                         acc[c] = a * lv[q];
+                        mag[c] = std::fabs(a * lv[q]);
                         cols.push_back(c);
                     } else {
                         acc[c] += a * lv[q];
+                        mag[c] += std::fabs(a * lv[q]);
                     }
                 }
             }
             std::sort(cols.begin(), cols.end());
             for (int32_t c : cols) {
+                if (prune && !(std::fabs(acc[c]) > kPruneRel * mag[c])) continue;
                 T.col.push_back(c);
                 T.val.push_back(acc[c]);
             }

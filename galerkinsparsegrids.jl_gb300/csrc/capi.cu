@@ -22,11 +22,14 @@ namespace sgdg {
 cudaError_t launch_csr_spmv(const DevCSR& A, const double* x, double* y, cudaStream_t st);
 cudaError_t mf_bounds_violations(unsigned int* out, bool reset);
 cudaError_t csr_bounds_violations(unsigned int* out, bool reset);
+cudaError_t step_bounds_violations(unsigned int* out, bool reset);
 cudaError_t asm_bounds_violations(unsigned int* out, bool reset);
-cudaError_t launch_csr_rk4_batch(const DevCSR& A, int64_t nb, int64_t bs, const double* uin, double* y, double* acc,
-                                 double* uout, double dt, int stage, cudaStream_t st);
 cudaError_t launch_csr_rk4(const DevCSR& A, const double* uin, double* y, double* acc, double* uout, double dt,
-                           int stage, cudaStream_t st);
+                           int stage, int* nonfinite, cudaStream_t st);
+int plain_set_size(const DevCSR& A, int64_t nb);
+cudaError_t launch_plain_steps(const DevCSR& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
+                               double dt, int64_t nsteps, int* nonfinite, cudaStream_t st);
+cudaError_t launch_plain_interleave(const DevCSR& A, int nv, int64_t nb, const double* y, double* u0, cudaStream_t st);
 cudaError_t launch_csr_spmv_multi(const DevCSR& A, int nv, const double* x, int64_t xi, int64_t xs, double* y,
                                   int64_t yi, int64_t ys, cudaStream_t st);
 cudaError_t launch_vlasov_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
@@ -50,6 +53,8 @@ struct sgdg_op {
     std::vector<std::unique_ptr<CSR>> dd;  // D_d, built on demand
     std::unique_ptr<CSR> lap, wave;
     std::map<int, std::unique_ptr<DeviceCSR>> dev;  // plain-form device copies by `which`
+    std::map<int, std::unique_ptr<DeviceCSR>> step_dev;  // without the rounding of zeros (stepping)
+    std::unique_ptr<DeviceAdvection> adv;
     std::map<int, std::unique_ptr<MFEngine>> mf_apply;
     cudaStream_t stream = nullptr;
 
@@ -92,8 +97,32 @@ struct sgdg_op {
                      .first;
         return it->second->d;
     }
+    // The operator the plain evolvers step with: without the entries that hold
+    // only the rounding of a zero (line_tables), which are most of the stored
+    // ones (3D k=3 n=7: 191 entries per row of the Laplacian, 41 of them
+    // nonzero).  They do carry NaN and infinities from one row to another, so
+    // a run that meets one is repeated with the whole operator (plain_run).
+    bool prunes() const { return basis == SGDG_BASIS_HIER && ix.k <= kPruneMaxK; }
+    const DevCSR& stepping(int which) {
+        if (!prunes()) return device(which);
+        auto it = step_dev.find(which);
+        if (it == step_dev.end())
+            it = step_dev.emplace(which, gpu_operator(ix, *dlf, which, stream, 0, true)).first;
+        return it->second->d;
+    }
+    // the whole operator, the pruned one making room for it where there is none
+    const DevCSR& whole(int which) {
+        try {
+            return device(which);
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET || step_dev.erase(which) == 0) throw;
+        }
+        return device(which);
+    }
     ~sgdg_op() {
         dev.clear();
+        step_dev.clear();
+        adv.reset();
         mf_apply.clear();
         if (stream) cudaStreamDestroy(stream);
     }
@@ -197,6 +226,47 @@ struct sgdg_vlasov {
         if (e == cudaSuccess) e = launch_csr_spmv(dT[2]->d, c.as<double>(), z.as<double>(), stream);
         return e;
     }
+};
+
+// RK4 steps of the plain form: `per` steps captured as a graph (launches inside
+// it are programmatic dependents, so one comes up while the one before it
+// runs) and replayed, what is left over launched as it is.
+class StepGraph {
+   public:
+    static constexpr int64_t kPer = 8;
+    StepGraph() = default;
+    StepGraph(const StepGraph&) = delete;
+    StepGraph& operator=(const StepGraph&) = delete;
+    ~StepGraph() {
+        if (exec_) cudaGraphExecDestroy(exec_);
+    }
+    // launches nsteps steps on st (never the legacy stream), steps(n) launching n of them
+    template <class Steps>
+    void run(int64_t nsteps, cudaStream_t st, Steps&& steps) {
+        if (nsteps >= kPer && !exec_) capture(st, steps);
+        for (; nsteps >= kPer; nsteps -= kPer) CK(cudaGraphLaunch(exec_, st));
+        CK(steps(nsteps));
+    }
+
+   private:
+    template <class Steps>
+    void capture(cudaStream_t st, Steps&& steps) {
+        cudaGraph_t g = nullptr;
+        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        const cudaError_t e = steps(kPer);
+        const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+        if (e != cudaSuccess || e2 != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            throw Error(SGDG_ECUDA, std::string("capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
+        }
+        const cudaError_t e3 = cudaGraphInstantiate(&exec_, g, 0);
+        cudaGraphDestroy(g);
+        if (e3 != cudaSuccess) {
+            exec_ = nullptr;
+            throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
+        }
+    }
+    cudaGraphExec_t exec_ = nullptr;
 };
 
 struct sgdg_batch {
@@ -495,90 +565,136 @@ static std::vector<int64_t> out_steps(int64_t nsteps, int nout) {
     return s;
 }
 
-static void plain_evolve(sgdg_op* op, int which_or_adv, const DeviceCSR* Aadv, const double* y0, int64_t len,
-                         double t0, double t1, int64_t nsteps, int nout, double* times, double* states) {
-    cudaStream_t st = op_stream(op);
-    const DevCSR* A = Aadv ? &Aadv->d : &op->device(which_or_adv);
-    DevBuf y(sizeof(double) * len), acc(sizeof(double) * len), u0(sizeof(double) * len), u1(sizeof(double) * len);
-    CK(cudaMemcpyAsync(y.p, y0, sizeof(double) * len, cudaMemcpyHostToDevice, st));
+// One evolution y' = A y from host to host; returns whether a stage result
+// was not finite.
+static bool plain_run(const DevCSR& A, const double* y0, int64_t len, double t0, double t1, int64_t nsteps, int nout,
+                      double* times, double* states, cudaStream_t st) {
+    const size_t b = sizeof(double) * (size_t)len;
+    DevBuf work(4 * b + sizeof(int));
+    double* y = work.as<double>();
+    double *acc = y + len, *u0 = y + 2 * len, *u1 = y + 3 * len;
+    int* flag = reinterpret_cast<int*>(y + 4 * len);
+    CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    CK(cudaMemcpyAsync(y, y0, b, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
-    // one RK4 step as a graph
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = launch_csr_rk4(*A, y.as<double>(), y.as<double>(), acc.as<double>(), u0.as<double>(), dt, 1, st);
-    if (e == cudaSuccess)
-        e = launch_csr_rk4(*A, u0.as<double>(), y.as<double>(), acc.as<double>(), u1.as<double>(), dt, 2, st);
-    if (e == cudaSuccess)
-        e = launch_csr_rk4(*A, u1.as<double>(), y.as<double>(), acc.as<double>(), u0.as<double>(), dt, 3, st);
-    if (e == cudaSuccess)
-        e = launch_csr_rk4(*A, u0.as<double>(), y.as<double>(), acc.as<double>(), u1.as<double>(), dt, 4, st);
-    cudaError_t e2 = cudaStreamEndCapture(st, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        throw Error(SGDG_ECUDA, std::string("capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
-    }
-    cudaError_t e3 = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (e3 != cudaSuccess) throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
-    auto steps = out_steps(nsteps, nout);
+    const auto steps = out_steps(nsteps, nout);
+    StepGraph graph;
     int64_t done = 0;
-    cudaError_t err = cudaSuccess;
-    for (int i = 0; i < nout && err == cudaSuccess; i++) {
-        for (; done < steps[i] && err == cudaSuccess; done++) err = cudaGraphLaunch(ge, st);
-        if (err == cudaSuccess)
-            err = cudaMemcpyAsync(states + (size_t)i * len, y.p, sizeof(double) * len, cudaMemcpyDeviceToHost, st);
+    int bad = 0;
+    for (int i = 0; i < nout; i++) {
+        graph.run(steps[i] - done, st, [&](int64_t n) { return launch_plain_steps(A, 1, 1, y, acc, u0, u1, dt, n, flag, st); });
+        done = steps[i];
+        CK(cudaMemcpyAsync(states + (size_t)i * len, y, b, cudaMemcpyDeviceToHost, st));
         if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
     }
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-    cudaGraphExecDestroy(ge);
-    if (err != cudaSuccess) throw Error(SGDG_ECUDA, std::string("evolve: ") + cudaGetErrorString(err));
+    CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return bad != 0;
 }
 
+// The wave (a = null) or advection with velocity a, stepped with the pruned
+// operator; again with the whole one if a stage was not finite.
+static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t len, double t0, double t1,
+                         int64_t nsteps, int nout, double* times, double* states) {
+    cudaStream_t st = op_stream(op);
+    std::vector<double> s;  // -sum_d a_d D_d
+    for (int d = 0; a && d < op->ix.D; d++) s.push_back(-a[d]);
+    if (op->prunes()) {
+        const DevCSR* A = nullptr;
+        if (a) {
+            if (!op->adv) op->adv = gpu_advection(op->ix, *op->dlf, st);
+            CK(op->adv->scale(op->ix.D, s.data(), st));
+            A = &op->adv->A.d;
+        } else {
+            A = &op->stepping(SGDG_OP_WAVE_RHS);
+        }
+        if (!plain_run(*A, y0, len, t0, t1, nsteps, nout, times, states, st)) return;
+    }
+    if (a) {
+        op->adv.reset();
+        // assembled on the GPU (the same entries as add_scaled)
+        const auto A = gpu_scaled_sum(op->ix, *op->dlf, s.data(), st);
+        plain_run(A->d, y0, len, t0, t1, nsteps, nout, times, states, st);
+    } else {
+        plain_run(op->whole(SGDG_OP_WAVE_RHS), y0, len, t0, t1, nsteps, nout, times, states, st);
+    }
+}
+
+// The scratch of nsteps RK4 steps of nb solves sharing A.
+struct PlainScratch {
+    DevBuf acc, u0, u1, flag;
+    int nv;
+    PlainScratch(const DevCSR& A, int64_t nb, int nv_) : flag(sizeof(int)), nv(nv_) {
+        const size_t b = sizeof(double) * (size_t)((nb + nv - 1) / nv * nv * A.m);
+        acc.alloc(b);
+        u0.alloc(b);
+        u1.alloc(b);
+    }
+    // returns whether a stage result was not finite; waits for the steps
+    bool run(const DevCSR& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
+        int bad = 0;
+        StepGraph graph;
+        CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
+        CK(launch_plain_interleave(A, nv, nb, y, u0.as<double>(), st));
+        graph.run(nsteps, st, [&](int64_t n) {
+            return launch_plain_steps(A, nv, nb, y, acc.as<double>(), u0.as<double>(), u1.as<double>(), dt, n,
+                                      flag.as<int>(), st);
+        });
+        CK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        return bad != 0;
+    }
+};
+
 // nsteps plain FP64 RK4 steps of nsolves solves y' = A y sharing operator
-// `which`, states device-resident one after another; one RK4 step (four
-// batched stage launches) is captured as a graph and replayed.
+// `which`, states device-resident one after another.  The pruned operator
+// needs the states of the call's start beside the scratch vectors, to repeat
+// the steps with the whole one if a stage was not finite; without room for
+// them, or for sets padded to whole ones, the whole operator steps the solves
+// one by one from the start.
 static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y, double dt, int64_t nsteps,
                               cudaStream_t st) {
-    const DevCSR& A = op->device(which);
-    const int64_t len = A.m, total = nsolves * len;
-    DevBuf acc(sizeof(double) * total), u0(sizeof(double) * total), u1(sizeof(double) * total);
+    struct Own {  // work is captured and overlapped on a stream of its own where the caller gives none
+        cudaStream_t s = nullptr;
+        ~Own() {
+            if (s) cudaStreamDestroy(s);
+        }
+    } own;
     cudaStream_t cs = st;
-    cudaStream_t own = nullptr;
-    if (cs == nullptr) {  // graphs cannot be captured on the legacy stream
-        CK(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
-        cs = own;
+    if (cs == nullptr) {
+        CK(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+        cs = own.s;
         CK(cudaStreamSynchronize(nullptr));
     }
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
-    CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    double* a = acc.as<double>();
-    double* p0 = u0.as<double>();
-    double* p1 = u1.as<double>();
-    cudaError_t e = launch_csr_rk4_batch(A, nsolves, len, y, y, a, p0, dt, 1, cs);
-    if (e == cudaSuccess) e = launch_csr_rk4_batch(A, nsolves, len, p0, y, a, p1, dt, 2, cs);
-    if (e == cudaSuccess) e = launch_csr_rk4_batch(A, nsolves, len, p1, y, a, p0, dt, 3, cs);
-    if (e == cudaSuccess) e = launch_csr_rk4_batch(A, nsolves, len, p0, y, a, p1, dt, 4, cs);
-    cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        if (own) cudaStreamDestroy(own);
-        throw Error(SGDG_ECUDA, std::string("capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
+    std::unique_ptr<PlainScratch> work;
+    DevBuf keep;
+    const DevCSR* A = nullptr;
+    if (op->prunes()) {
+        try {
+            A = &op->stepping(which);
+            work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));
+            keep.alloc(sizeof(double) * (size_t)(nsolves * A->m));
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET) throw;
+            work.reset();
+            op->step_dev.erase(which);
+        }
     }
-    cudaError_t e3 = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (e3 != cudaSuccess) {
-        if (own) cudaStreamDestroy(own);
-        throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
+    if (keep.p) {
+        CK(cudaMemcpyAsync(keep.p, y, keep.bytes, cudaMemcpyDeviceToDevice, cs));
+        if (!work->run(*A, nsolves, y, dt, nsteps, cs)) return;
+        CK(cudaMemcpyAsync(y, keep.p, keep.bytes, cudaMemcpyDeviceToDevice, cs));
+        CK(cudaStreamSynchronize(cs));
+        work.reset();
+        keep.release();
     }
-    cudaError_t err = cudaSuccess;
-    for (int64_t i = 0; i < nsteps && err == cudaSuccess; i++) err = cudaGraphLaunch(ge, cs);
-    // the scratch vectors are freed on return: wait for the steps
-    if (err == cudaSuccess) err = cudaStreamSynchronize(cs);
-    cudaGraphExecDestroy(ge);
-    if (own) cudaStreamDestroy(own);
-    if (err != cudaSuccess) throw Error(SGDG_ECUDA, std::string("plain batch: ") + cudaGetErrorString(err));
+    A = &op->whole(which);
+    try {
+        work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));
+    } catch (const Error&) {
+        work.reset(new PlainScratch(*A, nsolves, 1));
+    }
+    work->run(*A, nsolves, y, dt, nsteps, cs);
 }
 
 static void mf_evolve(sgdg_op* op, int kind, const double* a, const double* y0, int64_t len, double t0, double t1,
@@ -638,7 +754,7 @@ int sgdg_debug_bounds(int* checked, int64_t* violations, int reset) {
 #endif
     require_gpu();
     unsigned int v = 0;
-    for (auto f : {mf_bounds_violations, csr_bounds_violations, asm_bounds_violations}) {
+    for (auto f : {mf_bounds_violations, csr_bounds_violations, step_bounds_violations, asm_bounds_violations}) {
         CK(f(&v, reset != 0));
         *violations += v;
     }
@@ -658,7 +774,7 @@ int sgdg_wave_evolve(sgdg_op* op, const double* f0, const double* v0, double t0,
     std::memcpy(y0.data(), f0, sizeof(double) * N);
     std::memcpy(y0.data() + N, v0, sizeof(double) * N);
     if (method == SGDG_METHOD_PLAIN)
-        plain_evolve(op, SGDG_OP_WAVE_RHS, nullptr, y0.data(), 2 * N, t0, t1, nsteps, nout, times, states);
+        plain_evolve(op, nullptr, y0.data(), 2 * N, t0, t1, nsteps, nout, times, states);
     else if (method == SGDG_METHOD_MATFREE)
         mf_evolve(op, MF_KIND_WAVE, nullptr, y0.data(), 2 * N, t0, t1, nsteps, nout, times, states);
     else
@@ -677,11 +793,7 @@ int sgdg_advect_evolve(sgdg_op* op, const double* a, const double* f0, double t0
     if (op->basis != SGDG_BASIS_HIER) throw Error(SGDG_EUNSUPPORTED, "advection is hierarchical only");
     const int64_t N = op->ix.N;
     if (method == SGDG_METHOD_PLAIN) {
-        // -sum_d a_d D_d, assembled on the GPU (the same entries as add_scaled)
-        std::vector<double> s;
-        for (int d = 1; d <= op->ix.D; d++) s.push_back(-a[d - 1]);
-        auto A = gpu_scaled_sum(op->ix, *op->dlf, s.data(), op_stream(op));
-        plain_evolve(op, 0, A.get(), f0, N, t0, t1, nsteps, nout, times, states);
+        plain_evolve(op, a, f0, N, t0, t1, nsteps, nout, times, states);
     } else if (method == SGDG_METHOD_MATFREE) {
         mf_evolve(op, MF_KIND_ADVECT, a, f0, N, t0, t1, nsteps, nout, times, states);
     } else {
@@ -915,7 +1027,7 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
         e = v->rhs_points(in[stage - 1]);
         if (e == cudaSuccess)
             e = launch_csr_rk4(v->dT[3]->d, v->z.as<double>(), y.as<double>(), acc.as<double>(), outv[stage - 1], dt,
-                               stage, st);
+                               stage, nullptr, st);
     }
     cudaError_t e2 = cudaStreamEndCapture(st, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {

@@ -21,13 +21,19 @@ struct DeviceCSR {
 constexpr int64_t kCsrSplit = 2048;  // entries a row group sums directly
 
 // bin of a row of L <= kCsrSplit entries: the fewest lanes 2^b (up to 32)
-// that give each lane at most `per_lane` entries (fewer lanes per row: fewer
-// FP64 additions in the lane reduction, which on GB300 cost as much as the
-// FMAs).  32 entries per lane suit single-vector passes: the 256-solve wave
-// batch steps in 20.1 ms against 26.2 at 16 and 31.8 at 8 (its rows hold ~96
-// entries); the nodal transforms, passed over four vectors at once, keep 8
-// (the Vlasov plain step 2.60 ms against 2.66 at 16 and 2.67 at 32).
-constexpr int kCsrLaneEntries = 32;
+// that give each lane at most `per_lane` entries.  Fewer lanes per row mean
+// fewer FP64 additions in the lane reduction, which on GB300 cost as much as
+// the FMAs; more lanes mean shorter chains, for operators too small to fill
+// the GPU.  us per RK4 step at 4, 8, 16 and 32 entries per lane: 2D wave k=3
+// n=5 (31 K entries) 8.9, 12.0, 17.2, 29.0; 4D advection k=2 n=6 (533 K) 24.4,
+// 21.2, 25.2, 34.3; 3D wave k=3 n=7 (1.9 M) 60.0, 47.8, 46.9, 59.0, and 48 of
+// them sharing it 1446, 1096, 939, 948.  The whole Laplacian of that grid
+// (8.8 M) is applied in 33 us at 16 and 28.5 us at 32.  The nodal transforms,
+// passed over four vectors at once, keep 8 (the Vlasov plain step 2.60 ms
+// against 2.66 at 16 and 2.67 at 32).
+inline int csr_lane_entries(int64_t nnz) {
+    return nnz < (128 << 10) ? 4 : nnz < (1 << 20) ? 8 : nnz < (4 << 20) ? 16 : 32;
+}
 constexpr int kCsrLaneEntriesMulti = 8;
 inline int csr_bin(int64_t L, int per_lane) {
     int b = 0;
@@ -38,8 +44,9 @@ inline int csr_bin(int64_t L, int per_lane) {
 // Fills D.d from D's buffers (already holding rowptr, col, val for m rows)
 // and builds the long-row segments from the host copy of the row pointers.
 inline void finish_device_csr(DeviceCSR& D, const std::vector<int64_t>& rowptr, int64_t m, cudaStream_t st,
-                              int per_lane = kCsrLaneEntries) {
+                              int per_lane = 0) {
     const int64_t nnz = rowptr[m];
+    if (per_lane == 0) per_lane = csr_lane_entries(nnz);
     D.d.m = m;
     D.d.nnz = nnz;
     D.d.rowptr = D.rowptr.as<int64_t>();
@@ -115,9 +122,19 @@ inline std::unique_ptr<DeviceCSR> to_device(const CSR& A, cudaStream_t st) {
 
 // The plain-form operators assembled on the GPU (gpu_assemble.cu): which =
 // 1..D for D_d, SGDG_OP_LAPLACIAN, SGDG_OP_WAVE_RHS; the same stored entries
-// and values as the host assembly (assemble.cpp).
+// and values as the host assembly (assemble.cpp).  prune: without the entries
+// that hold only the rounding of a zero (line_tables); for k <= kPruneMaxK.
 std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
-                                        int per_lane = kCsrLaneEntries);
+                                        int per_lane = 0, bool prune = false);
+// The D_d of a grid one after another in each row (pruned as above), the
+// dimension of every entry and the unscaled values kept: scale() makes the
+// values those of sum_d s[d] D_d.
+struct DeviceAdvection {
+    DeviceCSR A;
+    DevBuf base, dim;
+    cudaError_t scale(int D, const double* s, cudaStream_t st);
+};
+std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1D& dlf, cudaStream_t st);
 // sum_d s[d] D_d over the union of patterns (the plain advection operator)
 std::unique_ptr<DeviceCSR> gpu_scaled_sum(const SparseIndex& ix, const DLF1D& dlf, const double* s, cudaStream_t st);
 // The D-dim restricted Kronecker product of the 1D transform T1 (the same

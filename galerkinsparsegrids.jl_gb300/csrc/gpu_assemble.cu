@@ -97,6 +97,52 @@ __global__ void k_line_fill(LineArgs A, const int64_t* __restrict__ rowptr, int3
     }
 }
 
+// the rows of several dimensions one after another: row i's next entries go to
+// cursor[i], which moves on (each dimension's pencils hold every row once)
+__global__ void k_line_count_add(LineArgs A, int32_t* rowlen) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= A.N) return;
+    int P, row, a, b;
+    locate(A, e, P, row, a, b);
+    const PencilDesc pd = A.pen[P];
+    const int2 ri = A.rows[pd.roff + row];
+    const int64_t* rp = A.trowptr + A.troff[pd.lmax - 1];
+    const int64_t i = ri.x + a + ((int64_t)b << ri.y);
+    if (SGDG_IN(i, A.N)) rowlen[i] += (int32_t)(rp[row + 1] - rp[row]);
+}
+
+__global__ void k_line_append(LineArgs A, int64_t* __restrict__ cursor, const int64_t* __restrict__ rowptr,
+                              int32_t* __restrict__ col, double* __restrict__ val, uint8_t* __restrict__ dim, int d) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= A.N) return;
+    int P, row, a, b;
+    locate(A, e, P, row, a, b);
+    const PencilDesc pd = A.pen[P];
+    const int2 ri = A.rows[pd.roff + row];
+    const int64_t* rp = A.trowptr + A.troff[pd.lmax - 1];
+    const int64_t i = ri.x + a + ((int64_t)b << ri.y);
+    if (!SGDG_IN(i, A.N)) return;
+    int64_t w = cursor[i];
+    for (int64_t t = rp[row]; t < rp[row + 1]; t++, w++) {
+        const int2 rq = A.rows[pd.roff + A.tcol[t]];
+        const int64_t c = rq.x + a + ((int64_t)b << rq.y);
+        if (!SGDG_IN(w - rowptr[i], rowptr[i + 1] - rowptr[i]) || !SGDG_IN(c, A.N)) continue;
+        col[w] = (int32_t)c;
+        val[w] = A.tval[t];
+        dim[w] = (uint8_t)d;
+    }
+    cursor[i] = w;
+}
+
+struct Factors {
+    double s[kDMax];
+};
+__global__ void k_scale_entries(const double* __restrict__ base, const uint8_t* __restrict__ dim, Factors f, int64_t nnz,
+                                double* __restrict__ val) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x)
+        val[p] = f.s[dim[p]] * base[p];
+}
+
 constexpr int kSumMax = 8;
 struct SumArgs {
     int nt;
@@ -651,19 +697,19 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
 SGDG_BOUNDS_READER(asm_bounds_violations)
 
 std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
-                                        int per_lane) {
+                                        int per_lane, bool prune) {
     require_gpu();
     const int D = ix.D;
     std::vector<int64_t> rp;
     if (which >= 1 && which <= D) {
-        const LineTables T = line_tables(dlf, dlf.n + 1, false);
+        const LineTables T = line_tables(dlf, dlf.n + 1, false, prune);
         auto A = line_operator(ix, T, which - 1, st, rp);
         finish_device_csr(*A, rp, ix.N, st, per_lane);
         return A;
     }
     if (which != SGDG_OP_LAPLACIAN && which != SGDG_OP_WAVE_RHS)
         throw Error(SGDG_EINVAL, "operator selector must be 1..D, 0 (laplacian) or -1 (wave RHS)");
-    const LineTables T = line_tables(dlf, dlf.n + 1, true);
+    const LineTables T = line_tables(dlf, dlf.n + 1, true, prune);
     std::vector<std::unique_ptr<DeviceCSR>> sq;
     std::vector<const DeviceCSR*> terms;
     for (int d = 0; d < D; d++) {
@@ -692,6 +738,46 @@ std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf,
     CK(cudaStreamSynchronize(st));
     finish_device_csr(*W, wp, 2 * N, st);
     return W;
+}
+
+std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1D& dlf, cudaStream_t st) {
+    require_gpu();
+    const LineTables T = line_tables(dlf, dlf.n + 1, false, true);
+    std::vector<LineSetup> S(ix.D);
+    DevBuf rowlen(sizeof(int32_t) * (size_t)ix.N);
+    CK(cudaMemsetAsync(rowlen.p, 0, sizeof(int32_t) * (size_t)ix.N, st));
+    for (int d = 0; d < ix.D; d++) {
+        setup_line(S[d], ix, T, d, st);
+        k_line_count_add<<<grid_for(ix.N), 256, 0, st>>>(S[d].args, rowlen.as<int32_t>());
+        CK(cudaGetLastError());
+    }
+    const std::vector<int64_t> rp = scan_rows(rowlen, ix.N, st);
+    auto R = std::make_unique<DeviceAdvection>();
+    DeviceCSR& A = R->A;
+    const size_t nnz = (size_t)rp[ix.N];
+    A.rowptr = upload(rp, st);
+    A.col.alloc(sizeof(int32_t) * nnz);
+    A.val.alloc(sizeof(double) * nnz);
+    R->base.alloc(sizeof(double) * nnz);
+    R->dim.alloc(nnz);
+    DevBuf cursor = upload(rp, st);
+    for (int d = 0; d < ix.D; d++) {
+        k_line_append<<<grid_for(ix.N), 256, 0, st>>>(S[d].args, cursor.as<int64_t>(), A.rowptr.as<int64_t>(),
+                                                      A.col.as<int32_t>(), R->base.as<double>(), R->dim.as<uint8_t>(), d);
+        CK(cudaGetLastError());
+    }
+    finish_device_csr(A, rp, ix.N, st);
+    CK(cudaStreamSynchronize(st));  // S's tables and the cursor are freed on return
+    return R;
+}
+
+cudaError_t DeviceAdvection::scale(int D, const double* s, cudaStream_t st) {
+    Factors f{};
+    for (int d = 0; d < D; d++) f.s[d] = s[d];
+    if (A.d.nnz > 0)
+        k_scale_entries<<<std::min(grid_for(A.d.nnz), 4096), 256, 0, st>>>(base.as<double>(), dim.as<uint8_t>(), f, A.d.nnz,
+                                                                          A.val.as<double>());
+    return cudaGetLastError();
 }
 
 std::unique_ptr<DeviceCSR> gpu_scaled_sum(const SparseIndex& ix, const DLF1D& dlf, const double* s, cudaStream_t st) {

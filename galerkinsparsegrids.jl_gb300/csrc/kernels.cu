@@ -1,8 +1,8 @@
 // kernels.cu -- the plain form and small helpers.
 //
 //  * k_csr: FP64 CSR mat-vec (the closure body *(RHS, x) of src/pdes.jl:63)
-//    over NV vectors in one pass over A, or with NV = 1 fused with the
-//    classical RK4 stage combination.  Rows are binned by length
+//    over NV vectors in one pass over A (the passes fused with the RK4 stage
+//    update are in csr_step.cu).  Rows are binned by length
 //    (DevCSR.bin_*): a row of bin b gets 2^b lanes with at most eight entries
 //    each (four in flight), so the short and the long rows of one matrix (the
 //    nodal transforms hold both) keep the lanes equally busy and the lane
@@ -22,17 +22,10 @@
 #include <cstdint>
 
 #include "bounds.cuh"
+#include "csr.cuh"
 #include "engine.h"
-#include "rk.cuh"
 
 namespace sgdg {
-
-struct CsrRK {  // stage update of the RK4 epilogue: k = A uin, then rk_stage
-    double* acc;
-    double* uout;
-    double dt, hdt, dt6;
-    int stage;
-};
 
 // 256-bit read-only load (sm_100 and later); p 32-byte aligned
 __device__ __forceinline__ void ld_nc_v4(const double* p, double& a, double& b, double& c, double& d) {
@@ -56,67 +49,6 @@ __device__ __forceinline__ void csr_gather(const double* __restrict__ x, int64_t
     } else {
 #pragma unroll
         for (int j = 0; j < NV; j++) v[j] = __ldg(x + off + j * xs);
-    }
-}
-
-// Sum of s[0..NV) over the VS lanes of a row group.  With NV = 2 or 4 the
-// first steps exchange halves of the vector set instead of every value (a
-// lane keeps the half selected by its lane bit and adds its partner's copy),
-// so a row costs log2(VS) + NV - 2 FP64 additions per lane instead of
-// NV log2(VS); each vector's sum has the pairing, and therefore the value, of
-// the all-lane butterfly.  On return vector j's sum is in s[0] of the lanes
-// whose group index has j in its top bits (csr_owner), or in s[j] of every
-// lane when there was nothing to exchange (NV = 1 or 3, or VS too small).
-template <int VS, int NV>
-__device__ __forceinline__ void csr_reduce(double (&s)[NV], int lane) {
-    if constexpr ((NV == 4 && VS >= 4) || (NV == 2 && VS >= 2)) {
-        constexpr int o1 = VS / 2;
-        const bool up1 = lane & o1;
-        double h[NV / 2];
-#pragma unroll
-        for (int i = 0; i < NV / 2; i++) {
-            const double keep = up1 ? s[NV / 2 + i] : s[i];
-            const double give = up1 ? s[i] : s[NV / 2 + i];
-            h[i] = keep + __shfl_xor_sync(0xffffffffu, give, o1);
-        }
-        double r;
-        int o;
-        if constexpr (NV == 4) {
-            constexpr int o2 = VS / 4;
-            const bool up2 = lane & o2;
-            const double keep = up2 ? h[1] : h[0];
-            const double give = up2 ? h[0] : h[1];
-            r = keep + __shfl_xor_sync(0xffffffffu, give, o2);
-            o = VS / 8;
-        } else {
-            r = h[0];
-            o = VS / 4;
-        }
-        for (; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-        s[0] = r;
-    } else {
-#pragma unroll
-        for (int j = 0; j < NV; j++)
-#pragma unroll
-            for (int o = VS / 2; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
-    }
-}
-
-// Which vector's sum the lane holds after csr_reduce (-1: all of them, in
-// s[j]); only lanes whose low bits are zero store it.
-template <int VS, int NV>
-__device__ __forceinline__ int csr_owner(int lane, bool& stores) {
-    if constexpr ((NV == 4 && VS >= 4) || (NV == 2 && VS >= 2)) {
-        constexpr int per = VS / NV;  // lanes holding one vector's sum
-        stores = lane % per == 0;
-        // vector index: bit VS/2 selects the upper half of the set, then bit VS/4 within it
-        if constexpr (NV == 4)
-            return ((lane & (VS / 2)) ? 2 : 0) + ((lane & (VS / 4)) ? 1 : 0);
-        else
-            return (lane & (VS / 2)) ? 1 : 0;
-    } else {
-        stores = lane == 0;
-        return -1;
     }
 }
 
@@ -167,21 +99,10 @@ __device__ __forceinline__ void csr_row(const DevCSR& A, int64_t row, const doub
     csr_reduce<VS, NV>(s, lane);
 }
 
-__device__ __forceinline__ void csr_rk_update(const CsrRK& rk, int64_t row, double k, double* y) {
-    double yy = y[row], aa = rk.stage == 1 ? 0.0 : rk.acc[row], un;
-    rk_stage(rk.stage, rk.dt, rk.hdt, rk.dt6, k, yy, aa, un);
-    if (rk.stage == 4)
-        y[row] = yy;
-    else {
-        rk.acc[row] = aa;
-        rk.uout[row] = un;
-    }
-}
-
 // the rows of bin `bin`, 2^bin = VS lanes each
-template <int VS, int NV, int W, bool RK>
+template <int VS, int NV, int W>
 __device__ __forceinline__ void csr_bin(const DevCSR& A, int bin, int64_t rb, const double* __restrict__ x, int64_t xi,
-                                        int64_t xs, double* y, int64_t yi, int64_t ys, const CsrRK& rk) {
+                                        int64_t xs, double* y, int64_t yi, int64_t ys) {
     const int64_t t = (rb - A.bin_block[bin]) * blockDim.x + threadIdx.x;
     const int64_t idx = t / VS, first = A.bin_first[bin];
     const int lane = int(t % VS);
@@ -192,9 +113,7 @@ __device__ __forceinline__ void csr_bin(const DevCSR& A, int bin, int64_t rb, co
     bool stores;
     const int owner = csr_owner<VS, NV>(lane, stores);
     if (row >= 0 && stores) {
-        if constexpr (RK)
-            csr_rk_update(rk, row, s[0], y);
-        else if (owner >= 0)
+        if (owner >= 0)
             y[row * yi + owner * ys] = s[0];
         else {
 #pragma unroll
@@ -203,45 +122,19 @@ __device__ __forceinline__ void csr_bin(const DevCSR& A, int bin, int64_t rb, co
     }
 }
 
-// With nb > 1 solves sharing A (RK only; solve s's vectors at s * bs), block
-// b is (row block, solve): the solves go in groups of sg, and within a group
-// the solve index runs fastest, so the group's passes over a row block run
-// side by side and read its matrix entries from L2 while the group's vectors
-// stay there too (A is streamed once per group instead of once per solve).
-template <int NV, int W, bool RK>
+template <int NV, int W>
 __global__ void __launch_bounds__(256) k_csr(DevCSR A, const double* __restrict__ x, int64_t xi, int64_t xs,
-                                             double* y, int64_t yi, int64_t ys, CsrRK rk, int64_t bs, int64_t nb,
-                                             int sg) {
-    int64_t rb = blockIdx.x;
-    if constexpr (RK) {
-        if (nb > 1) {
-            const int64_t nrb = A.bin_block[kCsrBins], b = blockIdx.x, full = nb / sg, fb = full * nrb * sg;
-            int64_t sl;
-            if (b < fb) {
-                const int64_t g = b / (nrb * sg), r = b - g * nrb * sg;
-                rb = r / sg;
-                sl = g * sg + r % sg;
-            } else {
-                const int64_t tail = nb - full * sg, r = b - fb;
-                rb = r / tail;
-                sl = full * sg + r % tail;
-            }
-            const int64_t o = sl * bs;
-            x += o;
-            y += o;
-            rk.acc += o;
-            rk.uout += o;
-        }
-    }
+                                             double* y, int64_t yi, int64_t ys) {
+    const int64_t rb = blockIdx.x;
     int bin = 0;
     while (bin + 1 < kCsrBins && rb >= A.bin_block[bin + 1]) bin++;
     switch (bin) {
-        case 0: csr_bin<1, NV, W, RK>(A, 0, rb, x, xi, xs, y, yi, ys, rk); break;
-        case 1: csr_bin<2, NV, W, RK>(A, 1, rb, x, xi, xs, y, yi, ys, rk); break;
-        case 2: csr_bin<4, NV, W, RK>(A, 2, rb, x, xi, xs, y, yi, ys, rk); break;
-        case 3: csr_bin<8, NV, W, RK>(A, 3, rb, x, xi, xs, y, yi, ys, rk); break;
-        case 4: csr_bin<16, NV, W, RK>(A, 4, rb, x, xi, xs, y, yi, ys, rk); break;
-        default: csr_bin<32, NV, W, RK>(A, 5, rb, x, xi, xs, y, yi, ys, rk); break;
+        case 0: csr_bin<1, NV, W>(A, 0, rb, x, xi, xs, y, yi, ys); break;
+        case 1: csr_bin<2, NV, W>(A, 1, rb, x, xi, xs, y, yi, ys); break;
+        case 2: csr_bin<4, NV, W>(A, 2, rb, x, xi, xs, y, yi, ys); break;
+        case 3: csr_bin<8, NV, W>(A, 3, rb, x, xi, xs, y, yi, ys); break;
+        case 4: csr_bin<16, NV, W>(A, 4, rb, x, xi, xs, y, yi, ys); break;
+        default: csr_bin<32, NV, W>(A, 5, rb, x, xi, xs, y, yi, ys); break;
     }
 }
 
@@ -301,9 +194,8 @@ __global__ void __launch_bounds__(256) k_csr_segments(DevCSR A, const double* __
     }
 }
 
-// one thread per (long row, vector): the row's segment partials in order,
-// then the store or (rk_on, one vector) the RK4 stage update
-__global__ void k_csr_long_rows(DevCSR A, int nv, double* y, int64_t yi, int64_t ys, CsrRK rk, bool rk_on) {
+// one thread per (long row, vector): the row's segment partials in order
+__global__ void k_csr_long_rows(DevCSR A, int nv, double* y, int64_t yi, int64_t ys) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.nlong * nv) return;
     const int64_t i = t % A.nlong;
@@ -312,10 +204,7 @@ __global__ void k_csr_long_rows(DevCSR A, int nv, double* y, int64_t yi, int64_t
     for (int q = A.long_seg[i]; q < A.long_seg[i + 1]; q++) s += A.partial[j * A.nseg + q];
     const int64_t row = A.long_row[i];
     if (!SGDG_IN(row, A.m)) return;
-    if (rk_on)
-        csr_rk_update(rk, row, s, y);
-    else
-        y[row * yi + j * ys] = s;
+    y[row * yi + j * ys] = s;
 }
 
 __global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
@@ -354,19 +243,19 @@ static int grid_for(int64_t threads) {
     return (int)(b > (1LL << 30) ? (1LL << 30) : (b < 1 ? 1 : b));
 }
 
-template <int NV, int W, bool RK>
+template <int NV, int W>
 static void csr_pass(const DevCSR& A, const double* x, int64_t xi, int64_t xs, double* y, int64_t yi, int64_t ys,
-                     const CsrRK& rk, cudaStream_t st) {
+                     cudaStream_t st) {
     if (A.bin_block[kCsrBins] > 0)
-        k_csr<NV, W, RK><<<A.bin_block[kCsrBins], 256, 0, st>>>(A, x, xi, xs, y, yi, ys, rk, 0, 1, 1);
+        k_csr<NV, W><<<A.bin_block[kCsrBins], 256, 0, st>>>(A, x, xi, xs, y, yi, ys);
     if (A.nlong > 0) {
         k_csr_segments<NV, W><<<grid_for(A.nseg * 32), 256, 0, st>>>(A, x, xi, xs);
-        k_csr_long_rows<<<grid_for(A.nlong * NV), 256, 0, st>>>(A, NV, y, yi, ys, rk, RK);
+        k_csr_long_rows<<<grid_for(A.nlong * NV), 256, 0, st>>>(A, NV, y, yi, ys);
     }
 }
 
 cudaError_t launch_csr_spmv(const DevCSR& A, const double* x, double* y, cudaStream_t st) {
-    csr_pass<1, 1, false>(A, x, 1, 0, y, 1, 0, CsrRK{}, st);
+    csr_pass<1, 1>(A, x, 1, 0, y, 1, 0, st);
     return cudaGetLastError();
 }
 
@@ -381,55 +270,20 @@ cudaError_t launch_csr_spmv_multi(const DevCSR& A, int nv, const double* x, int6
         // one load per column for adjacent vectors whose group is aligned at every column
         const uintptr_t a = reinterpret_cast<uintptr_t>(xj);
         const int wide = xs != 1 ? 1 : (w == 4 && xi % 4 == 0 && a % 32 == 0) ? 4 : (w % 2 == 0 && xi % 2 == 0 && a % 16 == 0) ? 2 : 1;
-        const CsrRK none{};
         if (w == 4 && wide == 4)
-            csr_pass<4, 4, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<4, 4>(A, xj, xi, xs, yj, yi, ys, st);
         else if (w == 4 && wide == 2)
-            csr_pass<4, 2, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<4, 2>(A, xj, xi, xs, yj, yi, ys, st);
         else if (w == 4)
-            csr_pass<4, 1, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<4, 1>(A, xj, xi, xs, yj, yi, ys, st);
         else if (w == 3)
-            csr_pass<3, 1, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<3, 1>(A, xj, xi, xs, yj, yi, ys, st);
         else if (w == 2 && wide == 2)
-            csr_pass<2, 2, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<2, 2>(A, xj, xi, xs, yj, yi, ys, st);
         else if (w == 2)
-            csr_pass<2, 1, false>(A, xj, xi, xs, yj, yi, ys, none, st);
+            csr_pass<2, 1>(A, xj, xi, xs, yj, yi, ys, st);
         else
-            csr_pass<1, 1, false>(A, xj, xi, xs, yj, yi, ys, none, st);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_csr_rk4(const DevCSR& A, const double* uin, double* y, double* acc, double* uout, double dt,
-                           int stage, cudaStream_t st) {
-    const CsrRK rk{acc, uout, dt, 0.5 * dt, dt / 6.0, stage};
-    csr_pass<1, 1, true>(A, uin, 1, 0, y, 1, 0, rk, st);
-    return cudaGetLastError();
-}
-
-// solves per group of the batched row kernel: 16 solves of the 3D k=3 n=7 wave
-// (733 KB of state each) keep their vectors in L2 while they share A's rows;
-// 1, 4, 8, 32 and 64 measured 33.0, 32.0, 31.9, 31.8 and 31.8 ms per step of
-// 256 solves against 31.9 (the FP64 additions, not A's bytes, bound the pass)
-constexpr int kPlainSolveGroup = 16;
-
-// One RK4 stage of nb solves that share A, their vectors one after another
-// (solve s at s * bs): one launch of the row kernel over (row block, solve)
-// pairs, the solves in groups that stream A once each; a matrix with long
-// rows (segment partials) takes one pass per solve.
-cudaError_t launch_csr_rk4_batch(const DevCSR& A, int64_t nb, int64_t bs, const double* uin, double* y, double* acc,
-                                 double* uout, double dt, int stage, cudaStream_t st) {
-    const CsrRK rk{acc, uout, dt, 0.5 * dt, dt / 6.0, stage};
-    const int64_t nrb = A.bin_block[kCsrBins];
-    if (A.nlong == 0 && nb * nrb < (int64_t(1) << 31)) {
-        if (nrb > 0 && nb > 0)
-            k_csr<1, 1, true><<<(unsigned)(nrb * nb), 256, 0, st>>>(A, uin, 1, 0, y, 1, 0, rk, bs, nb,
-                                                                   kPlainSolveGroup);
-        return cudaGetLastError();
-    }
-    for (int64_t s = 0; s < nb; s++) {
-        const CsrRK r{acc + s * bs, uout + s * bs, dt, 0.5 * dt, dt / 6.0, stage};
-        csr_pass<1, 1, true>(A, uin + s * bs, 1, 0, y + s * bs, 1, 0, r, st);
+            csr_pass<1, 1>(A, xj, xi, xs, yj, yi, ys, st);
     }
     return cudaGetLastError();
 }

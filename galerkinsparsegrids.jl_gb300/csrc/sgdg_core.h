@@ -205,13 +205,23 @@ void pencil_rows(const Pencil& p, int k, int64_t kD, std::vector<int32_t>& out);
 // its square (accumulated as spgemm_sum does, so the values are the same),
 // as CSR over the line's 1D element index with sorted rows.  Table lm starts
 // at rowptr[roff[lm-1]]; its row pointers index col/val directly.
+// prune: without the entries that hold only the rounding of a zero.  A
+// wavelet has k vanishing moments, so its product with anything that is a
+// polynomial on its support is zero, and the reference's route stores what
+// rounding makes of that: for k <= kPruneMaxK at most 2e-12 of the operator's
+// largest entry, while the others reach 1e-4 of it and more (k = 1..5,
+// n = 2..10).  The bound is 1e-10, and for the square 1e-10 of the sum of the
+// magnitudes of an entry's terms (rounding leaves at most 1e-11 of it, other
+// entries 8e-4 and more).
+constexpr int kPruneMaxK = 5;
+constexpr double kPruneRel = 1e-10;
 struct LineTables {
     int k = 0, levels = 0;
     std::vector<int64_t> roff, rowptr;
     std::vector<int32_t> col;
     std::vector<double> val;
 };
-LineTables line_tables(const DLF1D& op, int levels, bool square);
+LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune = false);
 
 void set_error(const std::string& msg);
 }  // namespace sgdg

@@ -1,0 +1,133 @@
+"""Stepping of the plain form: operators without the entries that hold only
+the rounding of a zero, several solves per row, short and long rows."""
+import numpy as np
+import pytest
+
+
+def rk4(A, y, dt, nsteps):
+    for _ in range(nsteps):
+        k1 = A @ y
+        k2 = A @ (y + 0.5 * dt * k1)
+        k3 = A @ (y + 0.5 * dt * k2)
+        y = y + dt / 6 * (k1 + 2 * k2 + 2 * k3 + A @ (y + dt * k3))
+    return y
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("n", [2, 4, 6])
+def test_rounding_of_zeros_is_far_below_the_other_entries(sgdg, k, n):
+    # the bound 1e-10 lies in a gap of the 1D operator and of the squares of
+    # its leading blocks: at least a factor of 5 above what is dropped and
+    # 1e5 below what is kept (rounding at k = 5 reaches 2e-12 and 1e-11)
+    A = sgdg.periodic_DLF_matrix(k, n).toarray()
+    rel = np.abs(A) / np.abs(A).max()
+    assert not np.any((rel > 2e-11) & (rel < 1e-5))
+    B = np.where(rel > 1e-10, A, 0.0)
+    for levels in range(1, n + 2):
+        b = B[:k << (levels - 1), :k << (levels - 1)]
+        sums, terms = np.abs(b @ b), np.abs(b) @ np.abs(b)
+        rel2 = sums[terms > 0] / terms[terms > 0]
+        assert not np.any((rel2 > 2e-11) & (rel2 < 1e-5))
+
+
+SHAPES = [(1, 1, 2, "sparse"), (1, 5, 8, "sparse"), (2, 1, 4, "sparse"), (2, 4, 3, "full"), (3, 3, 4, "sparse"),
+          (2, 6, 3, "sparse"), (1, 8, 7, "sparse"), (4, 2, 3, "sparse")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,k,n,scheme", SHAPES)
+def test_evolvers_against_the_whole_operator(sgdg, D, k, n, scheme):
+    # 8-step graphs and what is left over of them (1, 7, 8, 17 steps); per step
+    # a result is off by a few roundings of dt |A| |y|, plus the dropped
+    # entries (2e-12 of the largest): 1e-10 of the state covers 17 steps at
+    # dt |A| <= 1
+    op = sgdg.SparseGridOperator(D, k, n, scheme)
+    rng = np.random.default_rng(D * 100 + k * 10 + n)
+    N = op.N
+    a = rng.uniform(-1, 1, D)
+    G = sum(-a[d] * op.csr(d + 1) for d in range(D))
+    W = op.csr(-1)
+    for A, y, evolve in ((W, rng.standard_normal(2 * N), "wave"), (G, rng.standard_normal(N), "advect")):
+        dt = 1.0 / max(np.abs(A).sum(1).max(), 1e-3) if evolve == "advect" else \
+            1.0 / np.sqrt(max(np.abs(A).sum(1).max(), 1e-3))
+        for steps in (1, 7, 8, 17):
+            ref = rk4(A, y, dt, steps)
+            if evolve == "wave":
+                _, st = sgdg.wave_evolve(D, k, n, y[:N], y[N:], 0.0, steps * dt, nsteps=steps, scheme=scheme, op=op)
+            else:
+                _, st = sgdg.advect_evolve(D, k, n, a, y, 0.0, steps * dt, nsteps=steps, scheme=scheme, op=op)
+            assert np.linalg.norm(st[-1] - ref) <= 1e-10 * np.linalg.norm(ref), (evolve, steps)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,k,n", [(2, 3, 4), (1, 8, 9)])
+@pytest.mark.parametrize("solves", [1, 2, 3, 4, 5, 18])
+def test_solves_of_a_set_equal_their_own_evolution(sgdg, D, k, n, solves):
+    # sets of 1, 2 and 4 with a remainder, and (1D k=8 n=9, rows of 4096
+    # entries) rows in segments; bit for bit
+    import torch
+    op = sgdg.SparseGridOperator(D, k, n)
+    N, dt, steps = op.N, 1e-6, 3
+    y = np.random.default_rng(solves).standard_normal((solves, 2 * N))
+    dev = torch.tensor(y, device="cuda")
+    op.plain_steps_device(dev.data_ptr(), solves, dt, steps)
+    got = dev.cpu().numpy()
+    for i in range(solves):
+        t1 = steps * dt
+        _, st = sgdg.wave_evolve(D, k, n, y[i, :N], y[i, N:], 0.0, t1, nsteps=steps, op=op)
+        assert t1 / steps != dt or np.array_equal(got[i], st[-1]), i
+        assert np.allclose(got[i], st[-1], rtol=0, atol=1e-12 * np.abs(st[-1]).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where,value", [(0, np.nan), (-1, np.inf), (7, -np.inf), (None, 1e306)])
+def test_what_is_not_finite_spreads_as_the_whole_operator_spreads_it(sgdg, where, value):
+    import torch
+    D, k, n, dt = 2, 3, 4, 1e-2
+    op = sgdg.SparseGridOperator(D, k, n)
+    N = op.N
+    rng = np.random.default_rng(3)
+    y = rng.standard_normal(2 * N)
+    if where is None:
+        y *= value
+    else:
+        y[where] = value
+    a = rng.uniform(-1, 1, D)
+    G = sum(-a[d] * op.csr(d + 1) for d in range(D))
+    fine = rng.standard_normal(2 * N)
+    with np.errstate(all="ignore"):
+        ref = rk4(op.csr(-1), y, dt, 2)
+        ref_a = rk4(G, y[:N], dt, 1)
+    _, st = sgdg.wave_evolve(D, k, n, y[:N], y[N:], 0.0, 2 * dt, nsteps=2, op=op)
+    assert np.array_equal(np.isfinite(st[-1]), np.isfinite(ref))
+    _, st = sgdg.advect_evolve(D, k, n, a, y[:N], 0.0, dt, nsteps=1, op=op)
+    assert np.array_equal(np.isfinite(st[-1]), np.isfinite(ref_a))
+    dev = torch.tensor(np.concatenate([y, fine]), device="cuda")
+    op.plain_steps_device(dev.data_ptr(), 2, dt, 2)
+    got = dev.cpu().numpy().reshape(2, -1)
+    assert np.array_equal(np.isfinite(got[0]), np.isfinite(ref)) and np.all(np.isfinite(got[1]))
+
+
+@pytest.mark.gpu
+def test_stepping_at_a_memory_limit(sgdg):
+    # no room to keep the states of the call's start, or for sets padded to
+    # whole ones: the whole operator steps them one by one in three scratch
+    # vectors; a budget below those is refused
+    import torch
+    D, k, n, solves, dt = 2, 3, 5, 65, 1e-4
+    op = sgdg.SparseGridOperator(D, k, n)
+    N = op.N
+    y = torch.tensor(np.random.default_rng(0).standard_normal(solves * 2 * N), device="cuda")
+    one, two, three = y.clone(), y.clone(), y.clone()
+    op.plain_steps_device(one.data_ptr(), solves, dt, 2)
+    op.device_csr(-1)  # the whole operator is there before the limit
+    try:
+        sgdg.set_hbm_budget(sgdg.hbm_in_use() + 8 * solves * 2 * N * 3 + 64)
+        op.plain_steps_device(two.data_ptr(), solves, dt, 2)
+        assert float((one - two).norm() / one.norm()) < 1e-12
+        sgdg.set_hbm_budget(sgdg.hbm_in_use() + 8 * solves * 2 * N * 2)
+        with pytest.raises(sgdg.SGDGError) as e:
+            op.plain_steps_device(three.data_ptr(), solves, dt, 2)
+        assert e.value.code == 2 and torch.equal(three, y)
+    finally:
+        sgdg.set_hbm_budget(0)
