@@ -331,4 +331,45 @@ CSR wave_rhs(const CSR& lap) {
     return R;
 }
 
+LineTables line_tables(const CSR& T1, int k, int levels) {
+    LineTables T;
+    T.k = k;
+    T.levels = levels;
+    // first and one past the last finest cell of 1D index j's support
+    auto cells = [&](int j, int64_t& lo, int64_t& hi) {
+        const int blk = j / k;
+        int L = 1;
+        while (L < 32 && (blk >> (L - 1)) != 0) L++;
+        const int64_t c = L >= 2 ? blk - (int64_t(1) << (L - 2)) : 0, w = (int64_t(1) << 32) / ncells(L);
+        lo = c * w;
+        hi = lo + w;
+    };
+    std::vector<std::pair<int32_t, double>> row;
+    for (int lm = 1; lm <= levels; lm++) {
+        const int m = k << (lm - 1);
+        T.roff.push_back((int64_t)T.rowptr.size());
+        T.rowptr.push_back((int64_t)T.col.size());
+        for (int r = 0; r < m; r++) {
+            int64_t a1, b1, a2, b2;
+            cells(r, a1, b1);
+            row.clear();
+            for (int64_t p = T1.rowptr[r]; p < T1.rowptr[r + 1]; p++) {
+                if (T1.col[p] >= m) continue;
+                cells(T1.col[p], a2, b2);
+                if ((a1 <= a2 && b1 >= b2) || (a1 >= a2 && b1 <= b2)) row.push_back({T1.col[p], T1.val[p]});
+            }
+            std::sort(row.begin(), row.end(),
+                      [](const std::pair<int32_t, double>& x, const std::pair<int32_t, double>& y) {
+                          return x.first < y.first;
+                      });
+            for (const auto& e : row) {
+                T.col.push_back(e.first);
+                T.val.push_back(e.second);
+            }
+            T.rowptr.push_back((int64_t)T.col.size());
+        }
+    }
+    return T;
+}
+
 }  // namespace sgdg

@@ -26,14 +26,24 @@ cudaError_t step_bounds_violations(unsigned int* out, bool reset);
 cudaError_t asm_bounds_violations(unsigned int* out, bool reset);
 cudaError_t launch_csr_rk4(const DevCSR& A, const double* uin, double* y, double* acc, double* uout, double dt,
                            int stage, int* nonfinite, cudaStream_t st);
+cudaError_t launch_csr_rk4(const DevSliced& A, const double* uin, double* y, double* acc, double* uout, double dt,
+                           int stage, int* nonfinite, cudaStream_t st);
 int plain_set_size(const DevCSR& A, int64_t nb);
+int plain_set_size(const DevSliced& A, int64_t nb);
 cudaError_t launch_plain_steps(const DevCSR& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
                                double dt, int64_t nsteps, int* nonfinite, cudaStream_t st);
-cudaError_t launch_plain_interleave(const DevCSR& A, int nv, int64_t nb, const double* y, double* u0, cudaStream_t st);
+cudaError_t launch_plain_steps(const DevSliced& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
+                               double dt, int64_t nsteps, int* nonfinite, cudaStream_t st);
+cudaError_t launch_plain_interleave(int64_t len, int nv, int64_t nb, const double* y, double* u0, cudaStream_t st);
 cudaError_t launch_csr_spmv_multi(const DevCSR& A, int nv, const double* x, int64_t xi, int64_t xs, double* y,
                                   int64_t yi, int64_t ys, cudaStream_t st);
 cudaError_t launch_vlasov_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                                  cudaStream_t st);
+cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, int* nonfinite, cudaStream_t st);
+cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x, double* y, cudaStream_t st);
+cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
+                          cudaStream_t st);
+cudaError_t launch_check_finite(const double* x, int64_t n, int* nonfinite, cudaStream_t st);
 cudaError_t launch_wait_selftest(const int* ctr, int need, int* err, cudaStream_t st);
 cudaError_t launch_convert_selftest(const double* x, int64_t n, unsigned long long* bad, cudaStream_t st);
 
@@ -53,7 +63,7 @@ struct sgdg_op {
     std::vector<std::unique_ptr<CSR>> dd;  // D_d, built on demand
     std::unique_ptr<CSR> lap, wave;
     std::map<int, std::unique_ptr<DeviceCSR>> dev;  // plain-form device copies by `which`
-    std::map<int, std::unique_ptr<DeviceCSR>> step_dev;  // without the rounding of zeros (stepping)
+    std::map<int, std::unique_ptr<DeviceSliced>> step_dev;  // without the rounding of zeros (stepping)
     std::unique_ptr<DeviceAdvection> adv;
     std::map<int, std::unique_ptr<MFEngine>> mf_apply;
     cudaStream_t stream = nullptr;
@@ -103,11 +113,9 @@ struct sgdg_op {
     // nonzero).  They do carry NaN and infinities from one row to another, so
     // a run that meets one is repeated with the whole operator (plain_run).
     bool prunes() const { return basis == SGDG_BASIS_HIER && ix.k <= kPruneMaxK; }
-    const DevCSR& stepping(int which) {
-        if (!prunes()) return device(which);
+    const DevSliced& stepping(int which) {
         auto it = step_dev.find(which);
-        if (it == step_dev.end())
-            it = step_dev.emplace(which, gpu_operator(ix, *dlf, which, stream, 0, true)).first;
+        if (it == step_dev.end()) it = step_dev.emplace(which, gpu_step_operator(ix, *dlf, which, stream)).first;
         return it->second->d;
     }
     // the whole operator, the pruned one making room for it where there is none
@@ -136,6 +144,15 @@ struct sgdg_op {
 // there; the host copies of the transforms are built only when asked for
 // (export), and the velocity points with the device transforms when a GPU
 // is present, else with the host ones.
+//
+// The right-hand side is stepped as sweeps: a D-dimensional transform is the
+// product of its 1D map along each dimension in turn, exactly, because the 1D
+// maps are triangular in the level (no intermediate leaves the sparse grid).
+// 2x2v k=2 n=8 multiplies 15 + 18 + 8 + 20 entries per coefficient that way
+// where the assembled transforms hold 147 + 120 + 12 + 244, and the derivatives
+// go without the rounding of zeros (22 entries instead of 50).  The assembled
+// operators (whole_rhs) are built and used when a run meets a value that is not
+// finite, which they spread over more rows.
 struct sgdg_vlasov {
     int D = 0, P = 0, k = 0, n = 0;
     SparseIndex ix;
@@ -143,9 +160,14 @@ struct sgdg_vlasov {
     mutable std::unique_ptr<CSR> T[4];    // m2n, n2p, p2n, n2m on the host, built on request
     mutable std::vector<double> v_point;  // D x N, built on request
     mutable bool have_vpoint = false;
+    // sweep[w][d]: transform w along dimension d; deriv[d]: D_d
+    std::unique_ptr<DeviceSliced> sweep[4][8], deriv[8];
+    // the assembled operators, built on request
     std::vector<std::unique_ptr<DeviceCSR>> dDs;
     std::unique_ptr<DeviceCSR> dT[4];
-    DevBuf vpt, F, t, s, p, c, z;  // t, s, p: P vectors each, interleaved (t[i * P + d])
+    DevBuf vpt, F, t, s, c, z;  // t, s: P vectors each, interleaved (t[i * P + d])
+    DevBuf p;                   // P vectors for the assembled operators
+    DevBuf flag;                // a result was not finite
     cudaStream_t stream = nullptr;
     ~sgdg_vlasov() {
         if (stream) cudaStreamDestroy(stream);
@@ -180,41 +202,100 @@ struct sgdg_vlasov {
         have_vpoint = true;
     }
     void to_gpu() {
-        if (stream) return;
+        if (flag.p) return;
         require_gpu();
-        CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        // the phase-space derivatives keep 8 entries per lane, like the transforms they feed
-        // (at 32 the Vlasov plain step took 2.67 ms against 2.60)
-        for (int d = 0; d < P; d++) dDs.push_back(gpu_operator(ix, *dlf, d + 1, stream, kCsrLaneEntriesMulti));
-        for (int w = 0; w < 4; w++) dT[w] = gpu_transform(ix, transform_1d(k, n, w), stream);
+        if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        build_sweeps();
+        const size_t b = sizeof(double) * (size_t)ix.N;
         if (!have_vpoint) {  // n2p m2n with the device transforms
-            const size_t b = sizeof(double) * (size_t)ix.N;
-            DevBuf x(b), y(b), w(b);
+            DevBuf x(b), y(b);
             v_point.assign((size_t)D * ix.N, 0.0);
             for (int d = 0; d < D; d++) {
                 const std::vector<double> vm = v_modal(d);
                 CK(cudaMemcpyAsync(x.p, vm.data(), b, cudaMemcpyHostToDevice, stream));
-                CK(launch_csr_spmv(dT[0]->d, x.as<double>(), y.as<double>(), stream));
-                CK(launch_csr_spmv(dT[1]->d, y.as<double>(), w.as<double>(), stream));
-                CK(cudaMemcpyAsync(v_point.data() + (size_t)d * ix.N, w.p, b, cudaMemcpyDeviceToHost, stream));
+                double *from = x.as<double>(), *to = y.as<double>();
+                CK(transform(0, 1, from, to));  // P sweeps: back in `from`
+                CK(transform(1, 1, from, to));
+                CK(cudaMemcpyAsync(v_point.data() + (size_t)d * ix.N, from, b, cudaMemcpyDeviceToHost, stream));
+                CK(cudaStreamSynchronize(stream));
             }
-            CK(cudaStreamSynchronize(stream));
             have_vpoint = true;
         }
         vpt = upload(v_point, stream);
-        const size_t b = sizeof(double) * (size_t)ix.N;
         F.alloc(b * D);
         t.alloc(b * P);
         s.alloc(b * P);
-        p.alloc(b * P);
         c.alloc(b);
         z.alloc(b);
+        flag.alloc(sizeof(int));
+        CK(cudaStreamSynchronize(stream));
+    }
+    void build_sweeps() {
+        if (sweep[3][P - 1]) return;
+        for (int d = 0; d < P; d++) deriv[d] = gpu_step_operator(ix, *dlf, d + 1, stream);
+        for (int w = 0; w < 4; w++) {
+            const LineTables T = line_tables(transform_1d(k, n, w), k, n + 1);
+            for (int d = 0; d < P; d++) sweep[w][d] = gpu_line_operator(ix, T, d, stream);
+        }
+    }
+    void drop_sweeps() {
+        for (int d = 0; d < 8; d++) {
+            deriv[d].reset();
+            for (int w = 0; w < 4; w++) sweep[w][d].reset();
+        }
+    }
+    // x = transform w of nv interleaved vectors x: P sweeps, P even, so the
+    // result is back in x; y: scratch
+    cudaError_t transform(int w, int nv, double* x, double* y) {
+        cudaError_t e = cudaSuccess;
+        for (int d = 0; d < P && e == cudaSuccess; d++, std::swap(x, y))
+            e = launch_sweep(sweep[w][d]->d, nv, x, y, nullptr, stream);
+        return e;
+    }
+    // z = all sweeps of n2m but the last, of p2n (-sum_d v_d .* n2p m2n Dx_d u
+    // + sum_d F_d .* n2p m2n Dp_d u): the P derivatives, interleaved, each
+    // transform's sweeps on all P of them at a time, the point products and the
+    // sweeps back.  The last sweep (last_sweep) takes z.
+    cudaError_t sweep_rhs(const double* u) {
+        double *tt = t.as<double>(), *ss = s.as<double>(), *cc = c.as<double>(), *zz = z.as<double>();
+        const DevSliced* D_[8];
+        for (int d = 0; d < P; d++) D_[d] = &deriv[d]->d;
+        cudaError_t e = launch_derivatives(D_, P, u, tt, stream);
+        if (e == cudaSuccess) e = transform(0, P, tt, ss);
+        if (e == cudaSuccess) e = transform(1, P, tt, ss);
+        if (e == cudaSuccess) e = launch_points(vpt.as<double>(), F.as<double>(), tt, D, ix.N, cc, stream);
+        if (e == cudaSuccess) e = transform(2, 1, cc, zz);
+        for (int d = 0; d + 1 < P && e == cudaSuccess; d++, std::swap(cc, zz))
+            e = launch_sweep(sweep[3][d]->d, 1, cc, zz, nullptr, stream);
+        return e;
+    }
+    const DevSliced& last_sweep() const { return sweep[3][P - 1]->d; }
+    // the assembled operators and their scratch; the sweeps make room for them where there is none
+    void build_whole() {
+        if (p.p) return;
+        auto build = [&] {
+            // the phase-space derivatives keep 8 entries per lane, like the transforms they feed
+            // (at 32 the plain step took 2.67 ms against 2.60)
+            for (int d = (int)dDs.size(); d < P; d++)
+                dDs.push_back(gpu_operator(ix, *dlf, d + 1, stream, kCsrLaneEntriesMulti));
+            for (int w = 0; w < 4; w++)
+                if (!dT[w]) dT[w] = gpu_transform(ix, transform_1d(k, n, w), stream);
+            p.alloc(sizeof(double) * (size_t)ix.N * P);
+            CK(cudaStreamSynchronize(stream));
+        };
+        try {
+            build();
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET || !sweep[3][P - 1]) throw;
+            drop_sweeps();
+            build();
+        }
     }
     // z = p2n (-sum_d v_d .* n2p m2n Dx_d u + sum_d F_d .* n2p m2n Dp_d u):
     // the P derivatives, interleaved (the P values of one coefficient share a
     // sector), then each transform on all P of them in one pass over its
     // matrix, the point products, and p2n
-    cudaError_t rhs_points(const double* u) {
+    cudaError_t whole_rhs(const double* u) {
         const int64_t N = ix.N;
         double *tt = t.as<double>(), *ss = s.as<double>(), *pp = p.as<double>();
         cudaError_t e = cudaSuccess;
@@ -228,13 +309,15 @@ struct sgdg_vlasov {
     }
 };
 
-// RK4 steps of the plain form: `per` steps captured as a graph (launches inside
-// it are programmatic dependents, so one comes up while the one before it
-// runs) and replayed, what is left over launched as it is.
+// RK4 steps of the plain form.  From `least` steps on, `per` steps are captured
+// as a graph (launches inside it are programmatic dependents, so one comes up
+// while the one before it runs) and replayed; fewer, and what is left over, are
+// launched as they are.  The evolvers take 8 steps (32 launches) from 8 on; a
+// Vlasov step alone is 40 to 136 launches, whose instantiation (0.2 ms at 72)
+// pays from 16 steps on (634 against 676 us per step).
 class StepGraph {
    public:
-    static constexpr int64_t kPer = 8;
-    StepGraph() = default;
+    StepGraph(int64_t per, int64_t least) : per_(per), least_(least) {}
     StepGraph(const StepGraph&) = delete;
     StepGraph& operator=(const StepGraph&) = delete;
     ~StepGraph() {
@@ -243,8 +326,8 @@ class StepGraph {
     // launches nsteps steps on st (never the legacy stream), steps(n) launching n of them
     template <class Steps>
     void run(int64_t nsteps, cudaStream_t st, Steps&& steps) {
-        if (nsteps >= kPer && !exec_) capture(st, steps);
-        for (; nsteps >= kPer; nsteps -= kPer) CK(cudaGraphLaunch(exec_, st));
+        if (nsteps >= least_ && !exec_) capture(st, steps);
+        for (; exec_ && nsteps >= per_; nsteps -= per_) CK(cudaGraphLaunch(exec_, st));
         CK(steps(nsteps));
     }
 
@@ -253,7 +336,7 @@ class StepGraph {
     void capture(cudaStream_t st, Steps&& steps) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const cudaError_t e = steps(kPer);
+        const cudaError_t e = steps(per_);
         const cudaError_t e2 = cudaStreamEndCapture(st, &g);
         if (e != cudaSuccess || e2 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
@@ -266,6 +349,7 @@ class StepGraph {
             throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
         }
     }
+    const int64_t per_, least_;
     cudaGraphExec_t exec_ = nullptr;
 };
 
@@ -565,9 +649,12 @@ static std::vector<int64_t> out_steps(int64_t nsteps, int nout) {
     return s;
 }
 
+}  // extern "C"
+
 // One evolution y' = A y from host to host; returns whether a stage result
 // was not finite.
-static bool plain_run(const DevCSR& A, const double* y0, int64_t len, double t0, double t1, int64_t nsteps, int nout,
+template <class Mat>
+static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, double t1, int64_t nsteps, int nout,
                       double* times, double* states, cudaStream_t st) {
     const size_t b = sizeof(double) * (size_t)len;
     DevBuf work(4 * b + sizeof(int));
@@ -578,7 +665,7 @@ static bool plain_run(const DevCSR& A, const double* y0, int64_t len, double t0,
     CK(cudaMemcpyAsync(y, y0, b, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
     const auto steps = out_steps(nsteps, nout);
-    StepGraph graph;
+    StepGraph graph(8, 8);
     int64_t done = 0;
     int bad = 0;
     for (int i = 0; i < nout; i++) {
@@ -600,7 +687,7 @@ static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t
     std::vector<double> s;  // -sum_d a_d D_d
     for (int d = 0; a && d < op->ix.D; d++) s.push_back(-a[d]);
     if (op->prunes()) {
-        const DevCSR* A = nullptr;
+        const DevSliced* A = nullptr;
         if (a) {
             if (!op->adv) op->adv = gpu_advection(op->ix, *op->dlf, st);
             CK(op->adv->scale(op->ix.D, s.data(), st));
@@ -624,18 +711,20 @@ static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t
 struct PlainScratch {
     DevBuf acc, u0, u1, flag;
     int nv;
-    PlainScratch(const DevCSR& A, int64_t nb, int nv_) : flag(sizeof(int)), nv(nv_) {
+    template <class Mat>
+    PlainScratch(const Mat& A, int64_t nb, int nv_) : flag(sizeof(int)), nv(nv_) {
         const size_t b = sizeof(double) * (size_t)((nb + nv - 1) / nv * nv * A.m);
         acc.alloc(b);
         u0.alloc(b);
         u1.alloc(b);
     }
     // returns whether a stage result was not finite; waits for the steps
-    bool run(const DevCSR& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
+    template <class Mat>
+    bool run(const Mat& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
         int bad = 0;
-        StepGraph graph;
+        StepGraph graph(8, 8);
         CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-        CK(launch_plain_interleave(A, nv, nb, y, u0.as<double>(), st));
+        CK(launch_plain_interleave(A.m, nv, nb, y, u0.as<double>(), st));
         graph.run(nsteps, st, [&](int64_t n) {
             return launch_plain_steps(A, nv, nb, y, acc.as<double>(), u0.as<double>(), u1.as<double>(), dt, n,
                                       flag.as<int>(), st);
@@ -668,7 +757,7 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
     }
     std::unique_ptr<PlainScratch> work;
     DevBuf keep;
-    const DevCSR* A = nullptr;
+    const DevSliced* A = nullptr;
     if (op->prunes()) {
         try {
             A = &op->stepping(which);
@@ -688,14 +777,16 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
         work.reset();
         keep.release();
     }
-    A = &op->whole(which);
+    const DevCSR& W = op->whole(which);
     try {
-        work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));
+        work.reset(new PlainScratch(W, nsolves, plain_set_size(W, nsolves)));
     } catch (const Error&) {
-        work.reset(new PlainScratch(*A, nsolves, 1));
+        work.reset(new PlainScratch(W, nsolves, 1));
     }
-    work->run(*A, nsolves, y, dt, nsteps, cs);
+    work->run(W, nsolves, y, dt, nsteps, cs);
 }
+
+extern "C" {
 
 static void mf_evolve(sgdg_op* op, int kind, const double* a, const double* y0, int64_t len, double t0, double t1,
                       int64_t nsteps, int nout, double* times, double* states) {
@@ -963,12 +1054,24 @@ int sgdg_vlasov_rhs(sgdg_vlasov* v, const double* F_point, const double* f, doub
     const int64_t N = v->ix.N;
     const size_t b = sizeof(double) * (size_t)N;
     DevBuf u(b), r(b);
+    int bad = 0;
     CK(cudaMemcpyAsync(v->F.p, F_point, b * v->D, cudaMemcpyHostToDevice, v->stream));
     CK(cudaMemcpyAsync(u.p, f, b, cudaMemcpyHostToDevice, v->stream));
-    CK(v->rhs_points(u.as<double>()));
-    CK(launch_csr_spmv(v->dT[3]->d, v->z.as<double>(), r.as<double>(), v->stream));
+    CK(cudaMemsetAsync(v->flag.p, 0, sizeof(int), v->stream));
+    v->build_sweeps();
+    CK(launch_check_finite(u.as<double>(), N, v->flag.as<int>(), v->stream));
+    CK(v->sweep_rhs(u.as<double>()));
+    CK(launch_sweep(v->last_sweep(), 1, v->z.as<double>(), r.as<double>(), v->flag.as<int>(), v->stream));
     CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
+    CK(cudaMemcpyAsync(&bad, v->flag.p, sizeof(int), cudaMemcpyDeviceToHost, v->stream));
     CK(cudaStreamSynchronize(v->stream));
+    if (bad) {
+        v->build_whole();
+        CK(v->whole_rhs(u.as<double>()));
+        CK(launch_csr_spmv(v->dT[3]->d, v->z.as<double>(), r.as<double>(), v->stream));
+        CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
+        CK(cudaStreamSynchronize(v->stream));
+    }
     API_END
 }
 
@@ -1013,42 +1116,48 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
     const size_t b = sizeof(double) * (size_t)N;
     DevBuf y(b), acc(b), u0(b), u1(b);
     CK(cudaMemcpyAsync(v->F.p, F_point, b * v->D, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(y.p, f0, b, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
-    // one RK4 step as a graph: per stage the right-hand side in the point
-    // basis, then n2m fused with the stage update
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     const double* in[4] = {y.as<double>(), u0.as<double>(), u1.as<double>(), u0.as<double>()};
     double* outv[4] = {u0.as<double>(), u1.as<double>(), u0.as<double>(), u1.as<double>()};
-    cudaError_t e = cudaSuccess;
-    for (int stage = 1; stage <= 4 && e == cudaSuccess; stage++) {
-        e = v->rhs_points(in[stage - 1]);
-        if (e == cudaSuccess)
-            e = launch_csr_rk4(v->dT[3]->d, v->z.as<double>(), y.as<double>(), acc.as<double>(), outv[stage - 1], dt,
-                               stage, nullptr, st);
+    int* flag = v->flag.as<int>();
+    const auto steps = out_steps(nsteps, nout);
+    // per stage the right-hand side in the nodal basis, then the last sweep (or
+    // the whole) of n2m fused with the stage update; returns whether a stage
+    // was not finite
+    auto run = [&](bool whole) {
+        StepGraph graph(1, 16);
+        auto launch = [&](int64_t n) {
+            cudaError_t e = cudaSuccess;
+            for (int64_t i = 0; i < n; i++)
+                for (int stage = 1; stage <= 4 && e == cudaSuccess; stage++) {
+                    e = whole ? v->whole_rhs(in[stage - 1]) : v->sweep_rhs(in[stage - 1]);
+                    if (e == cudaSuccess)
+                        e = whole ? launch_csr_rk4(v->dT[3]->d, v->z.as<double>(), y.as<double>(), acc.as<double>(),
+                                                   outv[stage - 1], dt, stage, flag, st)
+                                  : launch_csr_rk4(v->last_sweep(), v->z.as<double>(), y.as<double>(), acc.as<double>(),
+                                                   outv[stage - 1], dt, stage, flag, st);
+                }
+            return e;
+        };
+        int bad = 0;
+        int64_t done = 0;
+        CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+        CK(cudaMemcpyAsync(y.p, f0, b, cudaMemcpyHostToDevice, st));
+        for (int i = 0; i < nout; i++) {
+            graph.run(steps[i] - done, st, launch);
+            done = steps[i];
+            CK(cudaMemcpyAsync(states + (size_t)i * N, y.p, b, cudaMemcpyDeviceToHost, st));
+            if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
+        }
+        CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        return bad != 0;
+    };
+    v->build_sweeps();
+    if (run(false)) {
+        v->build_whole();
+        run(true);
     }
-    cudaError_t e2 = cudaStreamEndCapture(st, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        throw Error(SGDG_ECUDA, std::string("capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
-    }
-    cudaError_t e3 = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (e3 != cudaSuccess) throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
-    auto steps = out_steps(nsteps, nout);
-    int64_t done = 0;
-    cudaError_t err = cudaSuccess;
-    for (int i = 0; i < nout && err == cudaSuccess; i++) {
-        for (; done < steps[i] && err == cudaSuccess; done++) err = cudaGraphLaunch(ge, st);
-        if (err == cudaSuccess)
-            err = cudaMemcpyAsync(states + (size_t)i * N, y.p, b, cudaMemcpyDeviceToHost, st);
-        if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
-    }
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-    cudaGraphExecDestroy(ge);
-    if (err != cudaSuccess) throw Error(SGDG_ECUDA, std::string("vlasov evolve: ") + cudaGetErrorString(err));
     API_END
 }
 

@@ -1,28 +1,41 @@
-// csr_step.cu -- the plain form's stepping: FP64 CSR mat-vec (the closure body
-// *(RHS, x) of src/pdes.jl:63) fused with the classical RK4 stage update, for
-// one solve or for sets of solves that share the operator.
+// csr_step.cu -- the plain form's stepping: FP64 sparse mat-vec (the closure
+// body *(RHS, x) of src/pdes.jl:63) fused with the classical RK4 stage update,
+// for one solve or for sets of solves that share the operator, and the sweeps
+// of the Vlasov right-hand side (src/pdes.jl:174-192).
 //
-//  * k_csr_rk: rows binned by length (DevCSR.bin_*), a row of bin b summed by
-//    2^b lanes with a few entries each (csr_lane_entries); every block of the
-//    grid serves one bin.  NV solves go through a row together: a matrix entry
-//    is loaded once and meets the set's interleaved values in one 16- or
-//    32-byte load.  Bounds: large operators the FP64 pipe (2 operations per
-//    clock and SM, the additions of the lane reduction and of the stage update
-//    among them), small ones the latency of four dependent launches per step.
-//    For the second the launches are programmatic dependents (pdl_wait): a
-//    launch's blocks come up and fetch their row pointers, columns and values
-//    while the launch before it still runs, and wait for it only before the
-//    vectors.  200 steps of the 2D wave k=3 n=5 from host to host took 6.34 ms
-//    with one solve at a time, the whole operator and plain launches, 1.94 ms
-//    now; 60 steps of the 4D advection k=2 n=6 5.89 -> 1.42 ms; 3 steps of 48
-//    3D waves k=3 n=7 11.8 -> 3.2 ms (0.94 ms per step, of which the FP64 pipe
-//    needs 0.75).
+//  * k_csr_rk: a row of bin b summed by 2^b lanes with a few entries each
+//    (csr_lane_entries); every block of the grid serves one bin.  NV solves go
+//    through a row together: a matrix entry is loaded once and meets the set's
+//    interleaved values in one 16- or 32-byte load.  The stepping operators are
+//    in slices (DevSliced: rows sorted by length, a warp's entries adjacent),
+//    whole ones (DevCSR) in rows.
 //  * k_rk_segments, k_rk_long_rows: rows longer than A.split, one warp per
 //    segment, then the segment partials of each row in order and the update.
+//  * k_derivatives, k_sweep, k_points: the P derivatives of a phase-space
+//    vector, a transform along one dimension for P interleaved vectors or one,
+//    and the products at the points.
+//
+// Bounds: large operators the FP64 pipe (2 operations per clock and SM, the
+// additions of the lane reduction and of the stage update among them), small
+// ones the latency of four dependent launches per step (Vlasov: 4 (4P + 2)).
+// For the second the launches are programmatic dependents (pdl_wait): a
+// launch's blocks come up and fetch their rows, columns and values while the
+// launch before it still runs, and wait for it only before the vectors.
+//
+// Measured, from host to host: 200 steps of the 2D wave k=3 n=5 6.34 -> 2.0 ms
+// against one solve at a time with the whole operator and plain launches; 60
+// steps of the 4D advection k=2 n=6 5.89 -> 1.5 ms; 3 steps of 48 3D waves k=3
+// n=7 11.8 -> 3.1 ms (0.87 ms per step, of which the FP64 pipe needs 0.74).
+// In slices against rows: the single 3D wave 46.9 -> 38.1 us per step, 256 of
+// them 4.80 -> 4.49 ms, the Vlasov step below 810 -> 634 us.  Vlasov 2x2v k=2
+// n=8: 2595 -> 634 us per step against the assembled transforms, of which the
+// FP64 pipe needs 231 (a k_sweep<4> keeps it 78 % busy) and about 195 are the
+// latency of 72 launches (what the step takes at n=5, 8832 coefficients).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "bounds.cuh"
 #include "csr.cuh"
@@ -56,17 +69,17 @@ __device__ __forceinline__ void ld_v4(const double* p, double& a, double& b, dou
     asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p) : "memory");
 }
 
-// the values of a set of NV interleaved vectors at one column
+// the values of NV adjacent vectors at one element
 template <int NV>
-__device__ __forceinline__ void set_gather(const double* x, int64_t col, double (&v)[NV]) {
+__device__ __forceinline__ void set_gather(const double* x, double (&v)[NV]) {
     if constexpr (NV == 4) {
-        ld_v4(x + col * 4, v[0], v[1], v[2], v[3]);
+        ld_v4(x, v[0], v[1], v[2], v[3]);
     } else if constexpr (NV == 2) {
-        const double2 t = __ldca(reinterpret_cast<const double2*>(x + col * 2));
+        const double2 t = __ldca(reinterpret_cast<const double2*>(x));
         v[0] = t.x;
         v[1] = t.y;
     } else {
-        v[0] = __ldca(x + col);
+        v[0] = __ldca(x);
     }
 }
 
@@ -91,7 +104,8 @@ __device__ __forceinline__ void csr_fetch(const DevCSR& A, int64_t p, int64_t e,
     }
 }
 
-// s[j] = the row with entries [b, e) times vector j, summed over VS lanes: the
+// s[j] = the row with entries [b, e) times vector j (element i of the set at
+// x + i stride), summed over VS lanes: the
 // entries b + lane, b + lane + VS, ... in order, the first of them in t already
 // (b = e: zeros, but the lanes still take part); see csr_reduce for where the
 // sums end up.  The order does not depend on NV, so a solve's result is the
@@ -100,7 +114,7 @@ __device__ __forceinline__ void csr_fetch(const DevCSR& A, int64_t p, int64_t e,
 // would still take their turn on the FP64 pipe.
 template <int VS, int NV>
 __device__ __forceinline__ void row_sum(const DevCSR& A, int64_t b, int64_t e, CsrAhead& t, const double* x, int lane,
-                                        double (&s)[NV]) {
+                                        int64_t stride, double (&s)[NV]) {
 #pragma unroll
     for (int j = 0; j < NV; j++) s[j] = 0.0;
     const int most = __reduce_max_sync(0xffffffffu, (int)(e - b));
@@ -109,7 +123,7 @@ __device__ __forceinline__ void row_sum(const DevCSR& A, int64_t b, int64_t e, C
         double xv[kCsrAhead][NV];
 #pragma unroll
         for (int u = 0; u < kCsrAhead; u++)
-            if (t.c[u] >= 0) set_gather<NV>(x, t.c[u], xv[u]);
+            if (t.c[u] >= 0) set_gather<NV>(x + t.c[u] * stride, xv[u]);
         CsrAhead next;  // the entries after these, while the gathers are on their way
         p += kCsrAhead * VS;
         csr_fetch<VS>(A, p, e, next);
@@ -126,6 +140,8 @@ __device__ __forceinline__ void row_sum(const DevCSR& A, int64_t b, int64_t e, C
     csr_reduce<VS, NV>(s, lane);
 }
 
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+
 // RK4 stage update of one element: k its right-hand side, y its state, acc and
 // uout at element `o` of the scratch vectors
 __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double* y, int64_t o) {
@@ -136,14 +152,14 @@ __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double*
     else
         rk.acc[o] = aa;
     if (rk.stage != 4 || rk.write_u) rk.uout[o] = un;
-    if (rk.nonfinite && (__double2hiint(un) & 0x7ff00000) == 0x7ff00000) *rk.nonfinite = 1;
+    if (rk.nonfinite && not_finite(un)) *rk.nonfinite = 1;
 }
 
-// the rows of bin `bin`, 2^bin = VS lanes each; nv of the NV solves are stored,
-// solve j's state at y + j A.m
-template <int VS, int NV>
-__device__ __forceinline__ void rk_bin(const DevCSR& A, int bin, int64_t rb, const double* x, double* y,
-                                       const CsrRK& rk, int nv) {
+// Block rb's rows, 2^bin lanes each: out.one(row, j, sum) by the lane that
+// holds vector j's sum, or out.all(row, sums) where one lane holds them all.
+template <int VS, int NV, class Out>
+__device__ __forceinline__ void bin_rows(const DevCSR& A, int bin, int64_t rb, const double* x, int64_t stride,
+                                         const Out& out) {
     const int64_t t = (rb - A.bin_block[bin]) * blockDim.x + threadIdx.x;
     const int64_t idx = t / VS, first = A.bin_first[bin];
     const int lane = int(t % VS);
@@ -158,18 +174,118 @@ __device__ __forceinline__ void rk_bin(const DevCSR& A, int bin, int64_t rb, con
     csr_fetch<VS>(A, b + lane, e, ahead);
     pdl_wait();
     double s[NV];
-    row_sum<VS, NV>(A, b, e, ahead, x, lane, s);
+    row_sum<VS, NV>(A, b, e, ahead, x, lane, stride, s);
     bool stores;
     const int owner = csr_owner<VS, NV>(lane, stores);
     if (row < 0 || !stores) return;
-    if (owner >= 0) {
-        if (owner < nv) csr_rk_update(rk, s[0], y + row + owner * A.m, row * NV + owner);
-    } else {
+    if (owner >= 0)
+        out.one(row, owner, s[0]);
+    else
+        out.all(row, s);
+}
+
+// the same for slices
+template <int VS, int NV, class Out>
+__device__ __forceinline__ void bin_rows(const DevSliced& A, int64_t rb, const double* x, int64_t stride,
+                                         const Out& out) {
+    const int64_t slice = rb * kSliceWarps + (threadIdx.x >> 5);
+    const int l32 = threadIdx.x & 31;
+    int64_t row = __ldg(A.rows + slice * 32 + l32);
+    const int64_t first = __ldg(A.base + slice);
+    const int n = (int)(__ldg(A.base + slice + 1) - first);
+    if (row >= 0 && !SGDG_IN(row, A.m)) row = -1;
+    const int32_t* col = A.col + first * 32 + l32;
+    const double* val = A.val + first * 32 + l32;
+    auto fetch = [&](int u0, CsrAhead& t) {
 #pragma unroll
-        for (int j = 0; j < NV; j++)
-            if (j < nv) csr_rk_update(rk, s[j], y + row + j * A.m, row * NV + j);
+        for (int u = 0; u < kCsrAhead; u++) {
+            t.c[u] = -1;
+            t.v[u] = 0.0;
+            if (u0 + u < n) {  // the same for the whole warp
+                t.c[u] = __ldg(col + (u0 + u) * 32);
+                t.v[u] = __ldg(val + (u0 + u) * 32);
+                if (t.c[u] >= 0 && !SGDG_IN(t.c[u], A.m)) t.c[u] = -1;
+            }
+        }
+    };
+    CsrAhead t;
+    fetch(0, t);
+    pdl_wait();
+    double s[NV];
+#pragma unroll
+    for (int j = 0; j < NV; j++) s[j] = 0.0;
+    for (int u0 = 0; u0 < n; u0 += kCsrAhead) {
+        double xv[kCsrAhead][NV];
+#pragma unroll
+        for (int u = 0; u < kCsrAhead; u++)
+            if (t.c[u] >= 0) set_gather<NV>(x + t.c[u] * stride, xv[u]);
+        CsrAhead next;
+        fetch(u0 + kCsrAhead, next);
+#pragma unroll
+        for (int u = 0; u < kCsrAhead; u++) {
+            if (u0 + u >= n) break;
+            if (t.c[u] >= 0) {
+#pragma unroll
+                for (int j = 0; j < NV; j++) s[j] = fma(t.v[u], xv[u][j], s[j]);
+            }
+        }
+        t = next;
+    }
+    const int lane = l32 % VS;
+    csr_reduce<VS, NV>(s, lane);
+    bool stores;
+    const int owner = csr_owner<VS, NV>(lane, stores);
+    if (row < 0 || !stores) return;
+    if (owner >= 0)
+        out.one(row, owner, s[0]);
+    else
+        out.all(row, s);
+}
+
+template <int NV, class Out>
+__device__ __forceinline__ void block_rows(const DevSliced& A, int64_t rb, const double* x, int64_t stride,
+                                           const Out& out) {
+    int bin = 0;
+    while (bin + 1 < kCsrBins && rb >= A.bin_block[bin + 1]) bin++;
+    switch (bin) {
+        case 0: bin_rows<1, NV>(A, rb, x, stride, out); break;
+        case 1: bin_rows<2, NV>(A, rb, x, stride, out); break;
+        case 2: bin_rows<4, NV>(A, rb, x, stride, out); break;
+        case 3: bin_rows<8, NV>(A, rb, x, stride, out); break;
+        case 4: bin_rows<16, NV>(A, rb, x, stride, out); break;
+        default: bin_rows<32, NV>(A, rb, x, stride, out); break;
     }
 }
+
+template <int NV, class Out>
+__device__ __forceinline__ void block_rows(const DevCSR& A, int64_t rb, const double* x, int64_t stride, const Out& out) {
+    int bin = 0;
+    while (bin + 1 < kCsrBins && rb >= A.bin_block[bin + 1]) bin++;
+    switch (bin) {
+        case 0: bin_rows<1, NV>(A, 0, rb, x, stride, out); break;
+        case 1: bin_rows<2, NV>(A, 1, rb, x, stride, out); break;
+        case 2: bin_rows<4, NV>(A, 2, rb, x, stride, out); break;
+        case 3: bin_rows<8, NV>(A, 3, rb, x, stride, out); break;
+        case 4: bin_rows<16, NV>(A, 4, rb, x, stride, out); break;
+        default: bin_rows<32, NV>(A, 5, rb, x, stride, out); break;
+    }
+}
+
+// the stage update of nv of the NV solves of a set, solve j's state at y + j m
+template <int NV>
+struct RkOut {
+    const CsrRK& rk;
+    double* y;
+    int64_t m;
+    int nv;
+    __device__ __forceinline__ void one(int64_t row, int j, double s) const {
+        if (j < nv) csr_rk_update(rk, s, y + row + j * m, row * NV + j);
+    }
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+#pragma unroll
+        for (int j = 0; j < NV; j++) one(row, j, s[j]);
+    }
+};
 
 // Sets of NV solves sharing A: set g's vectors (interleaved x, acc and uout,
 // and the states one after another) start at g NV A.m.  Block b is (row block,
@@ -183,9 +299,9 @@ struct CsrSets {
     int last;  // solves of the last set
 };
 
-template <int NV>
-__global__ void __launch_bounds__(256, NV == 1 ? 6 : 4)
-    k_csr_rk(DevCSR A, const double* x, double* y, CsrRK rk, CsrSets q) {
+template <int NV, class Mat>
+__global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
+    k_csr_rk(Mat A, const double* x, double* y, CsrRK rk, CsrSets q) {
     int64_t rb = blockIdx.x, g = 0;
     if (q.count > 1) {
         const int64_t nrb = A.bin_block[kCsrBins], b = blockIdx.x, full = q.count / q.group, fb = full * nrb * q.group;
@@ -204,17 +320,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 6 : 4)
         rk.acc += o;
         rk.uout += o;
     }
-    const int nv = g + 1 == q.count ? q.last : NV;
-    int bin = 0;
-    while (bin + 1 < kCsrBins && rb >= A.bin_block[bin + 1]) bin++;
-    switch (bin) {
-        case 0: rk_bin<1, NV>(A, 0, rb, x, y, rk, nv); break;
-        case 1: rk_bin<2, NV>(A, 1, rb, x, y, rk, nv); break;
-        case 2: rk_bin<4, NV>(A, 2, rb, x, y, rk, nv); break;
-        case 3: rk_bin<8, NV>(A, 3, rb, x, y, rk, nv); break;
-        case 4: rk_bin<16, NV>(A, 4, rb, x, y, rk, nv); break;
-        default: rk_bin<32, NV>(A, 5, rb, x, y, rk, nv); break;
-    }
+    block_rows<NV>(A, rb, x, NV, RkOut<NV>{rk, y, A.m, g + 1 == q.count ? q.last : NV});
 }
 
 // one warp per segment of a long row
@@ -230,7 +336,7 @@ __global__ void __launch_bounds__(256) k_rk_segments(DevCSR A, const double* x) 
     csr_fetch<32>(A, b + lane, e, ahead);
     pdl_wait();
     double s[1];
-    row_sum<32, 1>(A, b, e, ahead, x, lane, s);
+    row_sum<32, 1>(A, b, e, ahead, x, lane, 1, s);
     if (seg < A.nseg && lane == 0) A.partial[seg] = s[0];
 }
 
@@ -246,6 +352,90 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
     csr_rk_update(rk, s, y + row, row);
 }
 
+// NV adjacent vectors of an interleaved set (element i of vector j at
+// y[i * stride + j]); a result that is not finite raises *nonfinite
+template <int NV>
+struct SweepOut {
+    double* y;
+    int64_t stride;
+    int* nonfinite;
+    __device__ __forceinline__ void one(int64_t row, int j, double s) const {
+        y[row * stride + j] = s;
+        if (nonfinite && not_finite(s)) *nonfinite = 1;
+    }
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+        double* p = y + row * stride;
+        if constexpr (NV == 4)
+            asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(s[0]), "d"(s[1]), "d"(s[2]), "d"(s[3])
+                         : "memory");
+        else if constexpr (NV == 2)
+            *reinterpret_cast<double2*>(p) = make_double2(s[0], s[1]);
+        else
+            one(row, 0, s[0]);
+    }
+};
+
+// One sweep y = T x of a transform along one dimension (DevCSR of the lines),
+// for sets of NV of `stride` interleaved vectors; blockIdx.y: the set.
+template <int NV>
+__global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
+    k_sweep(DevSliced A, const double* x, double* y, int64_t stride, int* nonfinite) {
+    const int64_t o = (int64_t)blockIdx.y * NV;
+    block_rows<NV>(A, blockIdx.x, x + o, stride, SweepOut<NV>{y + o, stride, nonfinite});
+}
+
+// The P derivatives of one vector, interleaved: y[i P + d] = (D_d x)_i; blockIdx.y: d.
+struct DerivativeSet {
+    DevSliced d[8];
+};
+__global__ void __launch_bounds__(256, 4)
+    k_derivatives(const __grid_constant__ DerivativeSet S, const double* x, double* y, int64_t P) {
+    const DevSliced& A = S.d[blockIdx.y];
+    if ((int)blockIdx.x >= A.bin_block[kCsrBins]) {
+        pdl_wait();
+        return;
+    }
+    block_rows<1>(A, blockIdx.x, x, 1, SweepOut<1>{y + blockIdx.y, P, nullptr});
+}
+
+// The point-basis combination of the Vlasov right-hand side (src/pdes.jl:
+// 185-191): with the 2D transformed derivatives interleaved, pt[i * 2D + d]
+// (x dimensions d < D, then p),
+//   out = -(sum_d v_d .* pt_d) + sum_d F_d .* pt_{D+d},
+// each sum left to right with separate roundings of products and sums.
+template <int D>
+__global__ void k_points(const double* __restrict__ v, const double* __restrict__ F, const double* pt, int64_t n,
+                         double* out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double vv[D], ff[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        vv[d] = i < n ? __ldg(v + d * n + i) : 0.0;
+        ff[d] = i < n ? __ldg(F + d * n + i) : 0.0;
+    }
+    pdl_wait();
+    if (i >= n) return;
+    double q[2 * D];
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        const double2 t = __ldca(reinterpret_cast<const double2*>(pt + i * 2 * D) + d);
+        q[2 * d] = t.x;
+        q[2 * d + 1] = t.y;
+    }
+    double c1 = __dmul_rn(vv[0], q[0]), c2 = __dmul_rn(ff[0], q[D]);
+#pragma unroll
+    for (int d = 1; d < D; d++) {
+        c1 = __dadd_rn(c1, __dmul_rn(vv[d], q[d]));
+        c2 = __dadd_rn(c2, __dmul_rn(ff[d], q[D + d]));
+    }
+    out[i] = __dadd_rn(-c1, c2);
+}
+
+__global__ void k_check_finite(const double* __restrict__ x, int64_t n, int* nonfinite) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (not_finite(x[i])) *nonfinite = 1;
+}
+
 SGDG_BOUNDS_READER(step_bounds_violations)
 
 // ------------------------------------------------------------ launchers ----
@@ -257,12 +447,12 @@ static int grid_for(int64_t threads) {
 // a launch that may come up while the one before it in the stream still runs
 // (its kernel calls pdl_wait before it touches what that one writes)
 template <class... P, class... Q>
-static void launch_dependent(void (*kernel)(P...), int64_t blocks, cudaStream_t st, Q... args) {
+static void launch_dependent(void (*kernel)(P...), dim3 grid, cudaStream_t st, Q... args) {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)blocks);
+    c.gridDim = grid;
     c.blockDim = dim3(256);
     c.stream = st;
     c.attrs = &at;
@@ -270,16 +460,24 @@ static void launch_dependent(void (*kernel)(P...), int64_t blocks, cudaStream_t 
     (void)cudaLaunchKernelEx(&c, kernel, P(args)...);  // the caller reads the error with cudaGetLastError
 }
 
+template <class Mat>
+static cudaError_t rk4_one(const Mat& A, const double* uin, double* y, const CsrRK& rk, cudaStream_t st) {
+    if (A.bin_block[kCsrBins] > 0)
+        launch_dependent(k_csr_rk<1, Mat>, A.bin_block[kCsrBins], st, A, uin, y, rk, CsrSets{1, 1, 1});
+    if constexpr (std::is_same_v<Mat, DevCSR>)
+        if (A.nlong > 0) {
+            launch_dependent(k_rk_segments, grid_for(A.nseg * 32), st, A, uin);
+            launch_dependent(k_rk_long_rows, grid_for(A.nlong), st, A, y, rk);
+        }
+    return cudaGetLastError();
+}
 cudaError_t launch_csr_rk4(const DevCSR& A, const double* uin, double* y, double* acc, double* uout, double dt,
                            int stage, int* nonfinite, cudaStream_t st) {
-    const CsrRK rk{acc, uout, dt, 0.5 * dt, dt / 6.0, stage, 0, nonfinite};
-    if (A.bin_block[kCsrBins] > 0)
-        launch_dependent(k_csr_rk<1>, A.bin_block[kCsrBins], st, A, uin, y, rk, CsrSets{1, 1, 1});
-    if (A.nlong > 0) {
-        launch_dependent(k_rk_segments, grid_for(A.nseg * 32), st, A, uin);
-        launch_dependent(k_rk_long_rows, grid_for(A.nlong), st, A, y, rk);
-    }
-    return cudaGetLastError();
+    return rk4_one(A, uin, y, CsrRK{acc, uout, dt, 0.5 * dt, dt / 6.0, stage, 0, nonfinite}, st);
+}
+cudaError_t launch_csr_rk4(const DevSliced& A, const double* uin, double* y, double* acc, double* uout, double dt,
+                           int stage, int* nonfinite, cudaStream_t st) {
+    return rk4_one(A, uin, y, CsrRK{acc, uout, dt, 0.5 * dt, dt / 6.0, stage, 0, nonfinite}, st);
 }
 
 // u[(g * len + i) * NV + j] = y[(g * NV + j) * len + i]: solve g NV + j of the
@@ -296,14 +494,15 @@ __global__ void k_interleave(const double* __restrict__ y, double* __restrict__ 
 }
 
 // solves that go through a row together, given nb of them
+int plain_set_size(const DevSliced&, int64_t nb) { return nb < 2 ? 1 : nb == 2 ? 2 : kCsrMaxVec; }
 int plain_set_size(const DevCSR& A, int64_t nb) { return A.nlong > 0 || nb < 2 ? 1 : nb == 2 ? 2 : kCsrMaxVec; }
 
 // sets per group of the batched row kernel: 4 sets of 4 solves of the 3D k=3
 // n=7 wave keep their vectors in L2 while they share A's rows
 constexpr int kPlainSetGroup = 4;
 
-template <int NV>
-static void rk4_sets(const DevCSR& A, int64_t nb, double* y, double* acc, double* u0, double* u1, double dt, int stage,
+template <int NV, class Mat>
+static void rk4_sets(const Mat& A, int64_t nb, double* y, double* acc, double* u0, double* u1, double dt, int stage,
                      int* nonfinite, cudaStream_t st) {
     const int64_t len = A.m, ng = (nb + NV - 1) / NV, nrb = A.bin_block[kCsrBins];
     const double* uin = stage % 2 ? u0 : u1;
@@ -311,7 +510,7 @@ static void rk4_sets(const DevCSR& A, int64_t nb, double* y, double* acc, double
     for (int64_t g = 0; g < ng && nrb > 0; g += most) {
         const int64_t n = std::min(most, ng - g), o = g * NV * len;
         const CsrRK rk{acc + o, (stage % 2 ? u1 : u0) + o, dt, 0.5 * dt, dt / 6.0, stage, 1, nonfinite};
-        launch_dependent(k_csr_rk<NV>, nrb * n, st, A, uin + o, y + o, rk,
+        launch_dependent(k_csr_rk<NV, Mat>, (unsigned)(nrb * n), st, A, uin + o, y + o, rk,
                          CsrSets{n, kPlainSetGroup, g + n == ng ? int(nb - (ng - 1) * NV) : NV});
     }
 }
@@ -323,7 +522,8 @@ static void rk4_sets(const DevCSR& A, int64_t nb, double* y, double* acc, double
 // load.  nv is plain_set_size or 1; acc, u0 and u1 hold whole sets of A.m
 // numbers a solve, and with nv > 1 u0 holds the interleaved states on entry
 // (launch_plain_interleave) and on return.
-cudaError_t launch_plain_steps(const DevCSR& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
+template <class Mat>
+static cudaError_t plain_steps(const Mat& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
                                double dt, int64_t nsteps, int* nonfinite, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     for (int64_t i = 0; i < nsteps && e == cudaSuccess; i++) {
@@ -346,18 +546,64 @@ cudaError_t launch_plain_steps(const DevCSR& A, int nv, int64_t nb, double* y, d
     return e;
 }
 
-cudaError_t launch_plain_interleave(const DevCSR& A, int nv, int64_t nb, const double* y, double* u0,
-                                    cudaStream_t st) {
-    if (nv == 1 || A.m == 0) return cudaSuccess;
+cudaError_t launch_plain_steps(const DevCSR& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
+                               double dt, int64_t nsteps, int* nonfinite, cudaStream_t st) {
+    return plain_steps(A, nv, nb, y, acc, u0, u1, dt, nsteps, nonfinite, st);
+}
+cudaError_t launch_plain_steps(const DevSliced& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
+                               double dt, int64_t nsteps, int* nonfinite, cudaStream_t st) {
+    return plain_steps(A, nv, nb, y, acc, u0, u1, dt, nsteps, nonfinite, st);
+}
+
+cudaError_t launch_plain_interleave(int64_t len, int nv, int64_t nb, const double* y, double* u0, cudaStream_t st) {
+    if (nv == 1 || len == 0) return cudaSuccess;
     const int64_t ng = (nb + nv - 1) / nv;
     for (int64_t g = 0; g < ng; g += 65535) {
-        const int64_t n = std::min<int64_t>(65535, ng - g), o = g * nv * A.m;
-        const dim3 grid((unsigned)((A.m + 255) / 256), (unsigned)n);
+        const int64_t n = std::min<int64_t>(65535, ng - g), o = g * nv * len;
+        const dim3 grid((unsigned)((len + 255) / 256), (unsigned)n);
         if (nv == 2)
-            k_interleave<2><<<grid, 256, 0, st>>>(y + o, u0 + o, A.m, nb - g * nv);
+            k_interleave<2><<<grid, 256, 0, st>>>(y + o, u0 + o, len, nb - g * nv);
         else
-            k_interleave<4><<<grid, 256, 0, st>>>(y + o, u0 + o, A.m, nb - g * nv);
+            k_interleave<4><<<grid, 256, 0, st>>>(y + o, u0 + o, len, nb - g * nv);
     }
+    return cudaGetLastError();
+}
+
+// y = T x for P interleaved vectors (P = 1, or even)
+cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, int* nonfinite, cudaStream_t st) {
+    const unsigned nb = (unsigned)A.bin_block[kCsrBins];
+    if (nb == 0) return cudaSuccess;
+    if (P % 4 == 0)
+        launch_dependent(k_sweep<4>, dim3(nb, P / 4), st, A, x, y, P, nonfinite);
+    else if (P % 2 == 0)
+        launch_dependent(k_sweep<2>, dim3(nb, P / 2), st, A, x, y, P, nonfinite);
+    else
+        launch_dependent(k_sweep<1>, dim3(nb, P), st, A, x, y, P, nonfinite);
+    return cudaGetLastError();
+}
+
+// y[i P + d] = (D_d x)_i for the P <= 8 operators D
+cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x, double* y, cudaStream_t st) {
+    DerivativeSet S;
+    int nb = 0;
+    for (int d = 0; d < P; d++) {
+        S.d[d] = *D[d];
+        nb = std::max(nb, D[d]->bin_block[kCsrBins]);
+    }
+    for (int d = P; d < 8; d++) S.d[d] = *D[0];
+    if (nb > 0) launch_dependent(k_derivatives, dim3((unsigned)nb, P), st, S, x, y, (int64_t)P);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
+                          cudaStream_t st) {
+    auto kernel = D == 1 ? k_points<1> : D == 2 ? k_points<2> : D == 3 ? k_points<3> : k_points<4>;
+    if (n > 0) launch_dependent(kernel, (unsigned)grid_for(n), st, v, F, pt, n, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_finite(const double* x, int64_t n, int* nonfinite, cudaStream_t st) {
+    if (n > 0) k_check_finite<<<std::min(grid_for(n), 1024), 256, 0, st>>>(x, n, nonfinite);
     return cudaGetLastError();
 }
 

@@ -18,6 +18,11 @@ struct DeviceCSR {
     DevCSR d{};
 };
 
+struct DeviceSliced {
+    DevBuf base, rows, col, val, extra;
+    DevSliced d{};
+};
+
 constexpr int64_t kCsrSplit = 2048;  // entries a row group sums directly
 
 // bin of a row of L <= kCsrSplit entries: the fewest lanes 2^b (up to 32)
@@ -122,16 +127,21 @@ inline std::unique_ptr<DeviceCSR> to_device(const CSR& A, cudaStream_t st) {
 
 // The plain-form operators assembled on the GPU (gpu_assemble.cu): which =
 // 1..D for D_d, SGDG_OP_LAPLACIAN, SGDG_OP_WAVE_RHS; the same stored entries
-// and values as the host assembly (assemble.cpp).  prune: without the entries
-// that hold only the rounding of a zero (line_tables); for k <= kPruneMaxK.
+// and values as the host assembly (assemble.cpp).
 std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
-                                        int per_lane = 0, bool prune = false);
+                                        int per_lane = 0);
+// The same without the entries that hold only the rounding of a zero
+// (line_tables), in slices; for k <= kPruneMaxK.
+std::unique_ptr<DeviceSliced> gpu_step_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st);
+// The 1D operators T of the lines (per line length) along dimension d (0-based)
+std::unique_ptr<DeviceSliced> gpu_line_operator(const SparseIndex& ix, const LineTables& T, int d, cudaStream_t st);
 // The D_d of a grid one after another in each row (pruned as above), the
 // dimension of every entry and the unscaled values kept: scale() makes the
 // values those of sum_d s[d] D_d.
 struct DeviceAdvection {
-    DeviceCSR A;
-    DevBuf base, dim;
+    DeviceSliced A;
+    DevBuf base;
+    int64_t slots = 0;
     cudaError_t scale(int D, const double* s, cudaStream_t st);
 };
 std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1D& dlf, cudaStream_t st);

@@ -35,6 +35,20 @@ struct DevCSR {
     double* partial;          // kCsrMaxVec * nseg: segment sums, one block of nseg per vector
 };
 
+// The stepping operators (csr_step.cu) in slices: a warp's 32 / 2^b rows of bin
+// b, the rows of a bin sorted by length, with slot u of lane l of slice s at
+// (base[s] + u) 32 + l: entry u 2^b + l % 2^b of row rows[s 32 + l].  A warp
+// loads 32 adjacent entries at a time and its rows are of (nearly) one length.
+struct DevSliced {
+    int64_t m;
+    const int64_t* base;   // slices + 1, in slots of 32
+    const int32_t* rows;   // 32 per slice, -1 past the last row of a bin
+    const int32_t* col;    // -1: padding
+    const double* val;
+    int bin_block[kCsrBins + 1];  // blocks of kSliceWarps slices per bin
+};
+constexpr int kSliceWarps = 8;
+
 // ---- chosen form: matrix-free FP32 pencil apply, FP64 RK state --------------
 //
 // Solves with equal (D, k, n, scheme, kind) form a class.  A class keeps its

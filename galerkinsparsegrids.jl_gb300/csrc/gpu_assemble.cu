@@ -696,17 +696,95 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
 
 SGDG_BOUNDS_READER(asm_bounds_violations)
 
-std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
-                                        int per_lane, bool prune) {
+// slots of a slice: entry u VS + l % VS of its lane's row, padded with col -1
+__global__ void k_slice(const int64_t* __restrict__ base, const int32_t* __restrict__ rows, const int8_t* __restrict__ vs,
+                        int64_t slices, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                        const double* __restrict__ val, const uint8_t* __restrict__ dim, int32_t* __restrict__ scol,
+                        double* __restrict__ sval, uint8_t* __restrict__ sdim) {
+    const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int l = threadIdx.x & 31;
+    if (s >= slices) return;
+    const int VS = 1 << vs[s];
+    const int64_t r = rows[s * 32 + l], b = r >= 0 ? rowptr[r] : 0, e = r >= 0 ? rowptr[r + 1] : 0;
+    int64_t p = b + l % VS;
+    for (int64_t q = base[s]; q < base[s + 1]; q++, p += VS) {
+        const int64_t w = q * 32 + l;
+        scol[w] = p < e ? col[p] : -1;
+        sval[w] = p < e ? val[p] : 0.0;
+        if (dim) sdim[w] = p < e ? dim[p] : 0;
+    }
+}
+
+// The CSR A (m rows, host row pointers rp; dim: a byte per entry, or null) in
+// slices: the rows by length (counting sort, ascending rows within a length),
+// each bin's rows in slices of 32 / 2^b and its slices padded to whole blocks.
+std::unique_ptr<DeviceSliced> to_sliced(const DeviceCSR& A, const std::vector<int64_t>& rp, int64_t m, cudaStream_t st,
+                                        int per_lane = 0, const DevBuf* dim = nullptr) {
+    if (per_lane == 0) per_lane = csr_lane_entries(rp[m]);
+    int64_t most = 0;
+    for (int64_t r = 0; r < m; r++) most = std::max(most, rp[r + 1] - rp[r]);
+    std::vector<int64_t> at(most + 2, 0);
+    for (int64_t r = 0; r < m; r++) at[rp[r + 1] - rp[r] + 1]++;
+    for (int64_t l = 0; l <= most; l++) at[l + 1] += at[l];
+    std::vector<int32_t> order(m);
+    for (int64_t r = 0; r < m; r++) order[at[rp[r + 1] - rp[r]]++] = (int32_t)r;
+    auto S = std::make_unique<DeviceSliced>();
+    std::vector<int64_t> base(1, 0);
+    std::vector<int32_t> rows;
+    std::vector<int8_t> vs;
+    int64_t next = 0;
+    for (int b = 0; b < kCsrBins; b++) {
+        S->d.bin_block[b] = (int)(vs.size() / kSliceWarps);
+        const int per = 32 >> b;
+        while (next < m && csr_bin(rp[order[next] + 1] - rp[order[next]], per_lane) == b) {
+            int64_t slots = 0;
+            for (int i = 0; i < per; i++) {
+                int32_t r = -1;
+                if (next < m && csr_bin(rp[order[next] + 1] - rp[order[next]], per_lane) == b) r = order[next++];
+                if (r >= 0) slots = std::max(slots, (rp[r + 1] - rp[r] + (1 << b) - 1) >> b);
+                for (int l = 0; l < 1 << b; l++) rows.push_back(r);
+            }
+            base.push_back(base.back() + slots);
+            vs.push_back((int8_t)b);
+        }
+        while (vs.size() % kSliceWarps) {
+            rows.insert(rows.end(), 32, -1);
+            base.push_back(base.back());
+            vs.push_back((int8_t)b);
+        }
+        if ((int64_t)vs.size() / kSliceWarps > (int64_t(1) << 30))
+            throw Error(SGDG_EINVAL, "operator too large for the CSR kernels");
+    }
+    S->d.bin_block[kCsrBins] = (int)(vs.size() / kSliceWarps);
+    const int64_t slots = base.back() * 32;
+    S->base = upload(base, st);
+    S->rows = upload(rows, st);
+    S->col.alloc(sizeof(int32_t) * (size_t)slots);
+    S->val.alloc(sizeof(double) * (size_t)slots);
+    if (dim) S->extra.alloc((size_t)slots);
+    DevBuf dvs = upload(vs, st);
+    if (!vs.empty())
+        k_slice<<<grid_for((int64_t)vs.size() * 32), 256, 0, st>>>(
+            S->base.as<int64_t>(), S->rows.as<int32_t>(), dvs.as<int8_t>(), (int64_t)vs.size(), A.rowptr.as<int64_t>(),
+            A.col.as<int32_t>(), A.val.as<double>(), dim ? dim->as<uint8_t>() : nullptr, S->col.as<int32_t>(),
+            S->val.as<double>(), S->extra.as<uint8_t>());
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
+    S->d.m = m;
+    S->d.base = S->base.as<int64_t>();
+    S->d.rows = S->rows.as<int32_t>();
+    S->d.col = S->col.as<int32_t>();
+    S->d.val = S->val.as<double>();
+    return S;
+}
+
+// the operator's CSR arrays (rp: its row pointers), without bins
+static std::unique_ptr<DeviceCSR> assemble_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
+                                                    bool prune, std::vector<int64_t>& rp) {
     require_gpu();
     const int D = ix.D;
-    std::vector<int64_t> rp;
-    if (which >= 1 && which <= D) {
-        const LineTables T = line_tables(dlf, dlf.n + 1, false, prune);
-        auto A = line_operator(ix, T, which - 1, st, rp);
-        finish_device_csr(*A, rp, ix.N, st, per_lane);
-        return A;
-    }
+    if (which >= 1 && which <= D)
+        return line_operator(ix, line_tables(dlf, dlf.n + 1, false, prune), which - 1, st, rp);
     if (which != SGDG_OP_LAPLACIAN && which != SGDG_OP_WAVE_RHS)
         throw Error(SGDG_EINVAL, "operator selector must be 1..D, 0 (laplacian) or -1 (wave RHS)");
     const LineTables T = line_tables(dlf, dlf.n + 1, true, prune);
@@ -718,11 +796,8 @@ std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf,
         terms.push_back(sq.back().get());
     }
     auto L = merge_terms(terms, nullptr, ix.N, st, rp);
+    if (which == SGDG_OP_LAPLACIAN) return L;
     sq.clear();
-    if (which == SGDG_OP_LAPLACIAN) {
-        finish_device_csr(*L, rp, ix.N, st);
-        return L;
-    }
     const int64_t N = ix.N, nnzL = rp[N];
     std::vector<int64_t> wp(2 * N + 1);
     for (int64_t i = 0; i <= N; i++) wp[i] = i;
@@ -736,8 +811,29 @@ std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf,
     CK(cudaMemcpyAsync(W->col.as<int32_t>() + N, L->col.p, sizeof(int32_t) * (size_t)nnzL, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(W->val.as<double>() + N, L->val.p, sizeof(double) * (size_t)nnzL, cudaMemcpyDeviceToDevice, st));
     CK(cudaStreamSynchronize(st));
-    finish_device_csr(*W, wp, 2 * N, st);
+    rp = std::move(wp);
     return W;
+}
+
+std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st,
+                                        int per_lane) {
+    std::vector<int64_t> rp;
+    auto A = assemble_operator(ix, dlf, which, st, false, rp);
+    finish_device_csr(*A, rp, (int64_t)rp.size() - 1, st, per_lane);
+    return A;
+}
+
+std::unique_ptr<DeviceSliced> gpu_step_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st) {
+    std::vector<int64_t> rp;
+    const auto A = assemble_operator(ix, dlf, which, st, true, rp);
+    return to_sliced(*A, rp, (int64_t)rp.size() - 1, st);
+}
+
+std::unique_ptr<DeviceSliced> gpu_line_operator(const SparseIndex& ix, const LineTables& T, int d, cudaStream_t st) {
+    require_gpu();
+    std::vector<int64_t> rp;
+    const auto A = line_operator(ix, T, d, st, rp);
+    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesMulti);
 }
 
 std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1D& dlf, cudaStream_t st) {
@@ -753,30 +849,32 @@ std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1
     }
     const std::vector<int64_t> rp = scan_rows(rowlen, ix.N, st);
     auto R = std::make_unique<DeviceAdvection>();
-    DeviceCSR& A = R->A;
+    DeviceCSR A;
+    DevBuf dim;
     const size_t nnz = (size_t)rp[ix.N];
     A.rowptr = upload(rp, st);
     A.col.alloc(sizeof(int32_t) * nnz);
     A.val.alloc(sizeof(double) * nnz);
-    R->base.alloc(sizeof(double) * nnz);
-    R->dim.alloc(nnz);
+    dim.alloc(nnz);
     DevBuf cursor = upload(rp, st);
     for (int d = 0; d < ix.D; d++) {
         k_line_append<<<grid_for(ix.N), 256, 0, st>>>(S[d].args, cursor.as<int64_t>(), A.rowptr.as<int64_t>(),
-                                                      A.col.as<int32_t>(), R->base.as<double>(), R->dim.as<uint8_t>(), d);
+                                                      A.col.as<int32_t>(), A.val.as<double>(), dim.as<uint8_t>(), d);
         CK(cudaGetLastError());
     }
-    finish_device_csr(A, rp, ix.N, st);
-    CK(cudaStreamSynchronize(st));  // S's tables and the cursor are freed on return
+    auto sliced = to_sliced(A, rp, ix.N, st, 0, &dim);  // waits for the stream: S's tables are freed on return
+    R->A = std::move(*sliced);
+    R->slots = (int64_t)(R->A.col.bytes / sizeof(int32_t));
+    R->base.alloc(sizeof(double) * (size_t)R->slots);
+    CK(cudaMemcpyAsync(R->base.p, R->A.val.p, sizeof(double) * (size_t)R->slots, cudaMemcpyDeviceToDevice, st));
     return R;
 }
 
 cudaError_t DeviceAdvection::scale(int D, const double* s, cudaStream_t st) {
     Factors f{};
     for (int d = 0; d < D; d++) f.s[d] = s[d];
-    if (A.d.nnz > 0)
-        k_scale_entries<<<std::min(grid_for(A.d.nnz), 4096), 256, 0, st>>>(base.as<double>(), dim.as<uint8_t>(), f, A.d.nnz,
-                                                                          A.val.as<double>());
+    k_scale_entries<<<std::min(grid_for(slots), 4096), 256, 0, st>>>(base.as<double>(), A.extra.as<uint8_t>(), f, slots,
+                                                                    A.val.as<double>());
     return cudaGetLastError();
 }
 

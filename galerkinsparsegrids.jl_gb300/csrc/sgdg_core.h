@@ -222,6 +222,8 @@ struct LineTables {
     std::vector<double> val;
 };
 LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune = false);
+// The same of a 1D transform T1 (its leading blocks, entries whose cells nest).
+LineTables line_tables(const CSR& T1, int k, int levels);
 
 void set_error(const std::string& msg);
 }  // namespace sgdg
