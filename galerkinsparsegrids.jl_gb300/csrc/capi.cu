@@ -40,6 +40,8 @@ cudaError_t launch_csr_spmv_multi(const DevCSR& A, int nv, const double* x, int6
 cudaError_t launch_vlasov_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                                  cudaStream_t st);
 cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, int* nonfinite, cudaStream_t st);
+cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, double* y, int* seen, int call,
+                         cudaStream_t st);
 cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x, double* y, cudaStream_t st);
 cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                           cudaStream_t st);
@@ -117,6 +119,30 @@ struct sgdg_op {
         auto it = step_dev.find(which);
         if (it == step_dev.end()) it = step_dev.emplace(which, gpu_step_operator(ix, *dlf, which, stream)).first;
         return it->second->d;
+    }
+    // Applications of an operator of kApplyPruned entries or more go through the
+    // pruned one (us per application, whole and pruned: Laplacian 2D k=3 n=7, 1.3
+    // M entries, 8.3 and 8.9; 4D k=2 n=6, 1.6 M, 10.3 and 8.9; 3D k=3 n=6, 2.2 M,
+    // 11.5 and 9.1; 3D k=3 n=7, 8.8 M, 28.3 and 9.0; 3D k=4 n=7, 27.8 M, 82.9 and
+    // 18.5; below 9 the time is the caller's, two launches for one), and where an element of x is not finite through the whole one
+    // after it (k_apply_whole).  Each call leaves its number in a word of its
+    // own among kApplyCalls: calls on other streams may still be in flight.
+    static constexpr int64_t kApplyPruned = 3 << 19;
+    static constexpr int kApplyCalls = 1024;
+    DevBuf apply_seen;
+    int apply_call = 0;
+    cudaError_t apply(int which, const double* x, double* y, cudaStream_t st) {
+        const DevCSR& A = device(which);
+        if (!prunes() || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
+        if (!apply_seen.p) {
+            stepping(which);
+            apply_seen.alloc(sizeof(int) * kApplyCalls);
+            CK(cudaMemsetAsync(apply_seen.p, 0, apply_seen.bytes, stream));
+            CK(cudaStreamSynchronize(stream));
+        }
+        const DevSliced& P = stepping(which);
+        apply_call = apply_call == INT32_MAX ? 1 : apply_call + 1;
+        return launch_apply(P, A, x, y, apply_seen.as<int>() + apply_call % kApplyCalls, apply_call, st);
     }
     // the whole operator, the pruned one making room for it where there is none
     const DevCSR& whole(int which) {
@@ -591,8 +617,7 @@ int sgdg_op_export_csr(sgdg_op* op, int which, int64_t* rowptr, int32_t* col, do
 
 static void apply_device_impl(sgdg_op* op, int which, int method, const double* x, double* y, cudaStream_t st) {
     if (method == SGDG_METHOD_PLAIN) {
-        const DevCSR& A = op->device(which);
-        CK(launch_csr_spmv(A, x, y, st));
+        CK(op->apply(which, x, y, st));
         return;
     }
     if (method != SGDG_METHOD_MATFREE) throw Error(SGDG_EINVAL, "method must be PLAIN (0) or MATFREE (1)");

@@ -384,6 +384,42 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
     block_rows<NV>(A, blockIdx.x, x + o, stride, SweepOut<NV>{y + o, stride, nonfinite});
 }
 
+// One application y = A x with the pruned operator; an element of x that is not
+// finite leaves `call` in *seen, for k_apply_whole
+struct ApplyOut {
+    const double* x;
+    double* y;
+    int* seen;
+    int call;
+    __device__ __forceinline__ void one(int64_t row, int, double s) const {
+        y[row] = s;
+        if (not_finite(__ldca(x + row))) *seen = call;
+    }
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[1]) const { one(row, 0, s[0]); }
+};
+__global__ void __launch_bounds__(256, 4) k_apply(DevSliced A, const double* x, double* y, int* seen, int call) {
+    block_rows<1>(A, blockIdx.x, x, 1, ApplyOut{x, y, seen, call});
+}
+
+// y = A x with the whole operator, where this call's k_apply met an element of
+// x that is not finite: the blocks share its row blocks, a warp takes a long row
+__global__ void __launch_bounds__(256) k_apply_whole(DevCSR A, const double* x, double* y, const int* seen, int call) {
+    pdl_wait();
+    if (*reinterpret_cast<const volatile int*>(seen) != call) return;
+    const SweepOut<1> out{y, 1, nullptr};
+    for (int64_t rb = blockIdx.x; rb < A.bin_block[kCsrBins]; rb += gridDim.x) block_rows<1>(A, rb, x, 1, out);
+    const int lane = threadIdx.x & 31;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < A.nlong;
+         i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t row = A.long_row[i], b = A.rowptr[row], e = A.rowptr[row + 1];
+        CsrAhead ahead;
+        csr_fetch<32>(A, b + lane, e, ahead);
+        double s[1];
+        row_sum<32, 1>(A, b, e, ahead, x, lane, 1, s);
+        if (lane == 0 && SGDG_IN(row, A.m)) y[row] = s[0];
+    }
+}
+
 // The P derivatives of one vector, interleaved: y[i P + d] = (D_d x)_i; blockIdx.y: d.
 struct DerivativeSet {
     DevSliced d[8];
@@ -579,6 +615,15 @@ cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, 
         launch_dependent(k_sweep<2>, dim3(nb, P / 2), st, A, x, y, P, nonfinite);
     else
         launch_dependent(k_sweep<1>, dim3(nb, P), st, A, x, y, P, nonfinite);
+    return cudaGetLastError();
+}
+
+// y = A x, P the pruned A; *seen is not `call` before
+cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, double* y, int* seen, int call,
+                         cudaStream_t st) {
+    if (P.bin_block[kCsrBins] == 0) return cudaSuccess;
+    launch_dependent(k_apply, (unsigned)P.bin_block[kCsrBins], st, P, x, y, seen, call);
+    launch_dependent(k_apply_whole, 152u, st, A, x, y, (const int*)seen, call);
     return cudaGetLastError();
 }
 

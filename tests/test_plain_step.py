@@ -131,3 +131,58 @@ def test_stepping_at_a_memory_limit(sgdg):
         assert e.value.code == 2 and torch.equal(three, y)
     finally:
         sgdg.set_hbm_budget(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,k,n,which", [(4, 2, 6, 0), (2, 3, 7, 0), (1, 3, 10, 0), (3, 3, 6, -1)])
+def test_application_with_the_pruned_operator(sgdg, D, k, n, which):
+    # either side of the size from which applications go through the pruned
+    # operator (4D: just above, 2D: just below; 1D: rows of 3072 entries).  The
+    # entries dropped are 2e-12 of the largest and the sums as long as a line:
+    # 1e-10 of the result for random vectors, whose result the largest entries make
+    op = sgdg.SparseGridOperator(D, k, n)
+    A = op.csr(which)
+    x = np.random.default_rng(D).standard_normal(A.shape[0])
+    ref = A @ x
+    assert np.linalg.norm(op.apply(x, which) - ref) <= 1e-10 * np.linalg.norm(ref)
+    for where, value in ((0, np.nan), (A.shape[0] - 1, np.inf), (A.shape[0] // 3, -np.inf)):
+        z = x.copy()
+        z[where] = value
+        with np.errstate(all="ignore"):
+            bad = A @ z
+        y = op.apply(z, which)
+        assert np.array_equal(np.isfinite(y), np.isfinite(bad)) and np.array_equal(np.isnan(y), np.isnan(bad))
+        fin = np.isfinite(bad)
+        assert np.linalg.norm(y[fin] - bad[fin]) <= 1e-10 * np.linalg.norm(ref)
+    assert np.linalg.norm(op.apply(x, which) - ref) <= 1e-10 * np.linalg.norm(ref)  # and finite data again
+
+
+@pytest.mark.gpu
+def test_applications_in_a_graph_and_on_two_streams(sgdg):
+    import torch
+    op = sgdg.SparseGridOperator(4, 2, 6)
+    A = op.csr(0)
+    x = torch.tensor(np.random.default_rng(1).standard_normal((2, op.N)), device="cuda")
+    y = torch.zeros_like(x)
+    op.apply_device(x[0].data_ptr(), y[0].data_ptr(), which=0)  # assembles
+    torch.cuda.synchronize()
+    ref = np.stack([A @ v for v in x.cpu().numpy()])
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for i in range(40):
+        op.apply_device(x[i % 2].data_ptr(), y[i % 2].data_ptr(), which=0, stream=streams[i % 2].cuda_stream)
+    torch.cuda.synchronize()
+    assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-10 * np.linalg.norm(ref)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        op.apply_device(x[0].data_ptr(), y[0].data_ptr(), which=0, stream=streams[0].cuda_stream)
+    for value in (1.0, float("nan"), 2.0):
+        x[0, 5] = value
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            ref = A @ x[0].cpu().numpy()
+        got = y[0].cpu().numpy()
+        fin = np.isfinite(ref)
+        assert np.array_equal(np.isfinite(got), fin)
+        assert np.linalg.norm(got[fin] - ref[fin]) <= 1e-10 * np.linalg.norm(ref[fin])
