@@ -9,11 +9,13 @@
 //   level l:  v = sqrt(2^l) h_m(2^l x - (2 cell - 1)),  h the multiwavelet
 //             piece for y < 0 or y >= 0, zero for |y| > 1 (array2poly,
 //             src/1d_dg_functions.jl:15-27).
-// Points are batched: one warp per point.  The lanes first tabulate the k 1D
+// Two kernels.  k_evaluate, one warp per point: the lanes first tabulate the k 1D
 // values and the cell of every (dimension, level) in shared memory, then
 // split the level blocks among themselves and contract each block's k^D
-// coefficients one dimension at a time; a shuffle tree sums the lanes.  All
-// arithmetic is FP64, like the reference.  A coordinate below 0 (or NaN)
+// coefficients one dimension at a time; a shuffle tree sums the lanes.  For
+// k <= 5 and kPencilPoints points or more, k_lines first sums the levels along
+// dimension 1 once for all points, and k_evaluate_pencils adds up one block per
+// pencil (see there).  All arithmetic is FP64, like the reference.  A coordinate below 0 (or NaN)
 // has no cell in the reference (an out-of-range index there) and is reported
 // as SGDG_EINVAL; above 1 the last cell is used and |y| > 1 gives zero, as
 // in the reference.
@@ -140,6 +142,190 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
     }
 }
 
+// ---- many points ------------------------------------------------------------
+// The hierarchical functions of a line along dimension 1 (levels 1..lmax, equal
+// in everything else) are piecewise polynomials on its 2^(lmax-1) finest
+// pieces, so the line's k 2^(lmax-1) coefficients can be exchanged for as many
+// Legendre coefficients on the pieces (an orthonormal change of basis: Alpert's
+// two-scale relations, coarse to fine).  A point then meets one block of k^D
+// numbers per pencil -- level tuple of the other dimensions -- instead of one
+// per level block: 36 instead of 120 for 3D n=7, and the FP64 operations, which
+// bound k_evaluate (61 % of that pipe's peak, 3.50 ms for 2^18 points at k=3),
+// fall as much (0.95 ms, of which the FP64 pipe needs 0.75).  A block's numbers are padded to a multiple of 32 bytes and
+// loaded 32 bytes at a time: the lanes of a warp are 32 points in blocks of
+// their own, so a load costs as many L1 accesses as it has lanes, whatever its
+// width.
+struct Pencils {
+    int D, n, np;
+    int inner, pad, outer;   // k^min(D,3), the same rounded up to 4, k^(D-3) (1 for D <= 3)
+    const int32_t* lmax;     // per pencil: levels along dimension 1
+    const int64_t* base;     // first number of its blocks
+    const int8_t* levels;    // D - 1 levels of the other dimensions, 1-based
+    const int64_t* item;     // first item (piece, cell and mode of the others) of k_lines; np + 1
+    const int32_t* lev_off;  // per pencil n + 1 offsets of its level blocks
+    const double* two;       // H_0, G_0, H_1, G_1 (k x k each): child b's Legendre coefficients from the
+                             // parent's and its wavelets'
+    const double* pieces;    // as EvalShape
+};
+
+// One item: the k Legendre coefficients of a piece, from the line's root down.
+template <int K>
+__global__ void __launch_bounds__(256)
+    k_lines(Pencils S, const double* __restrict__ c, int64_t kD, double* __restrict__ out, int* nonfinite) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= S.item[S.np]) return;
+    int lo = 0, hi = S.np - 1;
+    while (lo < hi) {  // last pencil with item <= e
+        const int mid = (lo + hi + 1) >> 1;
+        if (S.item[mid] <= e) lo = mid; else hi = mid - 1;
+    }
+    const int lmax = S.lmax[lo];
+    const int32_t* off = S.lev_off + (int64_t)lo * (S.n + 1);
+    const int64_t km = kD / K;  // modes of the other dimensions, fastest
+    const int64_t r = (e - S.item[lo]) / km, mo = (e - S.item[lo]) - r * km;
+    const int64_t j = r & ((1ll << (lmax - 1)) - 1), cl = r >> (lmax - 1);  // piece, cells of the others
+    double s[K];
+#pragma unroll
+    for (int m = 0; m < K; m++) s[m] = c[off[0] + kD * cl + K * mo + m];
+    bool bad = false;
+    for (int t = 1; t < lmax; t++) {
+        const int64_t ct = t > 1 ? j >> (lmax - t) : 0;
+        const double* d = c + off[t] + kD * (ct + (cl << (t > 1 ? t - 1 : 0))) + K * mo;
+        const double* H = S.two + ((j >> (lmax - 1 - t)) & 1) * 2 * K * K;
+        double w[K], x[K];
+#pragma unroll
+        for (int m = 0; m < K; m++) w[m] = d[m];
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            double v = 0.0;
+#pragma unroll
+            for (int m = 0; m < K; m++) v = fma(__ldg(H + i * K + m), s[m], fma(__ldg(H + K * K + i * K + m), w[m], v));
+            x[i] = v;
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) s[i] = x[i];
+    }
+    // within its block: the modes of dimensions 1..3 (padded), then the others
+    const int in = S.inner / K;
+    double* o = out + S.base[lo] + (int64_t)S.pad * S.outer * (j + (cl << (lmax - 1))) + S.pad * (mo / in) + K * (mo % in);
+#pragma unroll
+    for (int m = 0; m < K; m++) {
+        o[m] = s[m];
+        bad = bad || (__double2hiint(s[m]) & 0x7ff00000) == 0x7ff00000;
+    }
+    if (bad) *nonfinite = 1;
+}
+
+constexpr int kPencilPts = 32;    // points of a CTA, one per lane
+constexpr int kPencilParts = 4;   // warps that share them, every fourth pencil each
+
+// Values at points: a CTA tabulates the 1D values of its points in shared
+// memory ([entry][point]), then each warp adds up its pencils.  Bounds: FP64
+// pipe (k^D + k^(D-1) + ... operations per pencil and point, a quarter of it
+// the tables), then the gathers.
+template <int K, int DI>
+__global__ void __launch_bounds__(kPencilPts* kPencilParts)
+    k_evaluate_pencils(Pencils S, const double* __restrict__ G, int64_t npts, const double* __restrict__ xs,
+                       double* __restrict__ out, int* err) {
+    extern __shared__ double esm[];
+    constexpr int PT = kPencilPts, PAD = ((DI == 1 ? K : DI == 2 ? K * K : K * K * K) + 3) / 4 * 4;
+    const int nl = S.n + 1, D = S.D;
+    double* tab = esm;                                              // [(d nl + l) K + m][point]
+    double* part = tab + (size_t)D * nl * K * PT;                   // [warp][point]
+    int* cell = reinterpret_cast<int*>(part + kPencilParts * PT);   // [d][point]: floor(2^n x)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t p = (int64_t)blockIdx.x * PT + lane;
+    for (int e = warp; e < D * nl; e += kPencilParts) {
+        const int d = e / nl, l = e - d * nl;  // l: 0-based level; dimension 1: pieces of 2^-l
+        const double x = p < npts ? xs[p * D + d] : 0.0;
+        double v[K];
+#pragma unroll
+        for (int m = 0; m < K; m++) v[m] = 0.0;
+        if (!(x >= 0.0)) {
+            atomicExch(err, 1);
+        } else {
+            const int cells = d == 0 ? l : l > 1 ? l - 1 : 0;  // log2
+            int c = 0;  // 0-based
+            if (cells > 0) c = x >= 1.0 ? (1 << cells) - 1 : (int)floor(pow2(cells) * x);
+            double y, scale;
+            const double* pc;
+            if (d == 0 || l == 0) {
+                y = pow2(cells + 1) * x - (double)(2 * c + 1);
+                scale = 1.4142135623730951 * ((cells & 1) ? 1.4142135623730951 * pow2(cells >> 1) : pow2(cells >> 1));
+                pc = S.pieces;
+            } else {
+                y = pow2(l) * x - (double)(2 * c + 1);
+                scale = (l & 1) ? 1.4142135623730951 * pow2(l >> 1) : pow2(l >> 1);
+                pc = S.pieces + (y < 0.0 ? 1 : 2) * K * K;
+            }
+            if (fabs(y) <= 1.0)
+#pragma unroll
+                for (int m = 0; m < K; m++) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int i = K - 1; i >= 0; i--) s = fma(s, y, __ldg(pc + m * K + i));
+                    v[m] = scale * s;
+                }
+        }
+#pragma unroll
+        for (int m = 0; m < K; m++) tab[(e * K + m) * PT + lane] = v[m];
+        if (l == 0) cell[d * PT + lane] = !(x < 1.0) ? (1 << S.n) - 1 : x > 0.0 ? (int)floor(pow2(S.n) * x) : 0;
+    }
+    __syncthreads();
+    double acc = 0.0;
+    for (int q = warp; q < S.np; q += kPencilParts) {
+        const int lm = S.lmax[q];
+        const int8_t* L = S.levels + q * (D - 1);
+        int64_t cl = 0;
+        int sh = lm - 1;
+        for (int d = 1; d < D; d++) {
+            const int lc = L[d - 1] > 2 ? L[d - 1] - 2 : 0;
+            cl += (int64_t)(cell[d * PT + lane] >> (S.n - lc)) << sh;
+            sh += lc;
+        }
+        const double* g = G + S.base[q] + (int64_t)PAD * S.outer * ((cell[lane] >> (S.n - (lm - 1))) + cl);
+        double v0[K], v1[K], v2[K];
+#pragma unroll
+        for (int m = 0; m < K; m++) {
+            v0[m] = tab[((lm - 1) * K + m) * PT + lane];
+            if (DI > 1) v1[m] = tab[((nl + L[0] - 1) * K + m) * PT + lane];
+            if (DI > 2) v2[m] = tab[((2 * nl + L[1] - 1) * K + m) * PT + lane];
+        }
+        for (int o = 0; o < S.outer; o++) {
+            double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll
+            for (int u = 0; u < PAD; u += 4) {
+                double t[4];
+                asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                    : "=d"(t[0]), "=d"(t[1]), "=d"(t[2]), "=d"(t[3]) : "l"(g + (int64_t)o * PAD + u));
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int at = u + i, m0 = at % K, m1 = at / K % K, m2 = at / (K * K);
+                    if (at >= (DI == 1 ? K : DI == 2 ? K * K : K * K * K)) continue;
+                    s0 = m0 ? fma(v0[m0], t[i], s0) : v0[0] * t[i];
+                    if (DI > 1 && m0 == K - 1) {
+                        s1 = m1 ? fma(v1[m1], s0, s1) : v1[0] * s0;
+                        if (DI > 2 && m1 == K - 1) s2 = m2 ? fma(v2[m2], s1, s2) : v2[0] * s1;
+                    }
+                }
+            }
+            double r = DI == 1 ? s0 : DI == 2 ? s1 : s2;
+            if (S.outer > 1) {
+                int mo = o;
+                for (int d = 3; d < D; d++, mo /= K) r *= tab[((d * nl + L[d - 1] - 1) * K + mo % K) * PT + lane];
+            }
+            acc += r;
+        }
+    }
+    part[warp * PT + lane] = acc;
+    __syncthreads();
+    if (warp == 0 && p < npts) {
+        double s = 0.0;
+        for (int w = 0; w < kPencilParts; w++) s += part[w * PT + lane];
+        out[p] = s;
+    }
+}
+
 // Sum over terms of separable products (tensor_construct,
 // src/tensor_construct.jl:19-62, and sums of Fourier modes): coefficient i
 // of the D-dim vector is  sum_t amp_t * part_t( e^{i phi_t} prod_d Z_td[i_d] )
@@ -196,12 +382,130 @@ struct EvalTables {
     SparseIndex ix;
     DevBuf levels, lev_off, pieces;
     size_t smem = 0;
+    // the pencils along dimension 1 (k <= 5), built with the first call that uses them
+    std::mutex mu;
+    DevBuf lmax, base, plevels, item, plev_off, two;
+    Pencils P{};
+    int64_t items = 0, numbers = 0;  // of k_lines; of its output
+    size_t psmem = 0;
 };
+
+constexpr int kPencilMaxK = 5;
+// From these counts of points and of products with a coefficient on, the pencils
+// pay for k_lines (us per call, blocks and pencils: 3D k=3 n=7 64 and 69 at 1000
+// points, 90 and 69 at 4000, 3495 and 947 at 2^18; 4D k=3 n=4 90 and 104, 138 and
+// 105, 6579 and 2190; 2D k=2 n=6 39 and 41 at 4000, 64 and 46 at 16000, 524 and
+// 165; 1D k=3 n=8 39 and 45, 55 and 54, 448 and 141).
+constexpr int64_t kPencilPoints = 4096, kPencilTerms = 1 << 20;
+
+// H_b[i][m] = <child b's Legendre function i, the parent's m>, G_b the same with
+// the wavelets: 2^(-1/2) int leg_i(z) p_m((z + s) / 2) dz, s = 2b - 1, over
+// [-1, 1], p_m the parent's polynomial on that half.
+std::vector<double> two_scale(int k) {
+    std::vector<double> out((size_t)4 * k * k);
+    for (int b = 0; b < 2; b++)
+        for (int g = 0; g < 2; g++)
+            for (int m = 0; m < k; m++) {
+                const HierFn f = make_hier_fn(k, g, 1, m + 1);
+                const double* p = g && b ? f.right : f.left;
+                std::vector<double> q(k, 0.0);  // p((z + s) / 2) in z, by Horner
+                for (int i = k - 1; i >= 0; i--) {
+                    std::vector<double> t(k, 0.0);
+                    for (int a = 0; a < k; a++) {
+                        t[a] += 0.5 * (2 * b - 1) * q[a];
+                        if (a + 1 < k) t[a + 1] += 0.5 * q[a];
+                    }
+                    t[0] += p[i];
+                    q = t;
+                }
+                for (int i = 0; i < k; i++) {
+                    const HierFn l = make_hier_fn(k, 0, 1, i + 1);
+                    double v = 0.0;
+                    for (int a = 0; a < k; a++)
+                        for (int c = 0; c < k; c++)
+                            if ((a + c) % 2 == 0) v += l.left[a] * q[c] * 2.0 / (a + c + 1);
+                    out[(size_t)(2 * b + g) * k * k + i * k + m] = std::sqrt(0.5) * v;
+                }
+            }
+    return out;
+}
+
+const Pencils& eval_pencils(EvalTables& T) {
+    std::lock_guard<std::mutex> g(T.mu);
+    if (T.P.np > 0) return T.P;
+    const SparseIndex& ix = T.ix;
+    const int D = ix.D, k = ix.k, n = ix.n;
+    Pencils P{};
+    P.D = D;
+    P.n = n;
+    P.inner = 1;
+    P.outer = 1;
+    for (int d = 0; d < D; d++) (d < 3 ? P.inner : P.outer) *= k;
+    P.pad = (P.inner + 3) / 4 * 4;
+    std::vector<int32_t> lmax, off;
+    std::vector<int64_t> base, item(1, 0);
+    std::vector<int8_t> lev;
+    int64_t numbers = 0;
+    int L[kDMax];
+    for (int b = 0; b < ix.nlev; b++) {
+        const int* Lb = &ix.levels[(size_t)b * D];
+        if (Lb[0] != 1) continue;
+        for (int d = 0; d < D; d++) L[d] = Lb[d];
+        int lm = 0;
+        for (int l = 1; l <= n + 1; l++) {
+            L[0] = l;
+            if (ix.cut(L)) {
+                off.push_back(0);
+                continue;
+            }
+            off.push_back((int32_t)ix.lev_off[ix.lookup_level(L)]);
+            lm = l;
+        }
+        for (int d = 1; d < D; d++) lev.push_back((int8_t)Lb[d]);
+        lmax.push_back(lm);
+        base.push_back(numbers);
+        const int64_t blocks = ix.lev_cells[b] << (lm - 1);  // finest pieces x cells of the others
+        numbers += blocks * P.pad * P.outer;
+        item.push_back(item.back() + blocks * (ix.kD / k));
+    }
+    T.lmax = upload(lmax, nullptr);
+    T.base = upload(base, nullptr);
+    T.plevels = upload(lev, nullptr);
+    T.item = upload(item, nullptr);
+    T.plev_off = upload(off, nullptr);
+    T.two = upload(two_scale(k), nullptr);
+    CK(cudaStreamSynchronize(nullptr));
+    P.lmax = T.lmax.as<int32_t>();
+    P.base = T.base.as<int64_t>();
+    P.levels = T.plevels.as<int8_t>();
+    P.item = T.item.as<int64_t>();
+    P.lev_off = T.plev_off.as<int32_t>();
+    P.two = T.two.as<double>();
+    P.pieces = T.pieces.as<double>();
+    T.items = item.back();
+    T.numbers = numbers;
+    T.psmem = sizeof(double) * kPencilPts * ((size_t)D * (n + 1) * k + kPencilParts) + sizeof(int) * kPencilPts * D;
+    P.np = (int)lmax.size();
+    T.P = P;
+    return T.P;
+}
+
+template <int K>
+cudaError_t launch_pencils(const EvalTables& T, const Pencils& P, const double* coeffs, int64_t npts, const double* xs,
+                           double* out, double* G, int* err, cudaStream_t st) {
+    k_lines<K><<<(unsigned)((T.items + 255) / 256), 256, 0, st>>>(P, coeffs, T.ix.kD, G, err + 1);
+    auto kernel = P.D == 1 ? k_evaluate_pencils<K, 1> : P.D == 2 ? k_evaluate_pencils<K, 2> : k_evaluate_pencils<K, 3>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return e;
+    kernel<<<(unsigned)((npts + kPencilPts - 1) / kPencilPts), kPencilPts * kPencilParts, T.psmem, st>>>(P, G, npts, xs, out,
+                                                                                                      err);
+    return cudaGetLastError();
+}
 
 std::mutex g_eval_mu;
 std::map<std::tuple<int, int, int, int>, std::unique_ptr<EvalTables>> g_eval;
 
-const EvalTables& eval_tables(int D, int k, int n, int scheme) {
+EvalTables& eval_tables(int D, int k, int n, int scheme) {
     std::lock_guard<std::mutex> g(g_eval_mu);
     auto key = std::make_tuple(D, k, n, scheme);
     auto f = g_eval.find(key);
@@ -226,7 +530,7 @@ const EvalTables& eval_tables(int D, int k, int n, int scheme) {
     T->pieces = upload(pc, nullptr);
     CK(cudaStreamSynchronize(nullptr));
     T->smem = sizeof(double) * (size_t)kEvalWarps * ((size_t)D * (n + 1) * k + (size_t)D * (n + 1));
-    const EvalTables& r = *T;
+    EvalTables& r = *T;
     g_eval.emplace(key, std::move(T));
     return r;
 }
@@ -234,8 +538,30 @@ const EvalTables& eval_tables(int D, int k, int n, int scheme) {
 void evaluate_impl(int D, int k, int n, int scheme, const double* coeffs, int64_t npts, const double* xs,
                    double* out, cudaStream_t st) {
     if (npts < 0) throw Error(SGDG_EINVAL, "npts must be >= 0");
-    const EvalTables& T = eval_tables(D, k, n, scheme);
+    EvalTables& T = eval_tables(D, k, n, scheme);
     if (npts == 0) return;
+    if (k <= kPencilMaxK && npts >= kPencilPoints && npts * T.ix.nlev * T.ix.kD >= kPencilTerms &&
+        npts < (int64_t(1) << 31) * kPencilPts) {
+        const Pencils& P = eval_pencils(T);
+        DevBuf work;
+        if (T.psmem <= 200 * 1024) try {
+                work.alloc(sizeof(double) * (size_t)T.numbers + 2 * sizeof(int));
+            } catch (const Error&) {  // no room: k_evaluate needs none
+            }
+        if (work.p) {
+            int* err = reinterpret_cast<int*>(work.as<double>() + T.numbers);
+            CK(cudaMemsetAsync(err, 0, 2 * sizeof(int), st));
+            auto launch = k == 1 ? launch_pencils<1> : k == 2 ? launch_pencils<2> : k == 3 ? launch_pencils<3>
+                        : k == 4 ? launch_pencils<4> : launch_pencils<5>;
+            CK(launch(T, P, coeffs, npts, xs, out, work.as<double>(), err, st));
+            int h[2] = {0, 0};
+            CK(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            if (h[0]) throw Error(SGDG_EINVAL, "a point coordinate is below 0 or NaN (no cell contains it)");
+            if (!h[1]) return;
+            // a coefficient that is not finite: block by block, as the sum over levels spreads it
+        }
+    }
     if (T.smem > 200 * 1024) throw Error(SGDG_EUNSUPPORTED, "point tables exceed shared memory");
     static bool configured = false;
     if (!configured) {
