@@ -168,7 +168,8 @@ constexpr int kMFThreadsLog2 = 8;
 static_assert(1 << kMFThreadsLog2 == kMFThreads, "kMFThreadsLog2");
 constexpr int kSpinLimit = 1 << 22;  // polls of a dependency counter before giving up
 
-// Tile shape of the pass tiles of one (D, k), chosen by the autotuner:
+// Tile shape of the pass tiles of one (D, k), chosen by the autotuner (without
+// a tuned shape the width follows the items per phase, mf_auto_wlog):
 // a tile has cpt * max(1, kMFThreads / nrb) * 2^wlog columns (at least cpt; nrb =
 // row blocks of the pencil), and the row blocks of levels <= lmax - coop are
 // warp-cooperative.  Narrower tiles need less shared memory (more CTAs per
@@ -178,7 +179,7 @@ struct MFTile {
     int coop = 4;
 };
 constexpr int kMFWlogMin = -2, kMFWlogMax = 3;
-MFTile mf_tile(int D, int k);                 // tuned shape, or the default
+MFTile mf_tile(int D, int k);                 // tuned shape, or the default {0, 4}
 bool mf_tile_tuned(int D, int k);
 void mf_set_tile(int D, int k, const MFTile& t);
 void mf_clear_tiles();

@@ -46,6 +46,11 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem_src) : "memory");
 }
 
+__device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 
@@ -97,7 +102,7 @@ __device__ __forceinline__ void wait_counter(const int* ctr, int need, int* err)
             atomicExch(err, 1);
             break;
         }
-        __nanosleep(100);
+        __nanosleep(20);
     }
 }
 
@@ -201,7 +206,6 @@ __device__ void pass_tile(const MFItem& it, const MFClass& C, const OpTable& T, 
                     xc[row * W] = 0.f;
             }
         });
-        cp_async_wait_all();
     } else {
         // a scratch vector written in this launch by other SMs: L2 loads (.cg)
         const float* __restrict__ vin = C.vbase + (size_t)it.src * C.vstride;
@@ -239,6 +243,7 @@ __device__ void pass_tile(const MFItem& it, const MFClass& C, const OpTable& T, 
             }
         });
     }
+    cp_async_wait_all();  // the gather, and the operator table where it was copied for this item
     __syncthreads();
     const int lwq = lw - (CPT == 4 ? 2 : 1);
     const int rlong = it.rlong;  // row blocks of levels <= lmax - coop (tile shape)
@@ -442,7 +447,9 @@ __global__ void __launch_bounds__(kMFThreads, 3)
     __shared__ MFItem s_it;
     __shared__ MFClass s_cls;
     __shared__ int s_cls_id;   // class in s_cls (-1: none)
-    __shared__ const int32_t* s_cached;  // the table in shared memory, by its global row pointers (null: none)
+    // the table in shared memory, by its global row pointers (null: none): as of
+    // the last item, and including the current one's copy
+    __shared__ const int32_t *s_cached, *s_copied;
     const int tid = threadIdx.x;
     unsigned long long pol;  // L2 evict-first policy of the FP64 state streams
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -451,7 +458,7 @@ __global__ void __launch_bounds__(kMFThreads, 3)
     static_assert(kItemWords <= 32, "item fits one warp");
     if (tid == 0) {
         s_cls_id = -1;
-        s_cached = nullptr;
+        s_cached = s_copied = nullptr;
     }
     if (tid == 32) s_item = atomicAdd(ctr, 1);
     int done = -1;  // thread 0: completion counter of the last finished item
@@ -508,13 +515,16 @@ __global__ void __launch_bounds__(kMFThreads, 3)
             int* trow = reinterpret_cast<int*>(smem);
             int* tent = trow + tn[0];
             float* tval = smem + (((tn[0] + tn[1]) * 4 + 15) / 16) * 4;
-            if (s_cached != T.rowptr) {  // copy the table (uniform branch; classes of one (k, n) share it)
-                for (int i = tid; i < tn[0]; i += kMFThreads) trow[i] = T.rowptr[i];
-                for (int i = tid; i < tn[1]; i += kMFThreads) tent[i] = T.ent[i];
-                for (int i = tid; i < tn[2] / 4; i += kMFThreads)
-                    reinterpret_cast<float4*>(tval)[i] = reinterpret_cast<const float4*>(T.val)[i];
-                __syncthreads();
-                if (tid == 0) s_cached = T.rowptr;
+            if (s_cached != T.rowptr) {
+                // copy the table (uniform branch; classes of one (k, n) share it);
+                // it arrives with the gather, under the offset tables and the
+                // waits (the uneven batch, whose items alternate between tables:
+                // 259 -> 251 us per step against a copy of its own)
+                for (int i = tid; i < tn[0]; i += kMFThreads) cp_async4(smem + i, reinterpret_cast<const float*>(T.rowptr) + i);
+                for (int i = tid; i < tn[1]; i += kMFThreads)
+                    cp_async4(smem + tn[0] + i, reinterpret_cast<const float*>(T.ent) + i);
+                for (int i = tid; i < tn[2] / 4; i += kMFThreads) cp_async16(tval + 4 * i, T.val + 4 * i);
+                if (tid == 0) s_copied = T.rowptr;
             }
             T = OpTable{trow, tent, tval};
         }
@@ -544,6 +554,7 @@ __global__ void __launch_bounds__(kMFThreads, 3)
                 if (tid == 32) s_item = nitems;  // unreachable (k in 1..5): stop
                 break;
         }
+        if (tid == 0) s_cached = s_copied;  // every thread has compared it
     }
 }
 

@@ -424,6 +424,40 @@ void MFEngine::plan() {
     dirty_ = false;
 }
 
+// Tile width factor 2^w (w = 0, -1, -2) of the classes without a tuned shape.  A
+// phase's tiles run side by side and the next phase waits for all of them, so
+// where a step holds fewer items per phase of its longest chain than the GPU
+// has resident CTAs (456 of 256 threads), narrower tiles shorten every phase;
+// beyond that they only add items.  us at w = -2, -1, 0 and the items per phase:
+// 50 steps of one 3D wave k=3 n=7 8634 (87), 9114 (52), 10651 (37); 10 steps of 4
+// of them 1322 (240), 1383 (142), 1891 (89), of 16 2527 (918), 2261 (477), 2331
+// (249), of 64 9099, 6283, 5422 (1006); 8 steps of 8 Vlasov 2x2v k=2 n=6 5323
+// (929), 3837 (464), 4104 (257).  The width does not change any column's sums.
+constexpr double kTileItems = 512;
+static int mf_auto_wlog(const std::vector<WLClass>& cls, bool pass_only) {
+    for (int w = -2; w < 0; w++) {
+        double items = 0, chain = 1;
+        for (const WLClass& c : cls) {
+            const bool vlasov = c.kind == MF_KIND_VLASOV;
+            const int cpt = mf_columns_per_thread(c.k), stages = c.apply || pass_only ? 1 : 4;
+            int phases = 0;
+            for (int d = 0; d < c.D; d++) {
+                if (c.apply && c.apply_dim >= 0 && d != c.apply_dim) continue;
+                // Vlasov: D_d, two transforms of each of the D derivatives, two back
+                const int times = vlasov ? 2 * c.D + 3 : 1;
+                phases++;
+                for (const Pencil& p : c.pencils[d]) {
+                    const int W = mf_tile_cols(c.k, cpt, 1 << (p.lmax - 1), w);
+                    items += double(stages * times) * double(((int64_t)c.nslots * p.R + W - 1) / W);
+                }
+            }
+            chain = std::max(chain, double(stages) * (vlasov ? 4 * c.D + 2 : phases));
+        }
+        if (items <= kTileItems * chain) return w;
+    }
+    return 0;
+}
+
 // Work list.  Each class is cut into groups of slots; a group has one phase
 // per dimension pass (the last one also applies the RK stage update, unless
 // applying only), and phase p of a group depends on phase p-1 of the same
@@ -448,12 +482,14 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
     };
     std::vector<Group> groups;
     size_t smem = 64;
+    const int auto_wlog = mf_auto_wlog(cls, pass_only);
     for (size_t ci = 0; ci < cls.size(); ci++) {
         const WLClass& c = cls[ci];
         const WLClass& sp = c;
         const int D = sp.D, k = sp.k;
         const int cpt = mf_columns_per_thread(k);
         MFTile tile = mf_tile(D, k);
+        if (!mf_tile_tuned(D, k)) tile.wlog = auto_wlog;
         if (shapes) {
             auto f = shapes->find({D, k});
             if (f != shapes->end()) tile = f->second;
@@ -518,6 +554,7 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
                         mf_divisor(it.R, &it.rmagic, &it.rshift);
                         it.g0 = (int32_t)g0;
                         it.W = Wp;
+                        while (it.W > cpt && it.W / 2 >= cend - g0) it.W /= 2;  // no wider than its columns
                         it.Wv = (int32_t)std::min<int64_t>(Wp, cend - g0);
                         it.kd1 = kd1;
                         it.kDm1 = kDm1;
