@@ -655,6 +655,8 @@ int sgdg_apply(sgdg_op* op, int which, int method, const double* x, double* y) {
     apply_device_impl(op, which, method, dx.as<double>(), dy.as<double>(), st);
     CK(cudaMemcpyAsync(y, dy.p, sizeof(double) * len, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    dx.recycle();
+    dy.recycle();
     API_END
 }
 
@@ -701,6 +703,7 @@ static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, do
     }
     CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    work.recycle();
     return bad != 0;
 }
 
@@ -742,6 +745,9 @@ struct PlainScratch {
         acc.alloc(b);
         u0.alloc(b);
         u1.alloc(b);
+    }
+    void recycle() {  // after run
+        for (DevBuf* b : {&acc, &u0, &u1, &flag}) b->recycle();
     }
     // returns whether a stage result was not finite; waits for the steps
     template <class Mat>
@@ -796,11 +802,15 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
     }
     if (keep.p) {
         CK(cudaMemcpyAsync(keep.p, y, keep.bytes, cudaMemcpyDeviceToDevice, cs));
-        if (!work->run(*A, nsolves, y, dt, nsteps, cs)) return;
-        CK(cudaMemcpyAsync(y, keep.p, keep.bytes, cudaMemcpyDeviceToDevice, cs));
-        CK(cudaStreamSynchronize(cs));
+        const bool bad = work->run(*A, nsolves, y, dt, nsteps, cs);
+        if (bad) {
+            CK(cudaMemcpyAsync(y, keep.p, keep.bytes, cudaMemcpyDeviceToDevice, cs));
+            CK(cudaStreamSynchronize(cs));
+        }
+        work->recycle();
+        keep.recycle();
+        if (!bad) return;
         work.reset();
-        keep.release();
     }
     const DevCSR& W = op->whole(which);
     try {
@@ -809,6 +819,7 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
         work.reset(new PlainScratch(W, nsolves, 1));
     }
     work->run(W, nsolves, y, dt, nsteps, cs);
+    work->recycle();
 }
 
 extern "C" {
@@ -836,6 +847,7 @@ static void mf_evolve(sgdg_op* op, int kind, const double* a, const double* y0, 
         eng.get_state(id, states + (size_t)i * len);
         if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
     }
+    eng.recycle();
 }
 
 static void check_evolve_args(int64_t nsteps, int nout, double t0, double t1) {
@@ -1097,6 +1109,8 @@ int sgdg_vlasov_rhs(sgdg_vlasov* v, const double* F_point, const double* f, doub
         CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
         CK(cudaStreamSynchronize(v->stream));
     }
+    u.recycle();
+    r.recycle();
     API_END
 }
 
@@ -1132,6 +1146,7 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
             eng.get_state(id, states + (size_t)i * v->ix.N);
             if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
         }
+        eng.recycle();
         return SGDG_OK;
     }
     if (method != SGDG_METHOD_PLAIN) throw Error(SGDG_EINVAL, "method must be PLAIN (0) or MATFREE (1)");
@@ -1183,6 +1198,7 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
         v->build_whole();
         run(true);
     }
+    for (DevBuf* w : {&y, &acc, &u0, &u1}) w->recycle();
     API_END
 }
 
@@ -1496,6 +1512,7 @@ int sgdg_set_hbm_budget(int64_t bytes) {
     API_BEGIN
     if (bytes < 0) throw Error(SGDG_EINVAL, "budget must be >= 0");
     g_budget = bytes;
+    if (bytes > 0) device_pool().trim((size_t)std::max<int64_t>(0, bytes - g_in_use.load()));
     API_END
 }
 

@@ -3,6 +3,10 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <iterator>
+#include <map>
+#include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -36,24 +40,98 @@ inline void require_gpu() {
     state = 1;
 }
 
+// Blocks handed back with DevBuf::recycle, kept for the next allocation of their
+// size: a call that allocates its vectors, arenas or work list pays 10 to 100 us
+// per block for cudaMalloc and cudaFree otherwise (an evolver's call 0.1 to 0.4
+// ms).  Only a block whose work has finished is recycled (its owner has waited
+// for every stream that used it), so any stream or thread may take it; the others
+// are freed, and cudaFree waits.  At most kPoolBytes are kept; they count against
+// the HBM budget, and are given back where an allocation or the budget needs them
+// and when the library holds nothing else.
+class DevPool {
+   public:
+    static constexpr size_t kPoolBytes = size_t(1) << 30;
+    static size_t rounded(size_t n) { return (n + 511) & ~size_t(511); }
+    // a kept block of at least n bytes (at most an eighth more, or exactly n
+    // rounded where a budget is set): its size in got, or null
+    void* take(size_t n, bool exact, size_t& got) {
+        const size_t want = rounded(n);
+        std::lock_guard<std::mutex> g(mu_);
+        auto& m = kept_[device()];
+        const auto it = m.lower_bound(want);
+        if (it == m.end() || it->first > (exact ? want : want + want / 8)) return nullptr;
+        void* p = it->second;
+        got = it->first;
+        m.erase(it);
+        held_ -= got;
+        return p;
+    }
+    // keeps p (size bytes on device dev) or frees it
+    void give(void* p, size_t size, int dev) {
+        if (size <= kPoolBytes / 2 && dev == device()) {
+            std::lock_guard<std::mutex> g(mu_);
+            if (held_ + size <= kPoolBytes) {
+                try {
+                    kept_[dev].emplace(size, p);
+                    held_ += size;
+                    return;
+                } catch (const std::bad_alloc&) {
+                }
+            }
+        }
+        cudaFree(p);
+    }
+    // frees kept blocks, the largest first, until at most `most` bytes are kept
+    void trim(size_t most) {
+        std::lock_guard<std::mutex> g(mu_);
+        for (auto& d : kept_)
+            while (held_ > most && !d.second.empty()) {
+                const auto it = std::prev(d.second.end());
+                cudaFree(it->second);
+                held_ -= it->first;
+                d.second.erase(it);
+            }
+    }
+    size_t held() const { return held_.load(); }
+    static int device() {
+        int d = 0;
+        cudaGetDevice(&d);
+        return d;
+    }
+
+   private:
+    std::mutex mu_;
+    std::map<int, std::multimap<size_t, void*>> kept_;  // per device, by size
+    std::atomic<size_t> held_{0};
+};
+inline DevPool& device_pool() {
+    static DevPool* p = new DevPool;  // outlives the buffers of static objects
+    return *p;
+}
+
 // Device allocation counted against the HBM budget (sgdg_set_hbm_budget).
 struct DevBuf {
     void* p = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;  // asked for
+    size_t size = 0;   // of the block
+    int dev = 0;       // it is on
     DevBuf() = default;
     explicit DevBuf(size_t n) { alloc(n); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes) {
+    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), size(o.size), dev(o.dev) {
         o.p = nullptr;
-        o.bytes = 0;
+        o.bytes = o.size = 0;
     }
     DevBuf& operator=(DevBuf&& o) noexcept {
+        if (this == &o) return *this;
         release();
         p = o.p;
         bytes = o.bytes;
+        size = o.size;
+        dev = o.dev;
         o.p = nullptr;
-        o.bytes = 0;
+        o.bytes = o.size = 0;
         return *this;
     }
     void alloc(size_t n) {
@@ -64,24 +142,41 @@ struct DevBuf {
             throw Error(SGDG_ENOMEM_BUDGET, "HBM budget exceeded: requested " + std::to_string(n) + " bytes, " +
                                                 std::to_string(g_in_use.load()) + " of " + std::to_string(b) +
                                                 " in use");
-        cudaError_t e = cudaMalloc(&p, n);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            p = nullptr;
-            throw Error(SGDG_ENOMEM_BUDGET, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        p = device_pool().take(n, b > 0, size);
+        if (!p) {
+            size = DevPool::rounded(n);
+            if (b > 0) device_pool().trim((size_t)(b - g_in_use.load() - (int64_t)n));
+            cudaError_t e = cudaMalloc(&p, size);
+            if (e == cudaErrorMemoryAllocation && device_pool().held() > 0) {
+                cudaGetLastError();
+                device_pool().trim(0);
+                e = cudaMalloc(&p, size);
+            }
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+                throw Error(SGDG_ENOMEM_BUDGET, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+            }
         }
         bytes = n;
+        dev = DevPool::device();
         g_in_use += (int64_t)n;
     }
-    void release() {
+    void release() { drop(false); }
+    // as release, where everything that used the buffer has finished
+    void recycle() { drop(true); }
+    ~DevBuf() { release(); }
+    void drop(bool keep) {
         if (p) {
-            cudaFree(p);
-            g_in_use -= (int64_t)bytes;
+            if (keep)
+                device_pool().give(p, size, dev);
+            else
+                cudaFree(p);
+            if ((g_in_use -= (int64_t)bytes) == 0) device_pool().trim(0);
         }
         p = nullptr;
-        bytes = 0;
+        bytes = size = 0;
     }
-    ~DevBuf() { release(); }
     template <class T>
     T* as() const {
         return static_cast<T*>(p);

@@ -557,6 +557,7 @@ void evaluate_impl(int D, int k, int n, int scheme, const double* coeffs, int64_
             int h[2] = {0, 0};
             CK(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
+            work.recycle();
             if (h[0]) throw Error(SGDG_EINVAL, "a point coordinate is below 0 or NaN (no cell contains it)");
             if (!h[1]) return;
             // a coefficient that is not finite: block by block, as the sum over levels spreads it
@@ -581,6 +582,7 @@ void evaluate_impl(int D, int k, int n, int scheme, const double* coeffs, int64_
     int h_err = 0;
     CK(cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    err.recycle();
     if (h_err) throw Error(SGDG_EINVAL, "a point coordinate is below 0 or NaN (no cell contains it)");
 }
 
@@ -626,6 +628,7 @@ int sgdg_evaluate(int D, int k, int n, int scheme, const double* coeffs, int64_t
     evaluate_impl(D, k, n, scheme, dc.as<double>(), npts, dx.as<double>(), dv.as<double>(), st);
     CK(cudaMemcpyAsync(values, dv.p, sizeof(double) * (size_t)npts, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    for (DevBuf* b : {&dc, &dx, &dv}) b->recycle();
     API_END
 }
 

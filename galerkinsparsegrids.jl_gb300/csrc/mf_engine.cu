@@ -66,6 +66,24 @@ void MFEngine::drop_graph() {
     chunks_.clear();
 }
 
+void MFEngine::recycle() {
+    drop_graph();
+    for (auto& c : classes_) c->recycle();
+    classes_.clear();
+    solves_.clear();
+    for (DevBuf* b : {&classes_d_, &items_d_, &ctr_d_, &err_d_}) b->recycle();
+    for (auto& s : stabs_)
+        for (DevBuf* b : {&s.second.rowptr, &s.second.ent, &s.second.val}) b->recycle();
+    stabs_.clear();
+    for (auto& q : qtabs_)
+        for (DevBuf* b : {&q.second.rowptr, &q.second.ent, &q.second.val}) b->recycle();
+    qtabs_.clear();
+    for (auto& t : ttabs_)
+        for (STable& s : t.second.t)
+            for (DevBuf* b : {&s.rowptr, &s.ent, &s.val}) b->recycle();
+    ttabs_.clear();
+}
+
 MFEngine::Solve& MFEngine::at(int id) {
     if (id < 0 || id >= (int)solves_.size() || !solves_[id].live) throw Error(SGDG_EINVAL, "no such solve id");
     return solves_[id];
@@ -212,6 +230,7 @@ const MFEngine::QTable& MFEngine::qtab(int k, int n) {
 void MFEngine::plan() {
     if (!dirty_) return;
     drop_graph();
+    CK(cudaStreamSynchronize(stream_));  // the old arenas' work: their blocks are reused below
     if (!err_d_.p) {
         err_d_.alloc(sizeof(int));
         CK(cudaMemsetAsync(err_d_.p, 0, sizeof(int), stream_));
@@ -256,12 +275,12 @@ void MFEngine::plan() {
         }
         ClassArena& c = *next[ci];
         if (old_c) {  // free what the new arena does not need from the old one first
-            old_c->acc.release();
-            old_c->u0.release();
-            old_c->u1.release();
-            old_c->u2.release();
-            old_c->u3.release();
-            old_c->rhs.release();
+            old_c->acc.recycle();
+            old_c->u0.recycle();
+            old_c->u1.recycle();
+            old_c->u2.recycle();
+            old_c->u3.recycle();
+            old_c->rhs.recycle();
         }
         const int ns = (int)c.slots.size();
         if ((int64_t)ns * c.Ns >= (int64_t(1) << 31))
@@ -328,12 +347,17 @@ void MFEngine::plan() {
         c.coef = upload(coef, stream_);
         c.status = upload(status, stream_);
         CK(launch_f64_to_f32(c.y.as<double>(), c.u0.as<float>(), (int64_t)ns * c.Ns, stream_));
-        if (old_c) old_c->y.release();  // cudaFree waits for the copies above
+        if (old_c) {
+            CK(cudaStreamSynchronize(stream_));  // the copies above
+            old_c->y.recycle();
+        }
     }
     CK(cudaStreamSynchronize(stream_));
     pending_bytes_ = 0;
     // the old arenas are no longer referenced
     classes_.swap(next);
+    for (auto& c : next)
+        if (c) c->recycle();
     next.clear();
     for (size_t ci = 0; ci < classes_.size(); ci++)
         for (size_t sl = 0; sl < classes_[ci]->slots.size(); sl++) {
@@ -408,6 +432,7 @@ void MFEngine::plan() {
     std::vector<MFItem> items;
     int nctr = 0;
     build_items(items, nctr);
+    for (DevBuf* b : {&classes_d_, &items_d_, &ctr_d_}) b->recycle();
     classes_d_ = upload(ch, stream_);
     items_d_ = upload(items, stream_);
     ctr_d_.alloc(sizeof(int) * (size_t)std::max(nctr, 1));

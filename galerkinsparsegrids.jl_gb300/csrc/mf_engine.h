@@ -84,6 +84,9 @@ class MFEngine {
 
     double dof_updates_per_step() const;
     int64_t launches_per_step() const { return 1; }  // the whole RK4 step in one launch
+    // hands the device blocks back for reuse and forgets the solves; only after a
+    // call that waited for the stream (get_state)
+    void recycle();
     int check_error();  // returns SGDG_OK or SGDG_ETIMEOUT after a bounded wait gave up
     static int64_t solve_bytes(int64_t N, int64_t Ns, int kind = MF_KIND_ADVECT, int D = 0);  // device bytes of a solve
     int64_t pending_bytes() const { return pending_bytes_; }
@@ -121,6 +124,9 @@ class MFEngine {
         std::vector<int> slots;                    // solve id per slot
         DevBuf y, acc, u0, u1, u2, u3, rhs, dt, coef, status, blockoff;
         DevBuf vb, vw;  // Vlasov: 2 scratch vectors per phase dimension and slot, point weights per slot
+        void recycle() {  // after the stream has been waited for
+            for (DevBuf* b : {&y, &acc, &u0, &u1, &u2, &u3, &rhs, &dt, &coef, &status, &blockoff, &vb, &vw}) b->recycle();
+        }
     };
 
     void plan();
