@@ -45,6 +45,8 @@ cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, d
 cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x, double* y, cudaStream_t st);
 cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                           cudaStream_t st);
+cudaError_t launch_sweep_points(const DevSliced& A, int D, const double* x, const double* v, const double* F, double* out,
+                                cudaStream_t st);
 cudaError_t launch_check_finite(const double* x, int64_t n, int* nonfinite, cudaStream_t st);
 cudaError_t launch_wait_selftest(const int* ctr, int need, int* err, cudaStream_t st);
 cudaError_t launch_convert_selftest(const double* x, int64_t n, unsigned long long* bad, cudaStream_t st);
@@ -186,8 +188,9 @@ struct sgdg_vlasov {
     mutable std::unique_ptr<CSR> T[4];    // m2n, n2p, p2n, n2m on the host, built on request
     mutable std::vector<double> v_point;  // D x N, built on request
     mutable bool have_vpoint = false;
-    // sweep[w][d]: transform w along dimension d; deriv[d]: D_d
-    std::unique_ptr<DeviceSliced> sweep[4][8], deriv[8];
+    // sweep[w]: transform w in turn along the dimensions, one or a few at a time; deriv[d]: D_d
+    std::vector<std::unique_ptr<DeviceSliced>> sweep[4];
+    std::unique_ptr<DeviceSliced> deriv[8];
     // the assembled operators, built on request
     std::vector<std::unique_ptr<DeviceCSR>> dDs;
     std::unique_ptr<DeviceCSR> dT[4];
@@ -240,8 +243,7 @@ struct sgdg_vlasov {
                 const std::vector<double> vm = v_modal(d);
                 CK(cudaMemcpyAsync(x.p, vm.data(), b, cudaMemcpyHostToDevice, stream));
                 double *from = x.as<double>(), *to = y.as<double>();
-                CK(transform(0, 1, from, to));  // P sweeps: back in `from`
-                CK(transform(1, 1, from, to));
+                for (int w : {0, 1}) CK(transform(w, sweep[w].size(), 1, from, to));
                 CK(cudaMemcpyAsync(v_point.data() + (size_t)d * ix.N, from, b, cudaMemcpyDeviceToHost, stream));
                 CK(cudaStreamSynchronize(stream));
             }
@@ -256,46 +258,71 @@ struct sgdg_vlasov {
         flag.alloc(sizeof(int));
         CK(cudaStreamSynchronize(stream));
     }
+    // Dimensions a sweep of transform w takes at once.  More at once multiply
+    // more entries (the product of the dimensions' rows instead of their sum) in
+    // fewer launches of about 2.5 us each.  points -> nodal has at most 3 entries
+    // per row and dimension: four at once are 12 entries instead of 7.7 (2x2v k=2
+    // n=8).  modal -> nodal and nodal -> points take pairs up to 128 K values (us per step,
+    // one by one and in pairs: 2x2v k=2 n=5 173 and 125, n=6 219 and 214; k=3 n=5,
+    // 179 K values, 347 and 369), nodal -> modal, whose coarsest rows span a line
+    // or for a pair a plane, up to 16 K coefficients in planes of 1 K (2x2v k=2 n=5
+    // 184 and 173; n=6, 24 K, 220 and 226); in two dimensions, where a pair's
+    // rows reach the whole grid, all three up to such a plane (1x1v k=2 n=6 82 and
+    // 64, k=3 n=5 86 and 70; k=2 n=8, a plane of 5 K, 100 and 139).
+    int at_once(int w) const {
+        if (w == TRANSFORM_POINTS_TO_NODAL) return 4;
+        if (w == TRANSFORM_NODAL_TO_MODAL)
+            return ix.N <= 16 << 10 && make_index(2, k, n, ix.scheme).N <= 1 << 10 ? 2 : 1;
+        return ix.N * P <= (P == 2 ? 4 << 10 : 128 << 10) ? 2 : 1;
+    }
     void build_sweeps() {
-        if (sweep[3][P - 1]) return;
+        if (!sweep[3].empty()) return;
+        std::vector<std::unique_ptr<DeviceSliced>> s[4];
         for (int d = 0; d < P; d++) deriv[d] = gpu_step_operator(ix, *dlf, d + 1, stream);
         for (int w = 0; w < 4; w++) {
-            const LineTables T = line_tables(transform_1d(k, n, w), k, n + 1);
-            for (int d = 0; d < P; d++) sweep[w][d] = gpu_line_operator(ix, T, d, stream);
+            const CSR T1 = transform_1d(k, n, w);
+            const LineTables T = line_tables(T1, k, n + 1);
+            const int step = at_once(w);
+            for (int d = 0; d < P; d += step)
+                s[w].push_back(step == 1 ? gpu_line_operator(ix, T, d, stream)
+                                         : gpu_partial_transform(ix, T1, ((1u << std::min(step, P - d)) - 1) << d, stream));
         }
+        for (int w = 0; w < 4; w++) sweep[w] = std::move(s[w]);
     }
     void drop_sweeps() {
-        for (int d = 0; d < 8; d++) {
-            deriv[d].reset();
-            for (int w = 0; w < 4; w++) sweep[w][d].reset();
-        }
+        for (auto& d : deriv) d.reset();
+        for (auto& s : sweep) s.clear();
     }
-    // x = transform w of nv interleaved vectors x: P sweeps, P even, so the
-    // result is back in x; y: scratch
-    cudaError_t transform(int w, int nv, double* x, double* y) {
+    // the first `count` sweeps of transform w of nv interleaved vectors, from x;
+    // the result is in x, y is scratch (the two pointers change places)
+    cudaError_t transform(int w, size_t count, int nv, double*& x, double*& y) {
         cudaError_t e = cudaSuccess;
-        for (int d = 0; d < P && e == cudaSuccess; d++, std::swap(x, y))
-            e = launch_sweep(sweep[w][d]->d, nv, x, y, nullptr, stream);
+        for (size_t i = 0; i < count && e == cudaSuccess; i++, std::swap(x, y))
+            e = launch_sweep(sweep[w][i]->d, nv, x, y, nullptr, stream);
         return e;
     }
-    // z = all sweeps of n2m but the last, of p2n (-sum_d v_d .* n2p m2n Dx_d u
-    // + sum_d F_d .* n2p m2n Dp_d u): the P derivatives, interleaved, each
-    // transform's sweeps on all P of them at a time, the point products and the
-    // sweeps back.  The last sweep (last_sweep) takes z.
-    cudaError_t sweep_rhs(const double* u) {
+    // all sweeps of n2m but the last, of p2n (-sum_d v_d .* n2p m2n Dx_d u + sum_d
+    // F_d .* n2p m2n Dp_d u): the P derivatives, interleaved, each transform's
+    // sweeps on all P of them at a time, the point products (with the last sweep
+    // for P <= 4) and the sweeps back.  last_sweep takes `result`.
+    cudaError_t sweep_rhs(const double* u, double** result) {
         double *tt = t.as<double>(), *ss = s.as<double>(), *cc = c.as<double>(), *zz = z.as<double>();
+        const double *v = vpt.as<double>(), *f = F.as<double>();
         const DevSliced* D_[8];
         for (int d = 0; d < P; d++) D_[d] = &deriv[d]->d;
+        const size_t np = sweep[1].size();
         cudaError_t e = launch_derivatives(D_, P, u, tt, stream);
-        if (e == cudaSuccess) e = transform(0, P, tt, ss);
-        if (e == cudaSuccess) e = transform(1, P, tt, ss);
-        if (e == cudaSuccess) e = launch_points(vpt.as<double>(), F.as<double>(), tt, D, ix.N, cc, stream);
-        if (e == cudaSuccess) e = transform(2, 1, cc, zz);
-        for (int d = 0; d + 1 < P && e == cudaSuccess; d++, std::swap(cc, zz))
-            e = launch_sweep(sweep[3][d]->d, 1, cc, zz, nullptr, stream);
+        if (e == cudaSuccess) e = transform(0, sweep[0].size(), P, tt, ss);
+        if (e == cudaSuccess) e = transform(1, P <= 4 ? np - 1 : np, P, tt, ss);
+        if (e == cudaSuccess)
+            e = P <= 4 ? launch_sweep_points(sweep[1][np - 1]->d, D, tt, v, f, cc, stream)
+                       : launch_points(v, f, tt, D, ix.N, cc, stream);
+        if (e == cudaSuccess) e = transform(2, sweep[2].size(), 1, cc, zz);
+        if (e == cudaSuccess) e = transform(3, sweep[3].size() - 1, 1, cc, zz);
+        *result = cc;
         return e;
     }
-    const DevSliced& last_sweep() const { return sweep[3][P - 1]->d; }
+    const DevSliced& last_sweep() const { return sweep[3].back()->d; }
     // the assembled operators and their scratch; the sweeps make room for them where there is none
     void build_whole() {
         if (p.p) return;
@@ -312,7 +339,7 @@ struct sgdg_vlasov {
         try {
             build();
         } catch (const Error& e) {
-            if (e.code != SGDG_ENOMEM_BUDGET || !sweep[3][P - 1]) throw;
+            if (e.code != SGDG_ENOMEM_BUDGET || sweep[3].empty()) throw;
             drop_sweeps();
             build();
         }
@@ -1097,8 +1124,9 @@ int sgdg_vlasov_rhs(sgdg_vlasov* v, const double* F_point, const double* f, doub
     CK(cudaMemsetAsync(v->flag.p, 0, sizeof(int), v->stream));
     v->build_sweeps();
     CK(launch_check_finite(u.as<double>(), N, v->flag.as<int>(), v->stream));
-    CK(v->sweep_rhs(u.as<double>()));
-    CK(launch_sweep(v->last_sweep(), 1, v->z.as<double>(), r.as<double>(), v->flag.as<int>(), v->stream));
+    double* last = nullptr;
+    CK(v->sweep_rhs(u.as<double>(), &last));
+    CK(launch_sweep(v->last_sweep(), 1, last, r.as<double>(), v->flag.as<int>(), v->stream));
     CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
     CK(cudaMemcpyAsync(&bad, v->flag.p, sizeof(int), cudaMemcpyDeviceToHost, v->stream));
     CK(cudaStreamSynchronize(v->stream));
@@ -1170,11 +1198,12 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
             cudaError_t e = cudaSuccess;
             for (int64_t i = 0; i < n; i++)
                 for (int stage = 1; stage <= 4 && e == cudaSuccess; stage++) {
-                    e = whole ? v->whole_rhs(in[stage - 1]) : v->sweep_rhs(in[stage - 1]);
+                    double* last = v->z.as<double>();
+                    e = whole ? v->whole_rhs(in[stage - 1]) : v->sweep_rhs(in[stage - 1], &last);
                     if (e == cudaSuccess)
-                        e = whole ? launch_csr_rk4(v->dT[3]->d, v->z.as<double>(), y.as<double>(), acc.as<double>(),
-                                                   outv[stage - 1], dt, stage, flag, st)
-                                  : launch_csr_rk4(v->last_sweep(), v->z.as<double>(), y.as<double>(), acc.as<double>(),
+                        e = whole ? launch_csr_rk4(v->dT[3]->d, last, y.as<double>(), acc.as<double>(), outv[stage - 1],
+                                                   dt, stage, flag, st)
+                                  : launch_csr_rk4(v->last_sweep(), last, y.as<double>(), acc.as<double>(),
                                                    outv[stage - 1], dt, stage, flag, st);
                 }
             return e;

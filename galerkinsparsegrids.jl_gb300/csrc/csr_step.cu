@@ -11,13 +11,14 @@
 //    whole ones (DevCSR) in rows.
 //  * k_rk_segments, k_rk_long_rows: rows longer than A.split, one warp per
 //    segment, then the segment partials of each row in order and the update.
-//  * k_derivatives, k_sweep, k_points: the P derivatives of a phase-space
-//    vector, a transform along one dimension for P interleaved vectors or one,
-//    and the products at the points.
+//  * k_derivatives, k_sweep, k_sweep_points, k_points: the P derivatives of a
+//    phase-space vector; a transform along one dimension or a few for P
+//    interleaved vectors or one; the products at the points, with the last
+//    transform or alone.
 //
 // Bounds: large operators the FP64 pipe (2 operations per clock and SM, the
 // additions of the lane reduction and of the stage update among them), small
-// ones the latency of four dependent launches per step (Vlasov: 4 (4P + 2)).
+// ones the latency of four dependent launches per step (Vlasov: up to 4 (4P + 2)).
 // For the second the launches are programmatic dependents (pdl_wait): a
 // launch's blocks come up and fetch their rows, columns and values while the
 // launch before it still runs, and wait for it only before the vectors.
@@ -25,12 +26,12 @@
 // Measured, from host to host: 200 steps of the 2D wave k=3 n=5 6.34 -> 2.0 ms
 // against one solve at a time with the whole operator and plain launches; 60
 // steps of the 4D advection k=2 n=6 5.89 -> 1.5 ms; 3 steps of 48 3D waves k=3
-// n=7 11.8 -> 3.1 ms (0.87 ms per step, of which the FP64 pipe needs 0.74).
+// n=7 11.8 -> 2.6 ms (0.87 ms per step, of which the FP64 pipe needs 0.74).
 // In slices against rows: the single 3D wave 46.9 -> 38.1 us per step, 256 of
 // them 4.80 -> 4.49 ms, the Vlasov step below 810 -> 634 us.  Vlasov 2x2v k=2
-// n=8: 2595 -> 634 us per step against the assembled transforms, of which the
-// FP64 pipe needs 231 (a k_sweep<4> keeps it 78 % busy) and about 195 are the
-// latency of 72 launches (what the step takes at n=5, 8832 coefficients).
+// n=8: 2595 -> 627 us per step against the assembled transforms, of which the
+// FP64 pipe needs 240 (a k_sweep<4> keeps it 78 % busy) and about 150 are the
+// latency of 56 launches; n=5 296 -> 125 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -235,6 +236,16 @@ __device__ __forceinline__ void bin_rows(const DevSliced& A, int64_t rb, const d
     csr_reduce<VS, NV>(s, lane);
     bool stores;
     const int owner = csr_owner<VS, NV>(lane, stores);
+    if constexpr (Out::kTogether && ((NV == 4 && VS >= 4) || (NV == 2 && VS >= 2))) {
+        // the row's sums to its first lane (csr_owner's lanes)
+        const double mine = s[0];
+#pragma unroll
+        for (int j = 0; j < NV; j++)
+            s[j] = __shfl_sync(0xffffffffu, mine,
+                               NV == 4 ? (j & 2 ? VS / 2 : 0) + (j & 1 ? VS / 4 : 0) : (j & 1 ? VS / 2 : 0), VS);
+        if (row >= 0 && lane == 0) out.all(row, s);
+        return;
+    }
     if (row < 0 || !stores) return;
     if (owner >= 0)
         out.one(row, owner, s[0]);
@@ -274,6 +285,7 @@ __device__ __forceinline__ void block_rows(const DevCSR& A, int64_t rb, const do
 // the stage update of nv of the NV solves of a set, solve j's state at y + j m
 template <int NV>
 struct RkOut {
+    static constexpr bool kTogether = false;
     const CsrRK& rk;
     double* y;
     int64_t m;
@@ -356,6 +368,7 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
 // y[i * stride + j]); a result that is not finite raises *nonfinite
 template <int NV>
 struct SweepOut {
+    static constexpr bool kTogether = false;
     double* y;
     int64_t stride;
     int* nonfinite;
@@ -375,8 +388,41 @@ struct SweepOut {
     }
 };
 
-// One sweep y = T x of a transform along one dimension (DevCSR of the lines),
-// for sets of NV of `stride` interleaved vectors; blockIdx.y: the set.
+// The point-basis combination of the Vlasov right-hand side (src/pdes.jl:
+// 185-191) of the P = 2D transformed derivatives of a point q (x dimensions d <
+// D, then p): -(sum_d v_d q_d) + sum_d F_d q_{D+d}, each sum left to right with
+// separate roundings of products and sums.
+template <int D>
+__device__ __forceinline__ double point_product(const double* __restrict__ v, const double* __restrict__ F, int64_t n,
+                                                int64_t i, const double (&q)[2 * D]) {
+    double c1 = __dmul_rn(__ldg(v + i), q[0]), c2 = __dmul_rn(__ldg(F + i), q[D]);
+#pragma unroll
+    for (int d = 1; d < D; d++) {
+        c1 = __dadd_rn(c1, __dmul_rn(__ldg(v + d * n + i), q[d]));
+        c2 = __dadd_rn(c2, __dmul_rn(__ldg(F + d * n + i), q[D + d]));
+    }
+    return __dadd_rn(-c1, c2);
+}
+
+// the products of a row's P = NV values
+template <int NV>
+struct PointsOut {
+    static constexpr bool kTogether = true;
+    const double *v, *F;
+    double* out;
+    int64_t n;
+    __device__ __forceinline__ void one(int64_t, int, double) const {}
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+        out[row] = point_product<NV / 2>(v, F, n, row, s);
+    }
+};
+template <int NV>
+__global__ void __launch_bounds__(256, 3)
+    k_sweep_points(DevSliced A, const double* x, const double* v, const double* F, double* out) {
+    block_rows<NV>(A, blockIdx.x, x, NV, PointsOut<NV>{v, F, out, A.m});
+}
+
+// One sweep y = T x of a transform along one dimension or a few, for sets of NV of `stride` interleaved vectors; blockIdx.y: the set.
 template <int NV>
 __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
     k_sweep(DevSliced A, const double* x, double* y, int64_t stride, int* nonfinite) {
@@ -387,6 +433,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
 // One application y = A x with the pruned operator; an element of x that is not
 // finite leaves `call` in *seen, for k_apply_whole
 struct ApplyOut {
+    static constexpr bool kTogether = false;
     const double* x;
     double* y;
     int* seen;
@@ -434,21 +481,11 @@ __global__ void __launch_bounds__(256, 4)
     block_rows<1>(A, blockIdx.x, x, 1, SweepOut<1>{y + blockIdx.y, P, nullptr});
 }
 
-// The point-basis combination of the Vlasov right-hand side (src/pdes.jl:
-// 185-191): with the 2D transformed derivatives interleaved, pt[i * 2D + d]
-// (x dimensions d < D, then p),
-//   out = -(sum_d v_d .* pt_d) + sum_d F_d .* pt_{D+d},
-// each sum left to right with separate roundings of products and sums.
+// the same for P = 2D interleaved vectors pt[i 2D + d]
 template <int D>
 __global__ void k_points(const double* __restrict__ v, const double* __restrict__ F, const double* pt, int64_t n,
                          double* out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double vv[D], ff[D];
-#pragma unroll
-    for (int d = 0; d < D; d++) {
-        vv[d] = i < n ? __ldg(v + d * n + i) : 0.0;
-        ff[d] = i < n ? __ldg(F + d * n + i) : 0.0;
-    }
     pdl_wait();
     if (i >= n) return;
     double q[2 * D];
@@ -458,13 +495,7 @@ __global__ void k_points(const double* __restrict__ v, const double* __restrict_
         q[2 * d] = t.x;
         q[2 * d + 1] = t.y;
     }
-    double c1 = __dmul_rn(vv[0], q[0]), c2 = __dmul_rn(ff[0], q[D]);
-#pragma unroll
-    for (int d = 1; d < D; d++) {
-        c1 = __dadd_rn(c1, __dmul_rn(vv[d], q[d]));
-        c2 = __dadd_rn(c2, __dmul_rn(ff[d], q[D + d]));
-    }
-    out[i] = __dadd_rn(-c1, c2);
+    out[i] = point_product<D>(v, F, n, i, q);
 }
 
 __global__ void k_check_finite(const double* __restrict__ x, int64_t n, int* nonfinite) {
@@ -640,9 +671,18 @@ cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x
     return cudaGetLastError();
 }
 
+// out = the products of the points of y = T x, x 2D interleaved vectors (D <= 2)
+cudaError_t launch_sweep_points(const DevSliced& A, int D, const double* x, const double* v, const double* F, double* out,
+                                cudaStream_t st) {
+    const unsigned nb = (unsigned)A.bin_block[kCsrBins];
+    if (nb > 0) launch_dependent(D == 1 ? k_sweep_points<2> : k_sweep_points<4>, nb, st, A, x, v, F, out);
+    return cudaGetLastError();
+}
+
+// the products of 2D interleaved vectors (D = 3, 4)
 cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                           cudaStream_t st) {
-    auto kernel = D == 1 ? k_points<1> : D == 2 ? k_points<2> : D == 3 ? k_points<3> : k_points<4>;
+    auto kernel = D == 3 ? k_points<3> : k_points<4>;
     if (n > 0) launch_dependent(kernel, (unsigned)grid_for(n), st, v, F, pt, n, out);
     return cudaGetLastError();
 }

@@ -135,6 +135,9 @@ std::unique_ptr<DeviceCSR> gpu_operator(const SparseIndex& ix, const DLF1D& dlf,
 std::unique_ptr<DeviceSliced> gpu_step_operator(const SparseIndex& ix, const DLF1D& dlf, int which, cudaStream_t st);
 // The 1D operators T of the lines (per line length) along dimension d (0-based)
 std::unique_ptr<DeviceSliced> gpu_line_operator(const SparseIndex& ix, const LineTables& T, int d, cudaStream_t st);
+// The product of the 1D transform T1 along the dimensions `dims` (bits), the
+// identity along the others, with the entries gpu_transform keeps
+std::unique_ptr<DeviceSliced> gpu_partial_transform(const SparseIndex& ix, const CSR& T1, unsigned dims, cudaStream_t st);
 // The D_d of a grid one after another in each row (pruned as above), the
 // dimension of every entry and the unscaled values kept: scale() makes the
 // values those of sum_d s[d] D_d.

@@ -324,7 +324,9 @@ struct TransArgs {
     const int8_t* levels;
     const int32_t* lev_off;
     const int32_t* code2lev;  // (n+1)^D level tuple code -> block, or -1
-    const int64_t* rp1;       // filtered 1D rows
+    int n1;                   // 1D indices
+    unsigned ident;           // dimensions along which the identity is taken (bits)
+    const int64_t* rp1;       // filtered 1D rows, then those of the identity
     const int32_t* col1;
     const double* val1;
 };
@@ -449,6 +451,7 @@ __device__ void row_groups(const TransArgs& A, int64_t i, int d, int (*gs)[kTLev
         ml /= k;
         i1 = k * ((L >= 2 ? ((int64_t)1 << (L - 2)) : 0) + c) + m;
     }
+    if (A.ident >> d & 1) i1 += A.n1;
     const int a = (int)A.rp1[i1], b = (int)A.rp1[i1 + 1];  // 1D transforms hold < 2^31 entries
     int n = 0, last = -1;
     for (int e = a; e < b; e++) {
@@ -584,7 +587,10 @@ __global__ void __launch_bounds__(kTLongThreads)
 
 }  // namespace
 
-std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, cudaStream_t st) {
+// The product over the dimensions of T1, the identity along those of `ident`
+// (bits): its CSR arrays without bins, rph the row pointers
+static std::unique_ptr<DeviceCSR> transform_csr(const SparseIndex& ix, const CSR& T1, unsigned ident, cudaStream_t st,
+                                                std::vector<int64_t>& rph) {
     require_gpu();
     const int D = ix.D, k = ix.k, n = ix.n;
     if (n + 1 > kTLev) throw Error(SGDG_EUNSUPPORTED, "more than 16 levels per dimension");
@@ -623,13 +629,19 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
         }
         rp[r + 1] = (int64_t)cl.size();
     }
+    // the identity's rows after them
+    for (int64_t r = 0; ident && r < T1.m; r++) {
+        cl.push_back((int32_t)r);
+        vl.push_back(1.0);
+        rp.push_back((int64_t)cl.size());
+    }
     std::vector<int8_t> lv(ix.levels.size());
     for (size_t q = 0; q < lv.size(); q++) lv[q] = (int8_t)ix.levels[q];
     std::vector<int32_t> lo(ix.lev_off.begin(), ix.lev_off.end());
     DevBuf d_lv = upload(lv, st), d_lo = upload(lo, st), d_code = upload(ix.code2lev, st), d_rp = upload(rp, st),
            d_cl = upload(cl, st), d_vl = upload(vl, st);
     TransArgs A{D, k, n, ix.scheme, ix.nlev, ix.N, ix.kD, d_lv.as<int8_t>(), d_lo.as<int32_t>(), d_code.as<int32_t>(),
-                d_rp.as<int64_t>(), d_cl.as<int32_t>(), d_vl.as<double>()};
+                (int)T1.m, ident, d_rp.as<int64_t>(), d_cl.as<int32_t>(), d_vl.as<double>()};
     // rows with kTLongTuples level tuples or more (the product over the
     // dimensions of the levels present in each 1D row, as the kernels count
     // them) go to k_transform_long
@@ -659,7 +671,7 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
                     const int64_t i1 = k * ((L[d] >= 2 ? ((int64_t)1 << (L[d] - 2)) : 0) + cr % nc[d]) + mr % k;
                     cr /= nc[d];
                     mr /= k;
-                    ntup *= nlev1[(size_t)i1];
+                    if (!(ident >> d & 1)) ntup *= nlev1[(size_t)i1];
                 }
                 if (ntup >= kTLongTuples) long_rows.push_back((int32_t)(ix.lev_off[b] + c * ix.kD + m));
             }
@@ -675,7 +687,7 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
                                                                  nullptr, nullptr);
         CK(cudaGetLastError());
     }
-    std::vector<int64_t> rph = scan_rows(rowlen, ix.N, st);
+    rph = scan_rows(rowlen, ix.N, st);
     auto R = std::make_unique<DeviceCSR>();
     R->rowptr = upload(rph, st);
     R->col.alloc(sizeof(int32_t) * (size_t)rph[ix.N]);
@@ -690,7 +702,13 @@ std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, c
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(st));
-    finish_device_csr(*R, rph, ix.N, st, kCsrLaneEntriesMulti);  // the transforms take four vectors a pass
+    return R;
+}
+
+std::unique_ptr<DeviceCSR> gpu_transform(const SparseIndex& ix, const CSR& T1, cudaStream_t st) {
+    std::vector<int64_t> rp;
+    auto R = transform_csr(ix, T1, 0, st, rp);
+    finish_device_csr(*R, rp, ix.N, st, kCsrLaneEntriesMulti);  // the transforms take four vectors a pass
     return R;
 }
 
@@ -833,6 +851,12 @@ std::unique_ptr<DeviceSliced> gpu_line_operator(const SparseIndex& ix, const Lin
     require_gpu();
     std::vector<int64_t> rp;
     const auto A = line_operator(ix, T, d, st, rp);
+    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesMulti);
+}
+
+std::unique_ptr<DeviceSliced> gpu_partial_transform(const SparseIndex& ix, const CSR& T1, unsigned dims, cudaStream_t st) {
+    std::vector<int64_t> rp;
+    const auto A = transform_csr(ix, T1, ((1u << ix.D) - 1) & ~dims, st, rp);
     return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesMulti);
 }
 

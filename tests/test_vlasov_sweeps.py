@@ -22,9 +22,11 @@ def assembled(sgdg, D, k, n, scheme, F, v):
     return rhs
 
 
-# P = 2, 4 and 8 (4 vectors at a time), 6 (2 at a time); lines of 2 to 640 elements
+# P = 2, 4 and 8 (4 vectors at a time), 6 (2 at a time); lines of 2 to 640 elements;
+# transforms in pairs of dimensions and (1x1v n=7, 2x2v n=6 and k=3 n=5) one by one
 CASES = [(1, 2, 2, "sparse"), (1, 5, 7, "sparse"), (1, 3, 4, "full"), (2, 2, 4, "sparse"), (2, 3, 3, "sparse"),
-         (2, 5, 2, "sparse"), (3, 2, 2, "sparse"), (4, 2, 2, "sparse")]
+         (2, 5, 2, "sparse"), (3, 2, 2, "sparse"), (4, 2, 2, "sparse"),
+         (2, 2, 6, "sparse"), (2, 3, 5, "sparse")]
 
 
 @pytest.mark.parametrize("D,k,n,scheme", CASES)
