@@ -6,9 +6,7 @@
 // move into the new arena device-to-device), keeps the others as they are, and
 // rebuilds the ordered work list.
 // One RK4 step is one launch of k_mf_stage over a work list holding all four
-// stages (each group's stages in order, different groups' stages interleaved),
-// captured once in a CUDA graph; a membership change drops the graph and the
-// next step re-captures it.
+// stages (each group's stages in order, different groups' stages interleaved).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -20,6 +18,8 @@ namespace sgdg {
 
 cudaError_t launch_mf_stage(const MFItem* items, int nitems, const MFClass* classes, int* ctr, int nctr, int stage,
                             int in_sel, int* err, size_t smem, int table_bytes, int grid, cudaStream_t st);
+cudaError_t launch_mf_step(const MFItem* items, int nitems, const MFClass* classes, int* ctr, int nctr, int* err,
+                           size_t smem, int table_bytes, int grid, cudaStream_t st);
 cudaError_t mf_configure(size_t smem, int* blocks_per_sm);
 int mf_columns_per_thread(int k);
 cudaError_t launch_f64_to_f32(const double* a, float* b, int64_t n, cudaStream_t st);
@@ -44,30 +44,29 @@ static int wave_square_levels() {  // SGDG_MF_WAVE_SQUARE overrides (0: two swee
 }
 constexpr int64_t kGroupReuseBytes = 6LL << 20;  // reused u + rhs per group (~4 groups in flight)
 
+static double mf_chain(const std::vector<WLClass>& cls, bool pass_only);
+static int mf_ctas_per_sm(double items_per_phase, int most);
+
 // The arenas' cudaFree calls wait for outstanding work; the stream is not
 // touched here because a caller's stream may already be gone.
-MFEngine::~MFEngine() { drop_graph(); }
+MFEngine::~MFEngine() { drop_chunks(); }
 
 void MFEngine::set_stream(cudaStream_t st) {
-    if (st != stream_) drop_graph();
+    if (st != stream_) drop_chunks();
     stream_ = st;
 }
 
-void MFEngine::drop_graph() {
-    if (graph_) cudaGraphExecDestroy(graph_);
-    graph_ = nullptr;
-    for (Chunk& c : chunks_) {
-        if (c.graph) cudaGraphExecDestroy(c.graph);
+void MFEngine::drop_chunks() {
+    for (Chunk& c : chunks_)
         if (c.st) {
             cudaStreamSynchronize(c.st);
             cudaStreamDestroy(c.st);
         }
-    }
     chunks_.clear();
 }
 
 void MFEngine::recycle() {
-    drop_graph();
+    drop_chunks();
     for (auto& c : classes_) c->recycle();
     classes_.clear();
     solves_.clear();
@@ -229,7 +228,7 @@ const MFEngine::QTable& MFEngine::qtab(int k, int n) {
 
 void MFEngine::plan() {
     if (!dirty_) return;
-    drop_graph();
+    drop_chunks();
     CK(cudaStreamSynchronize(stream_));  // the old arenas' work: their blocks are reused below
     if (!err_d_.p) {
         err_d_.alloc(sizeof(int));
@@ -435,7 +434,8 @@ void MFEngine::plan() {
     for (DevBuf* b : {&classes_d_, &items_d_, &ctr_d_}) b->recycle();
     classes_d_ = upload(ch, stream_);
     items_d_ = upload(items, stream_);
-    ctr_d_.alloc(sizeof(int) * (size_t)std::max(nctr, 1));
+    ctr_d_.alloc(sizeof(int) * (size_t)(nctr + 1));
+    CK(cudaMemsetAsync(ctr_d_.p, 0, ctr_d_.bytes, stream_));
     nitems_ = (int)items.size();
     nctr_ = nctr;
     int bps = 0;
@@ -443,7 +443,7 @@ void MFEngine::plan() {
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    grid_ = std::max(1, bps) * sms;
+    grid_ = mf_ctas_per_sm(nitems_ / mf_chain(wl_classes(), false), std::max(1, bps)) * sms;
     sms_ = sms;
     CK(cudaStreamSynchronize(stream_));
     dirty_ = false;
@@ -453,34 +453,54 @@ void MFEngine::plan() {
 // phase's tiles run side by side and the next phase waits for all of them, so
 // where a step holds fewer items per phase of its longest chain than the GPU
 // has resident CTAs (456 of 256 threads), narrower tiles shorten every phase;
-// beyond that they only add items.  us at w = -2, -1, 0 and the items per phase:
-// 50 steps of one 3D wave k=3 n=7 8634 (87), 9114 (52), 10651 (37); 10 steps of 4
-// of them 1322 (240), 1383 (142), 1891 (89), of 16 2527 (918), 2261 (477), 2331
-// (249), of 64 9099, 6283, 5422 (1006); 8 steps of 8 Vlasov 2x2v k=2 n=6 5323
-// (929), 3837 (464), 4104 (257).  The width does not change any column's sums.
-constexpr double kTileItems = 512;
+// beyond that they only add items, a quarter's sooner than a half's.  us at w =
+// -2, -1, 0 and the items per phase: 50 steps of one 3D wave k=3 n=7 8634 (87),
+// 9114 (52), 10651 (37); 10 steps of 16 of them 2527 (918), 2261 (477), 2331
+// (249), of 64 9099, 6283 (1995), 5422 (1006); of 50 2D waves k=4 n=6 1251 (400),
+// 1533 (200), 2153 (103); of 3D waves k=2 n=6, 50 solves 1183 (545), 1019 (286),
+// 1351 (157), 120 solves 2411 (1290), 1585 (645), 1795 (330); 20 steps of the
+// uneven batch 8116, 5835, 5177 (575).  The width does not change any column's
+// sums.
+constexpr double kTileItems[2] = {420, 700};  // at most, at w = -2 and -1
+// phases of the longest chain of a list over these classes
+static double mf_chain(const std::vector<WLClass>& cls, bool pass_only) {
+    double chain = 1;
+    for (const WLClass& c : cls) {
+        const int passes = c.apply && c.apply_dim >= 0 ? 1 : c.D;
+        chain = std::max(chain, double(c.apply || pass_only ? 1 : 4) *
+                                    (c.kind == MF_KIND_VLASOV ? 4 * c.D + 2 : passes));
+    }
+    return chain;
+}
 static int mf_auto_wlog(const std::vector<WLClass>& cls, bool pass_only) {
     for (int w = -2; w < 0; w++) {
-        double items = 0, chain = 1;
+        double items = 0;
         for (const WLClass& c : cls) {
-            const bool vlasov = c.kind == MF_KIND_VLASOV;
-            const int cpt = mf_columns_per_thread(c.k), stages = c.apply || pass_only ? 1 : 4;
-            int phases = 0;
+            // Vlasov, along each dimension: D_d, two transforms of each of the D derivatives, two back
+            const int cpt = mf_columns_per_thread(c.k);
+            const double times = (c.apply || pass_only ? 1 : 4) * (c.kind == MF_KIND_VLASOV ? 2 * c.D + 3 : 1);
             for (int d = 0; d < c.D; d++) {
                 if (c.apply && c.apply_dim >= 0 && d != c.apply_dim) continue;
-                // Vlasov: D_d, two transforms of each of the D derivatives, two back
-                const int times = vlasov ? 2 * c.D + 3 : 1;
-                phases++;
                 for (const Pencil& p : c.pencils[d]) {
                     const int W = mf_tile_cols(c.k, cpt, 1 << (p.lmax - 1), w);
-                    items += double(stages * times) * double(((int64_t)c.nslots * p.R + W - 1) / W);
+                    items += times * double(((int64_t)c.nslots * p.R + W - 1) / W);
                 }
             }
-            chain = std::max(chain, double(stages) * (vlasov ? 4 * c.D + 2 : phases));
         }
-        if (items <= kTileItems * chain) return w;
+        if (items <= kTileItems[w + 2] * mf_chain(cls, pass_only)) return w;
     }
     return 0;
+}
+
+// CTAs per SM of a list's launch, of the `most` that fit: with fewer items per
+// phase than SMs, a second CTA on an SM only takes items that another SM would
+// run alone (and shared memory from its L1).  us with 1, 2 and 3, and the items
+// per phase: 10 steps of 4 2D waves k=3 n=7 786, 859, 880 (24), of 16 806, 975,
+// 1068 (96); 50 steps of one 3D wave k=3 n=7 7868, 8165, 8399 (87); 10 steps of 4
+// 3D waves k=4 n=5 1064, 850, 939 (136); of 16 3D waves k=2 n=6 996, 789, 736
+// (172); 8 of Vlasov 2x2v k=2 n=6 8286, 4645, 3862 (464).
+static int mf_ctas_per_sm(double items_per_phase, int most) {
+    return items_per_phase <= 100 ? 1 : items_per_phase <= 150 ? std::min(2, most) : most;
 }
 
 // Work list.  Each class is cut into groups of slots; a group has one phase
@@ -726,15 +746,20 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
     return smem;
 }
 
-void MFEngine::build_items(std::vector<MFItem>& items, int& nctr, bool pass_only,
-                           const std::map<std::pair<int, int>, MFTile>* shapes, int chunk, int nchunks,
-                           std::vector<std::array<int, 3>>* ranges) {
+std::vector<WLClass> MFEngine::wl_classes() const {
     std::vector<WLClass> cls;
     for (auto& cp : classes_) {
         const SolveSpec& sp = solves_[cp->slots[0]].spec;
         cls.push_back(WLClass{sp.kind, sp.D, sp.k, sp.n, sp.apply, sp.apply_dim, cp->N, cp->Ns,
                               (int)cp->slots.size(), cp->pencils, cp->boff_index});
     }
+    return cls;
+}
+
+void MFEngine::build_items(std::vector<MFItem>& items, int& nctr, bool pass_only,
+                           const std::map<std::pair<int, int>, MFTile>* shapes, int chunk, int nchunks,
+                           std::vector<std::array<int, 3>>* ranges) {
+    const std::vector<WLClass> cls = wl_classes();
     size_t smem = mf_work_list(cls, items, nctr, pass_only, shapes, chunk, nchunks, ranges);
     int tb = 0;
     for (auto& cp : classes_) {
@@ -857,55 +882,17 @@ std::vector<std::pair<int, int>> MFEngine::autotune() {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     dirty_ = true;  // rebuild the work list with the tuned shapes
-    drop_graph();
+    drop_chunks();
     plan();
     return done;
 }
 
-void MFEngine::capture() {
-    cudaStream_t cs = stream_;
-    cudaStream_t own = nullptr;
-    if (cs == nullptr) {  // graphs cannot be captured on the legacy stream
-        CK(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
-        cs = own;
-    }
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    // the work list holds the whole RK4 step (every item carries its stage)
-    cudaError_t err = launch_mf_stage(items_d_.as<MFItem>(), nitems_, classes_d_.as<MFClass>(), ctr_d_.as<int>(),
-                                      nctr_, 1, 0, err_d_.as<int>(), smem_, table_bytes_, grid_, cs);
-    cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-    if (own) cudaStreamDestroy(own);
-    if (err != cudaSuccess || e2 != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        throw Error(SGDG_ECUDA, std::string("graph capture: ") + cudaGetErrorString(err != cudaSuccess ? err : e2));
-    }
-    cudaError_t e3 = cudaGraphInstantiate(&graph_, g, 0);
-    cudaGraphDestroy(g);
-    if (e3 != cudaSuccess) {
-        graph_ = nullptr;
-        throw Error(SGDG_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e3));
-    }
-}
-
 void MFEngine::build_chunks(int nchunks) {
-    if ((int)chunks_.size() == nchunks) return;  // chunks_ is dropped with the graph on a re-plan
-    for (Chunk& c : chunks_) {
-        if (c.graph) cudaGraphExecDestroy(c.graph);
-        if (c.st) {
-            cudaStreamSynchronize(c.st);
-            cudaStreamDestroy(c.st);
-        }
-    }
-    chunks_.clear();
+    if ((int)chunks_.size() == nchunks) return;  // chunks_ is dropped on a re-plan
+    drop_chunks();
     chunks_.resize(nchunks);
     const size_t smem = smem_;
     const int tb = table_bytes_;
-    // a chunk holds a fraction of the groups, so its phases wait on one
-    // another more; with one CTA per SM per launch, as many chunks' stage
-    // launches as CTAs fit on an SM run side by side and cover each other's
-    // waits
-    const int cgrid = nchunks > 1 ? std::max(1, sms_) : grid_;
     for (int ci = 0; ci < nchunks; ci++) {
         Chunk& ch = chunks_[ci];
         std::vector<MFItem> items;
@@ -918,23 +905,16 @@ void MFEngine::build_chunks(int nchunks) {
         ch.nctr = nctr;
         if (ch.nitems == 0) continue;
         ch.items = upload(items, ch.st);
-        ch.ctr.alloc(sizeof(int) * (size_t)std::max(nctr, 1));
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(ch.st, cudaStreamCaptureModeThreadLocal));
-        cudaError_t err = launch_mf_stage(ch.items.as<MFItem>(), ch.nitems, classes_d_.as<MFClass>(), ch.ctr.as<int>(),
-                                          ch.nctr, 1, 0, err_d_.as<int>(), smem_, table_bytes_, cgrid, ch.st);
-        cudaError_t e2 = cudaStreamEndCapture(ch.st, &g);
-        if (err != cudaSuccess || e2 != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            throw Error(SGDG_ECUDA, std::string("graph capture: ") + cudaGetErrorString(err != cudaSuccess ? err : e2));
-        }
-        cudaError_t e3 = cudaGraphInstantiate(&ch.graph, g, 0);
-        cudaGraphDestroy(g);
-        if (e3 != cudaSuccess) {
-            ch.graph = nullptr;
-            throw Error(SGDG_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e3));
-        }
+        ch.ctr.alloc(sizeof(int) * (size_t)(nctr + 1));
+        CK(cudaMemsetAsync(ch.ctr.p, 0, ch.ctr.bytes, ch.st));
     }
+    // A chunk holds a fraction of the groups, so its phases wait on one another
+    // more; with one CTA per SM per launch, as many chunks' launches as CTAs fit
+    // on an SM run side by side and cover each other's waits.  Fewer chunks with
+    // groups share the GPU.
+    int used = 0;
+    for (const Chunk& ch : chunks_) used += ch.nitems > 0;
+    for (Chunk& ch : chunks_) ch.grid = std::max(sms_, grid_ / std::max(used, 1));
     for (Chunk& ch : chunks_) CK(cudaStreamSynchronize(ch.st));
 }
 
@@ -981,8 +961,9 @@ void MFEngine::step_host(const double* in, double* out, int64_t nsteps, int nchu
             CK(launch_f64_to_f32(c.y.as<double>() + (size_t)r[1] * c.Ns, c.u0.as<float>() + (size_t)r[1] * c.Ns,
                                  (int64_t)r[2] * c.Ns, ch.st));
         }
-        if (ch.graph)
-            for (int64_t i = 0; i < nsteps; i++) CK(cudaGraphLaunch(ch.graph, ch.st));
+        for (int64_t i = 0; i < nsteps; i++)
+            CK(launch_mf_step(ch.items.as<MFItem>(), ch.nitems, classes_d_.as<MFClass>(), ch.ctr.as<int>(), ch.nctr,
+                              err_d_.as<int>(), smem_, table_bytes_, ch.grid, ch.st));
         copies(ch, false);
     }
     for (Chunk& ch : chunks_) CK(cudaStreamSynchronize(ch.st));
@@ -993,8 +974,9 @@ void MFEngine::step_host(const double* in, double* out, int64_t nsteps, int nchu
 void MFEngine::step(int64_t nsteps) {
     plan();
     if (nitems_ == 0 || nsteps <= 0) return;
-    if (!graph_) capture();
-    for (int64_t i = 0; i < nsteps; i++) CK(cudaGraphLaunch(graph_, stream_));
+    for (int64_t i = 0; i < nsteps; i++)
+        CK(launch_mf_step(items_d_.as<MFItem>(), nitems_, classes_d_.as<MFClass>(), ctr_d_.as<int>(), nctr_,
+                          err_d_.as<int>(), smem_, table_bytes_, grid_, stream_));
 }
 
 int MFEngine::check_error() {

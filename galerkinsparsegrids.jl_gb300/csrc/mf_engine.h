@@ -75,7 +75,7 @@ class MFEngine {
     // Every live state from host_in (id order, like upload_all), nsteps RK4
     // steps, the results to host_out (may equal host_in); synchronises.  The
     // groups are split into nchunks chunks, each with its own work list,
-    // counters, graph and stream, so one chunk's copies overlap the others'
+    // counters and stream, so one chunk's copies overlap the others'
     // steps.  Host memory should be pinned for the copies to overlap.
     void step_host(const double* host_in, double* host_out, int64_t nsteps, int nchunks);
 
@@ -135,11 +135,11 @@ class MFEngine {
     void build_items(std::vector<MFItem>& items, int& nctr, bool pass_only = false,
                      const std::map<std::pair<int, int>, MFTile>* shapes = nullptr, int chunk = 0, int nchunks = 1,
                      std::vector<std::array<int, 3>>* ranges = nullptr);
+    std::vector<WLClass> wl_classes() const;  // the classes as the work list sees them
     const STable& stab(int k, int n);
     const TTables& ttab(int k, int n);
     const QTable& qtab(int k, int n);
-    void capture();
-    void drop_graph();
+    void drop_chunks();
     Solve& at(int id);
     const Solve& at(int id) const;
 
@@ -155,12 +155,11 @@ class MFEngine {
     size_t smem_ = 0;
     int table_bytes_ = 0;  // shared-memory operator table reserved ahead of the tile
     bool dirty_ = true;
-    cudaGraphExec_t graph_ = nullptr;
     struct Chunk {  // step_host's pipeline stage
         DevBuf items, ctr;
         int nitems = 0, nctr = 0;
+        int grid = 0;
         cudaStream_t st = nullptr;
-        cudaGraphExec_t graph = nullptr;
         std::vector<std::array<int, 3>> ranges;  // (class, first slot, slots)
     };
     std::vector<Chunk> chunks_;

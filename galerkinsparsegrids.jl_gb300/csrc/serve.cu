@@ -12,7 +12,7 @@
 //   3. retires the requests that are done: their state goes to host memory
 //      and their device memory is freed for the next admissions.
 // Only classes whose membership changed are re-laid out, so a join or leave
-// costs one class arena rebuild and a graph re-capture.
+// costs one class arena rebuild and a new work list.
 //
 // Each request's columns are computed exactly as when it runs alone (tiles
 // never mix columns' arithmetic), so its result does not depend on the mix.

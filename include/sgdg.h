@@ -212,7 +212,7 @@ int sgdg_vlasov_write_h5(const sgdg_vlasov *v, const char *path, int64_t nout, c
 /* Many solves of uneven D, k, n advance together: each RK4 step is one
  * persistent launch over the pencil tiles of every solve and every stage
  * (groups of solves reach the stages at different times; a stage waits only
- * for its own group's previous stage), replayed from a CUDA graph.  State
+ * for its own group's previous stage).  State
  * stays on the device between calls. */
 int sgdg_batch_create(sgdg_batch **out);
 int sgdg_batch_destroy(sgdg_batch *b);
