@@ -67,22 +67,24 @@ __device__ __forceinline__ int ld_relaxed(const int* p) {
 }
 
 // Applies the pencil's 1D operator to src for every (row block, column quad)
-// of the tile and hands each result to emit(rb, jq, out).  In the
+// of the tile and hands each result to emit(rb, jq, out), or value by value to
+// emit_one(rb, jq, i CPT + c, value).  In the
 // hierarchical basis a coarse row block couples to most blocks of the pencil
 // (row block 0 to all of them) while a fine one couples to O(levels), so the
 // coarse rows (rb < rlong) are shared by a warp -- lanes split the block list,
 // a fixed shuffle tree sums -- and the fine rows get one thread each.
-template <int K, int CPT, class Emit>
+template <int K, int CPT, class Emit, class EmitOne>
 __device__ __forceinline__ void apply_rows(const OpTable& T, const float* __restrict__ src, int W, int nrb, int lwq,
-                                           int rlong, Emit&& emit) {
+                                           int rlong, Emit&& emit, EmitOne&& emit_one) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nql = rlong << lwq;
     for (int u = warp; u < nql; u += kMFThreads / 32) {
         const int rb = u >> lwq, jq = u & ((1 << lwq) - 1);
         float o[K][CPT];
         sweep<K, CPT>(T, src, W, nrb, rb, jq, lane, 32, o);
-        warp_sum<K, CPT>(o);
-        if (lane == 0) emit(rb, jq, o);
+        int at;
+        const float r = warp_sum<K, CPT>(o, lane, at);
+        if (!(lane & 1)) emit_one(rb, jq, at, r);
     }
     const int nq = nrb << lwq;
     for (int q = nql + (int)threadIdx.x; q < nq; q += kMFThreads) {
@@ -257,15 +259,20 @@ __device__ void pass_tile(const MFItem& it, const MFClass& C, const OpTable& T, 
                 *reinterpret_cast<float2*>(yp) = make_float2(o[i][0], o[i][1]);
         }
     };
+    auto store_one = [&](float* dst, int rb, int jq, int at, float v) {
+        dst[(rb * K + at / CPT) * W + jq * CPT + at % CPT] = v;
+    };
     // result Z of the tile: X -> Y, or for the wave's D_d D_d without the
     // squared table X -> Y -> X (X is dead after the first sweep)
     float* Z = Y;
     if (TWICE) {
-        apply_rows<K, CPT>(T, X, W, nrb, lwq, rlong, [&](int rb, int jq, float(&o)[K][CPT]) { store(Y, rb, jq, o); });
+        apply_rows<K, CPT>(T, X, W, nrb, lwq, rlong, [&](int rb, int jq, float(&o)[K][CPT]) { store(Y, rb, jq, o); },
+                           [&](int rb, int jq, int at, float v) { store_one(Y, rb, jq, at, v); });
         __syncthreads();
         Z = X;
     }
-    apply_rows<K, CPT>(T, TWICE ? Y : X, W, nrb, lwq, rlong, [&](int rb, int jq, float(&o)[K][CPT]) { store(Z, rb, jq, o); });
+    apply_rows<K, CPT>(T, TWICE ? Y : X, W, nrb, lwq, rlong, [&](int rb, int jq, float(&o)[K][CPT]) { store(Z, rb, jq, o); },
+                       [&](int rb, int jq, int at, float v) { store_one(Z, rb, jq, at, v); });
     // the partial sums of this group's previous pass must be complete
     if (!(it.flags & TILE_WAIT_IN) && it.wait_ctr >= 0 && tid == 0) wait_counter(ctr + it.wait_ctr, it.wait_need, err);
     __syncthreads();

@@ -88,15 +88,42 @@ __device__ __forceinline__ void sweep(const OpTable& T, const float* __restrict_
         for (int c = 0; c < CPT; c++) out[i][c] = acc[i][c].x + acc[i][c].y;
 }
 
-// The shuffle tree that sums a warp-cooperative row's lane partials.
+// Sums a warp-cooperative row's lane partials o[i][c] by the pairing of a
+// shuffle butterfly over lane distances 16, 8, 4, 2, 1, but exchanges halves of
+// the values a lane still holds instead of all of them: lanes with the
+// distance's bit clear go on with the first half, the others with the last (an
+// odd number's middle one with both), each adding its partner's copy.  A 3 x 4
+// block takes 13 shuffles and additions instead of 60, and every sum has the
+// butterfly's value.  Returns the sum the lane ends up with; at is its index
+// i CPT + c (several lanes may hold one).
+template <int N>
+__device__ __forceinline__ float warp_sum_halves(float (&v)[N], int lane, int o, int& at) {
+    if constexpr (N == 1) {
+        float r = v[0];
+        for (; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        return r;
+    } else {
+        constexpr int H = (N + 1) / 2;
+        const bool up = lane & o;
+        float h[H];
+#pragma unroll
+        for (int j = 0; j < H; j++) {
+            const float keep = up ? v[N - H + j] : v[j], give = up ? v[j] : v[N - H + j];
+            h[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        at += up ? N - H : 0;
+        return warp_sum_halves<H>(h, lane, o >> 1, at);
+    }
+}
 template <int K, int CPT>
-__device__ __forceinline__ void warp_sum(float (&o)[K][CPT]) {
+__device__ __forceinline__ float warp_sum(const float (&o)[K][CPT], int lane, int& at) {
+    float v[K * CPT];
 #pragma unroll
     for (int i = 0; i < K; i++)
 #pragma unroll
-        for (int c = 0; c < CPT; c++)
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) o[i][c] += __shfl_xor_sync(0xffffffffu, o[i][c], off);
+        for (int c = 0; c < CPT; c++) v[i * CPT + c] = o[i][c];
+    at = 0;
+    return warp_sum_halves<K * CPT>(v, lane, 16, at);
 }
 
 }  // namespace sgdg
