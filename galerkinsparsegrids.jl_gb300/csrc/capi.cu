@@ -362,15 +362,18 @@ struct sgdg_vlasov {
     }
 };
 
-// RK4 steps of the plain form.  From `least` steps on, `per` steps are captured
-// as a graph (launches inside it are programmatic dependents, so one comes up
-// while the one before it runs) and replayed; fewer, and what is left over, are
-// launched as they are.  The evolvers take 8 steps (32 launches) from 8 on; a
-// Vlasov step alone is 40 to 136 launches, whose instantiation (0.2 ms at 72)
-// pays from 16 steps on (634 against 676 us per step).
+// RK4 steps of the plain form: launched as they are, or `per` steps captured as a
+// graph and replayed where the run is long enough to pay for the capture (launches
+// are programmatic dependents either way).  A graph costs a call about 110 us for
+// 32 launches and saves 0.5 to 1 us per step (us per step, launched and replayed:
+// 2D wave k=3 n=5 9.26 and 8.76, 4D advection k=2 n=6 20.1 and 19.1, 3D wave k=3
+// n=7 36.4 and 35.8; Vlasov 2x2v k=2 n=8, whose step alone is captured, 676 and
+// 634 with 72 launches, 0.2 ms).
+constexpr int64_t kGraphSteps = 256;       // of 4 launches
+constexpr int64_t kGraphStepsVlasov = 16;  // of 20 to 100
 class StepGraph {
    public:
-    StepGraph(int64_t per, int64_t least) : per_(per), least_(least) {}
+    StepGraph(int64_t per, bool use) : per_(per), use_(use) {}
     StepGraph(const StepGraph&) = delete;
     StepGraph& operator=(const StepGraph&) = delete;
     ~StepGraph() {
@@ -379,7 +382,7 @@ class StepGraph {
     // launches nsteps steps on st (never the legacy stream), steps(n) launching n of them
     template <class Steps>
     void run(int64_t nsteps, cudaStream_t st, Steps&& steps) {
-        if (nsteps >= least_ && !exec_) capture(st, steps);
+        if (use_ && nsteps >= per_ && !exec_) capture(st, steps);
         for (; exec_ && nsteps >= per_; nsteps -= per_) CK(cudaGraphLaunch(exec_, st));
         CK(steps(nsteps));
     }
@@ -402,7 +405,8 @@ class StepGraph {
             throw Error(SGDG_ECUDA, std::string("instantiate: ") + cudaGetErrorString(e3));
         }
     }
-    const int64_t per_, least_;
+    const int64_t per_;
+    const bool use_;
     cudaGraphExec_t exec_ = nullptr;
 };
 
@@ -719,7 +723,7 @@ static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, do
     CK(cudaMemcpyAsync(y, y0, b, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
     const auto steps = out_steps(nsteps, nout);
-    StepGraph graph(8, 8);
+    StepGraph graph(8, nsteps >= kGraphSteps);
     int64_t done = 0;
     int bad = 0;
     for (int i = 0; i < nout; i++) {
@@ -780,7 +784,7 @@ struct PlainScratch {
     template <class Mat>
     bool run(const Mat& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
         int bad = 0;
-        StepGraph graph(8, 8);
+        StepGraph graph(8, nsteps >= kGraphSteps);
         CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
         CK(launch_plain_interleave(A.m, nv, nb, y, u0.as<double>(), st));
         graph.run(nsteps, st, [&](int64_t n) {
@@ -1193,7 +1197,7 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
     // the whole) of n2m fused with the stage update; returns whether a stage
     // was not finite
     auto run = [&](bool whole) {
-        StepGraph graph(1, 16);
+        StepGraph graph(1, nsteps >= kGraphStepsVlasov);
         auto launch = [&](int64_t n) {
             cudaError_t e = cudaSuccess;
             for (int64_t i = 0; i < n; i++)

@@ -143,10 +143,10 @@ __device__ __forceinline__ void row_sum(const DevCSR& A, int64_t b, int64_t e, C
 
 __device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
 
-// RK4 stage update of one element: k its right-hand side, y its state, acc and
-// uout at element `o` of the scratch vectors
-__device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double* y, int64_t o) {
-    double yy = *y, aa = rk.stage == 1 ? 0.0 : rk.acc[o], un;
+// RK4 stage update of one element: k its right-hand side, yy its state and aa its
+// accumulator (from y and acc[o]), which go back there and uout[o]
+__device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double yy, double aa, double* y, int64_t o) {
+    double un;
     rk_stage(rk.stage, rk.dt, rk.hdt, rk.dt6, k, yy, aa, un);
     if (rk.stage == 4)
         *y = yy;
@@ -157,7 +157,9 @@ __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double*
 }
 
 // Block rb's rows, 2^bin lanes each: out.one(row, j, sum) by the lane that
-// holds vector j's sum, or out.all(row, sums) where one lane holds them all.
+// holds vector j's sum, or out.all(row, sums) where one lane holds them all; what
+// the lane needs for that besides is loaded before the sum (out.fetch), so that
+// its latency passes under the gathers.
 template <int VS, int NV, class Out>
 __device__ __forceinline__ void bin_rows(const DevCSR& A, int bin, int64_t rb, const double* x, int64_t stride,
                                          const Out& out) {
@@ -174,15 +176,17 @@ __device__ __forceinline__ void bin_rows(const DevCSR& A, int bin, int64_t rb, c
     CsrAhead ahead;
     csr_fetch<VS>(A, b + lane, e, ahead);
     pdl_wait();
-    double s[NV];
-    row_sum<VS, NV>(A, b, e, ahead, x, lane, stride, s);
     bool stores;
     const int owner = csr_owner<VS, NV>(lane, stores);
+    typename Out::Fetched f;
+    if (row >= 0 && stores) out.fetch(row, owner, f);
+    double s[NV];
+    row_sum<VS, NV>(A, b, e, ahead, x, lane, stride, s);
     if (row < 0 || !stores) return;
     if (owner >= 0)
-        out.one(row, owner, s[0]);
+        out.one(row, owner, s[0], f);
     else
-        out.all(row, s);
+        out.all(row, s, f);
 }
 
 // the same for slices
@@ -212,6 +216,11 @@ __device__ __forceinline__ void bin_rows(const DevSliced& A, int64_t rb, const d
     CsrAhead t;
     fetch(0, t);
     pdl_wait();
+    const int lane = l32 % VS;
+    bool stores;
+    const int owner = csr_owner<VS, NV>(lane, stores);
+    typename Out::Fetched f;
+    if (row >= 0 && stores) out.fetch(row, owner, f);
     double s[NV];
 #pragma unroll
     for (int j = 0; j < NV; j++) s[j] = 0.0;
@@ -232,10 +241,7 @@ __device__ __forceinline__ void bin_rows(const DevSliced& A, int64_t rb, const d
         }
         t = next;
     }
-    const int lane = l32 % VS;
     csr_reduce<VS, NV>(s, lane);
-    bool stores;
-    const int owner = csr_owner<VS, NV>(lane, stores);
     if constexpr (Out::kTogether && ((NV == 4 && VS >= 4) || (NV == 2 && VS >= 2))) {
         // the row's sums to its first lane (csr_owner's lanes)
         const double mine = s[0];
@@ -243,14 +249,14 @@ __device__ __forceinline__ void bin_rows(const DevSliced& A, int64_t rb, const d
         for (int j = 0; j < NV; j++)
             s[j] = __shfl_sync(0xffffffffu, mine,
                                NV == 4 ? (j & 2 ? VS / 2 : 0) + (j & 1 ? VS / 4 : 0) : (j & 1 ? VS / 2 : 0), VS);
-        if (row >= 0 && lane == 0) out.all(row, s);
+        if (row >= 0 && lane == 0) out.all(row, s, f);
         return;
     }
     if (row < 0 || !stores) return;
     if (owner >= 0)
-        out.one(row, owner, s[0]);
+        out.one(row, owner, s[0], f);
     else
-        out.all(row, s);
+        out.all(row, s, f);
 }
 
 template <int NV, class Out>
@@ -282,20 +288,35 @@ __device__ __forceinline__ void block_rows(const DevCSR& A, int64_t rb, const do
     }
 }
 
-// the stage update of nv of the NV solves of a set, solve j's state at y + j m
+// The stage update of nv of the NV solves of a set, solve j's state at y + j m.
+// One solve, whose time is latency, fetches its state and accumulator before the
+// sum (3D wave k=3 n=7 38.1 -> 35.8 us per step); sets, bound by the FP64 pipe,
+// after it (256 of them 4.49 ms, 4.59 with the registers held across the sum).
 template <int NV>
 struct RkOut {
     static constexpr bool kTogether = false;
+    struct Fetched {
+        double y, acc;
+    };
     const CsrRK& rk;
     double* y;
     int64_t m;
     int nv;
-    __device__ __forceinline__ void one(int64_t row, int j, double s) const {
-        if (j < nv) csr_rk_update(rk, s, y + row + j * m, row * NV + j);
+    __device__ __forceinline__ void load(int64_t row, int j, Fetched& f) const {
+        f.y = y[row + j * m];
+        f.acc = rk.stage != 1 ? rk.acc[row * NV + j] : 0.0;
     }
-    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+    __device__ __forceinline__ void fetch(int64_t row, int, Fetched& f) const {
+        if constexpr (NV == 1) load(row, 0, f);
+    }
+    __device__ __forceinline__ void one(int64_t row, int j, double s, Fetched& f) const {
+        if (j >= nv) return;
+        if constexpr (NV > 1) load(row, j, f);
+        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j);
+    }
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], Fetched& f) const {
 #pragma unroll
-        for (int j = 0; j < NV; j++) one(row, j, s[j]);
+        for (int j = 0; j < NV; j++) one(row, j, s[j], f);
     }
 };
 
@@ -361,7 +382,7 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
     for (int q = A.long_seg[i]; q < A.long_seg[i + 1]; q++) s += A.partial[q];
     const int64_t row = A.long_row[i];
     if (!SGDG_IN(row, A.m)) return;
-    csr_rk_update(rk, s, y + row, row);
+    csr_rk_update(rk, s, y[row], rk.stage == 1 ? 0.0 : rk.acc[row], y + row, row);
 }
 
 // NV adjacent vectors of an interleaved set (element i of vector j at
@@ -369,14 +390,16 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
 template <int NV>
 struct SweepOut {
     static constexpr bool kTogether = false;
+    struct Fetched {};
     double* y;
     int64_t stride;
     int* nonfinite;
-    __device__ __forceinline__ void one(int64_t row, int j, double s) const {
+    __device__ __forceinline__ void fetch(int64_t, int, Fetched&) const {}
+    __device__ __forceinline__ void one(int64_t row, int j, double s, const Fetched&) const {
         y[row * stride + j] = s;
         if (nonfinite && not_finite(s)) *nonfinite = 1;
     }
-    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], const Fetched& f) const {
         double* p = y + row * stride;
         if constexpr (NV == 4)
             asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(s[0]), "d"(s[1]), "d"(s[2]), "d"(s[3])
@@ -384,7 +407,7 @@ struct SweepOut {
         else if constexpr (NV == 2)
             *reinterpret_cast<double2*>(p) = make_double2(s[0], s[1]);
         else
-            one(row, 0, s[0]);
+            one(row, 0, s[0], f);
     }
 };
 
@@ -411,8 +434,10 @@ struct PointsOut {
     const double *v, *F;
     double* out;
     int64_t n;
-    __device__ __forceinline__ void one(int64_t, int, double) const {}
-    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV]) const {
+    struct Fetched {};
+    __device__ __forceinline__ void fetch(int64_t, int, Fetched&) const {}
+    __device__ __forceinline__ void one(int64_t, int, double, const Fetched&) const {}
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], const Fetched&) const {
         out[row] = point_product<NV / 2>(v, F, n, row, s);
     }
 };
@@ -438,11 +463,15 @@ struct ApplyOut {
     double* y;
     int* seen;
     int call;
-    __device__ __forceinline__ void one(int64_t row, int, double s) const {
+    struct Fetched {
+        double x;
+    };
+    __device__ __forceinline__ void fetch(int64_t row, int, Fetched& f) const { f.x = __ldca(x + row); }
+    __device__ __forceinline__ void one(int64_t row, int, double s, const Fetched& f) const {
         y[row] = s;
-        if (not_finite(__ldca(x + row))) *seen = call;
+        if (not_finite(f.x)) *seen = call;
     }
-    __device__ __forceinline__ void all(int64_t row, const double (&s)[1]) const { one(row, 0, s[0]); }
+    __device__ __forceinline__ void all(int64_t row, const double (&s)[1], const Fetched& f) const { one(row, 0, s[0], f); }
 };
 __global__ void __launch_bounds__(256, 4) k_apply(DevSliced A, const double* x, double* y, int* seen, int call) {
     block_rows<1>(A, blockIdx.x, x, 1, ApplyOut{x, y, seen, call});

@@ -37,10 +37,10 @@ SHAPES = [(1, 1, 2, "sparse"), (1, 5, 8, "sparse"), (2, 1, 4, "sparse"), (2, 4, 
 @pytest.mark.gpu
 @pytest.mark.parametrize("D,k,n,scheme", SHAPES)
 def test_evolvers_against_the_whole_operator(sgdg, D, k, n, scheme):
-    # 8-step graphs and what is left over of them (1, 7, 8, 17 steps); per step
+    # launched as they are, and as 8-step graphs and what is left over of them; per step
     # a result is off by a few roundings of dt |A| |y|, plus the dropped
-    # entries (2e-12 of the largest): 1e-10 of the state covers 17 steps at
-    # dt |A| <= 1
+    # entries (2e-12 of the largest): 1e-10 of the state covers 259 steps at
+    # dt |A| <= 1/8
     op = sgdg.SparseGridOperator(D, k, n, scheme)
     rng = np.random.default_rng(D * 100 + k * 10 + n)
     N = op.N
@@ -50,12 +50,12 @@ def test_evolvers_against_the_whole_operator(sgdg, D, k, n, scheme):
     for A, y, evolve in ((W, rng.standard_normal(2 * N), "wave"), (G, rng.standard_normal(N), "advect")):
         dt = 1.0 / max(np.abs(A).sum(1).max(), 1e-3) if evolve == "advect" else \
             1.0 / np.sqrt(max(np.abs(A).sum(1).max(), 1e-3))
-        for steps in (1, 7, 8, 17):
-            ref = rk4(A, y, dt, steps)
+        for steps, h in ((1, dt), (7, dt), (17, dt), (259, dt / 8)):
+            ref = rk4(A, y, h, steps)
             if evolve == "wave":
-                _, st = sgdg.wave_evolve(D, k, n, y[:N], y[N:], 0.0, steps * dt, nsteps=steps, scheme=scheme, op=op)
+                _, st = sgdg.wave_evolve(D, k, n, y[:N], y[N:], 0.0, steps * h, nsteps=steps, scheme=scheme, op=op)
             else:
-                _, st = sgdg.advect_evolve(D, k, n, a, y, 0.0, steps * dt, nsteps=steps, scheme=scheme, op=op)
+                _, st = sgdg.advect_evolve(D, k, n, a, y, 0.0, steps * h, nsteps=steps, scheme=scheme, op=op)
             assert np.linalg.norm(st[-1] - ref) <= 1e-10 * np.linalg.norm(ref), (evolve, steps)
 
 
