@@ -10,7 +10,9 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <queue>
 
 #include "mf_engine.h"
 
@@ -26,6 +28,16 @@ cudaError_t launch_f64_to_f32(const double* a, float* b, int64_t n, cudaStream_t
 cudaError_t launch_f32_to_f64(const float* a, double* b, int64_t n, cudaStream_t st);
 
 static constexpr size_t kWaveLag = 3;       // steps between a group's consecutive phases in the work list
+// List order of the work list (mf_work_list): up to these bytes of vectors (L2
+// holds 126 MB, and the list does not keep the groups in flight few), this many
+// items times groups (the host's work), and from these items per phase on: below,
+// every CTA is ahead of the list's end and only waits longer.  us for 20 steps of
+// uneven advection solves (D 2-3, k 2-4, n 4-7), wavefront and list order: 128
+// solves 6614 and 5804, 96 4905 and 4349, 40 3773 and 3469, 20 2750 and 2750, 8
+// 1534 and 1575; eight served requests 7.9 and 8.7 ms.  CTAs it reckons with: all
+// that are resident.
+constexpr double kListBytes = 96e6, kListWork = 4e6, kListItems = 300;
+constexpr int kListCtas = 456;
 static constexpr int kStageKey = 1 << 22;   // counter keys of a whole-step list: key + (stage - 1) * kStageKey
 
 // The wave's D_d D_d on a pencil of line length lmax: one sweep of the
@@ -524,9 +536,12 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
     };
     struct Group {
         std::vector<Phase> phases;
+        int k = 0, sweeps = 1;  // of its items' cost
     };
     std::vector<Group> groups;
     size_t smem = 64;
+    double bytes = 0;     // stage inputs, partial sums and FP64 state of all groups
+    bool chains = true;   // every group's phases follow one another
     const int auto_wlog = mf_auto_wlog(cls, pass_only);
     for (size_t ci = 0; ci < cls.size(); ci++) {
         const WLClass& c = cls[ci];
@@ -696,6 +711,10 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
                         grp.phases.push_back(std::move(q));
                     }
             }
+            grp.k = k;
+            grp.sweeps = sp.kind == MF_KIND_WAVE ? 2 : 1;
+            chains = chains && sp.kind != MF_KIND_VLASOV && rk;
+            bytes += double(s1 - s0) * double(24 * c.Ns + 4 * c.N);
             groups.push_back(std::move(grp));
         }
     }
@@ -709,6 +728,80 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
             if (!ctr_of[g].count(ph.done_key)) ctr_of[g][ph.done_key] = nctr++;
             items_of[g][ph.done_key] += (int)ph.items.size();
         }
+    auto emit = [&](size_t g, const Phase& ph, MFItem it) {
+        it.done_ctr = ctr_of[g].at(ph.done_key);
+        it.wait_ctr = ph.wait_key >= 0 ? ctr_of[g].at(ph.wait_key) : -1;
+        it.wait_need = ph.wait_key >= 0 ? items_of[g].at(ph.wait_key) : 0;
+        it.win_ctr = ph.win_key >= 0 ? ctr_of[g].at(ph.win_key) : -1;
+        it.win_need = ph.win_key >= 0 ? items_of[g].at(ph.win_key) : 0;
+        items.push_back(it);
+    };
+    size_t total = 0;
+    for (auto& g : groups)
+        for (const Phase& ph : g.phases) total += ph.items.size();
+    if (chains && groups.size() > 1 && bytes <= kListBytes && double(total) * double(groups.size()) <= kListWork &&
+        total > kListItems * mf_chain(cls, pass_only)) {
+        // List order: the items as kListCtas CTAs would take them, each free CTA
+        // the item of the group with the most work ahead (its remaining phases)
+        // among the groups whose next output would not wait, else of the one whose
+        // wait ends first.  An item's cycles are estimated from its elements, and
+        // its output (the last third) waits for the group's previous phase.
+        struct State {
+            size_t phase = 0, item = 0;
+            double ready = 0, done = 0;  // end of the previous phase; of this one's items so far
+            std::vector<double> ahead;   // per phase: estimated cycles from its start on
+        };
+        auto cost = [](const Group& g, const MFItem& it) {
+            const double e = double(it.W) * g.k * double(1 << (it.lmax - 1));
+            return 8000.0 + e * (4.0 + 0.7 * g.k * g.sweeps + (it.flags & TILE_RK ? 4.0 : 0.0));
+        };
+        std::vector<State> state(groups.size());
+        for (size_t g = 0; g < groups.size(); g++) {
+            const auto& ph = groups[g].phases;
+            state[g].ahead.assign(ph.size() + 1, 0.0);
+            for (size_t p = ph.size(); p-- > 0;) {
+                double sum = 0, most = 0;
+                for (const MFItem& it : ph[p].items) {
+                    sum += cost(groups[g], it);
+                    most = std::max(most, cost(groups[g], it));
+                }
+                state[g].ahead[p] = state[g].ahead[p + 1] + std::max(most, sum / kListCtas);
+            }
+        }
+        std::priority_queue<double, std::vector<double>, std::greater<double>> cta;
+        for (int i = 0; i < kListCtas; i++) cta.push(0.0);
+        for (size_t left = total; left > 0; left--) {
+            const double t = cta.top();
+            cta.pop();
+            size_t best = groups.size();
+            double best_wait = 0;
+            for (size_t g = 0; g < groups.size(); g++) {
+                State& s = state[g];
+                const auto& ph = groups[g].phases;
+                while (s.phase < ph.size() && s.item == ph[s.phase].items.size()) {  // on to the next phase
+                    s.ready = std::max(s.ready, s.done);
+                    s.phase++;
+                    s.item = 0;
+                }
+                if (s.phase == ph.size()) continue;
+                const double c = cost(groups[g], ph[s.phase].items[s.item]);
+                const double wait = std::max(0.0, s.ready - (t + 0.65 * c));
+                if (best == groups.size() || wait < best_wait ||
+                    (wait == best_wait && s.ahead[s.phase] > state[best].ahead[state[best].phase])) {
+                    best = g;
+                    best_wait = wait;
+                }
+            }
+            State& s = state[best];
+            const Phase& ph = groups[best].phases[s.phase];
+            const MFItem& it = ph.items[s.item++];
+            const double c = cost(groups[best], it), end = std::max(t + 0.65 * c, s.ready) + 0.35 * c;
+            s.done = std::max(s.done, end);
+            cta.push(end);
+            emit(best, ph, it);
+        }
+        return smem;
+    }
     // wavefront order: a phase of depth p of stage s (0-based) of group g in
     // step s SO + g + kWaveLag p, older stages and then deeper phases (older
     // groups) first within a step, so a phase's predecessors were handed out
@@ -733,14 +826,7 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
                 const size_t g = t - t0;
                 for (const Phase& ph : groups[g].phases) {
                     if (ph.depth != (int)pp || std::max(ph.stage, 1) != st + 1) continue;
-                    for (MFItem it : ph.items) {
-                        it.done_ctr = ctr_of[g].at(ph.done_key);
-                        it.wait_ctr = ph.wait_key >= 0 ? ctr_of[g].at(ph.wait_key) : -1;
-                        it.wait_need = ph.wait_key >= 0 ? items_of[g].at(ph.wait_key) : 0;
-                        it.win_ctr = ph.win_key >= 0 ? ctr_of[g].at(ph.win_key) : -1;
-                        it.win_need = ph.win_key >= 0 ? items_of[g].at(ph.win_key) : 0;
-                        items.push_back(it);
-                    }
+                    for (const MFItem& it : ph.items) emit(g, ph, it);
                 }
             }
     return smem;

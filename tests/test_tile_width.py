@@ -27,6 +27,21 @@ def test_widths_of_untuned_tiles(sgdg, batch):
     assert np.all((it["W"] == cpt) | (it["W"] // 2 < it["Wv"]))  # no wider than its columns
 
 
+@pytest.mark.parametrize("big,small", [(40, 60), (64, 1), (3, 90)])
+def test_list_order_of_uneven_groups(sgdg, big, small):
+    # groups of very different lengths, in list order (the first two) and in
+    # wavefronts: either way a schedule whose waits point backwards and whose
+    # phases cover every element once
+    sgdg.clear_tile_shapes()
+    batch = [(ADVECT, 3, 4, 5, 0, big, 0, 0), (ADVECT, 2, 3, 4, 0, small, 0, 0), (WAVE, 2, 2, 5, 0, small, 0, 0),
+             (ADVECT, 1, 3, 6, 0, 2, 0, 0)]
+    it, spec, cls, boff, nctr = dryrun(sgdg, batch)
+    check_schedule(it, nctr)
+    check_coverage(it, spec, cls, boff)
+    check_stages(it)
+    check_rk_once(it, spec, cls, boff)
+
+
 def test_width_follows_the_items_per_phase(sgdg):
     sgdg.clear_tile_shapes()
     widest = []
