@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
 // numbers per pencil -- level tuple of the other dimensions -- instead of one
 // per level block: 36 instead of 120 for 3D n=7, and the FP64 operations, which
 // bound k_evaluate (61 % of that pipe's peak, 3.50 ms for 2^18 points at k=3),
-// fall as much (0.95 ms, of which the FP64 pipe needs 0.75).  A block's numbers are padded to a multiple of 32 bytes and
+// fall as much (0.87 ms with that pipe 91 % busy).  A block's numbers are padded to a multiple of 32 bytes and
 // loaded 32 bytes at a time: the lanes of a warp are 32 points in blocks of
 // their own, so a load costs as many L1 accesses as it has lanes, whatever its
 // width.
@@ -160,6 +160,8 @@ struct Pencils {
     int inner, pad, outer;   // k^min(D,3), the same rounded up to 4, k^(D-3) (1 for D <= 3)
     const int32_t* lmax;     // per pencil: levels along dimension 1
     const int64_t* base;     // first number of its blocks
+    const double* scale;     // product of the scales of its 1D functions (2^(1/2) at level 0, 2^(l/2) at l,
+                             // 2^((lmax)/2) on the pieces), which k_lines puts into the blocks
     const int8_t* levels;    // D - 1 levels of the other dimensions, 1-based
     const int64_t* item;     // first item (piece, cell and mode of the others) of k_lines; np + 1
     const int32_t* lev_off;  // per pencil n + 1 offsets of its level blocks
@@ -208,9 +210,10 @@ __global__ void __launch_bounds__(256)
     // within its block: the modes of dimensions 1..3 (padded), then the others
     const int in = S.inner / K;
     double* o = out + S.base[lo] + (int64_t)S.pad * S.outer * (j + (cl << (lmax - 1))) + S.pad * (mo / in) + K * (mo % in);
+    const double scale = S.scale[lo];
 #pragma unroll
     for (int m = 0; m < K; m++) {
-        o[m] = s[m];
+        o[m] = scale * s[m];
         bad = bad || (__double2hiint(s[m]) & 0x7ff00000) == 0x7ff00000;
     }
     if (bad) *nonfinite = 1;
@@ -247,24 +250,22 @@ __global__ void __launch_bounds__(kPencilPts* kPencilParts)
             const int cells = d == 0 ? l : l > 1 ? l - 1 : 0;  // log2
             int c = 0;  // 0-based
             if (cells > 0) c = x >= 1.0 ? (1 << cells) - 1 : (int)floor(pow2(cells) * x);
-            double y, scale;
+            double y;
             const double* pc;
             if (d == 0 || l == 0) {
                 y = pow2(cells + 1) * x - (double)(2 * c + 1);
-                scale = 1.4142135623730951 * ((cells & 1) ? 1.4142135623730951 * pow2(cells >> 1) : pow2(cells >> 1));
                 pc = S.pieces;
             } else {
                 y = pow2(l) * x - (double)(2 * c + 1);
-                scale = (l & 1) ? 1.4142135623730951 * pow2(l >> 1) : pow2(l >> 1);
                 pc = S.pieces + (y < 0.0 ? 1 : 2) * K * K;
             }
             if (fabs(y) <= 1.0)
 #pragma unroll
                 for (int m = 0; m < K; m++) {
-                    double s = 0.0;
+                    double s = __ldg(pc + m * K + K - 1);
 #pragma unroll
-                    for (int i = K - 1; i >= 0; i--) s = fma(s, y, __ldg(pc + m * K + i));
-                    v[m] = scale * s;
+                    for (int i = K - 2; i >= 0; i--) s = fma(s, y, __ldg(pc + m * K + i));
+                    v[m] = s;
                 }
         }
 #pragma unroll
@@ -384,7 +385,7 @@ struct EvalTables {
     size_t smem = 0;
     // the pencils along dimension 1 (k <= 5), built with the first call that uses them
     std::mutex mu;
-    DevBuf lmax, base, plevels, item, plev_off, two;
+    DevBuf lmax, base, scale, plevels, item, plev_off, two;
     Pencils P{};
     int64_t items = 0, numbers = 0;  // of k_lines; of its output
     size_t psmem = 0;
@@ -395,7 +396,8 @@ constexpr int kPencilMaxK = 5;
 // pay for k_lines (us per call, blocks and pencils: 3D k=3 n=7 64 and 69 at 1000
 // points, 90 and 69 at 4000, 3495 and 947 at 2^18; 4D k=3 n=4 90 and 104, 138 and
 // 105, 6579 and 2190; 2D k=2 n=6 39 and 41 at 4000, 64 and 46 at 16000, 524 and
-// 165; 1D k=3 n=8 39 and 45, 55 and 54, 448 and 141).
+// 165; 1D k=3 n=8 39 and 45, 55 and 54, 448 and 141; the pencils' since 5 to 25 %
+// less at 2^18 points).
 constexpr int64_t kPencilPoints = 4096, kPencilTerms = 1 << 20;
 
 // H_b[i][m] = <child b's Legendre function i, the parent's m>, G_b the same with
@@ -445,6 +447,7 @@ const Pencils& eval_pencils(EvalTables& T) {
     std::vector<int32_t> lmax, off;
     std::vector<int64_t> base, item(1, 0);
     std::vector<int8_t> lev;
+    std::vector<double> scale;
     int64_t numbers = 0;
     int L[kDMax];
     for (int b = 0; b < ix.nlev; b++) {
@@ -461,7 +464,12 @@ const Pencils& eval_pencils(EvalTables& T) {
             off.push_back((int32_t)ix.lev_off[ix.lookup_level(L)]);
             lm = l;
         }
-        for (int d = 1; d < D; d++) lev.push_back((int8_t)Lb[d]);
+        int half = lm;  // log2 of the square of the scale
+        for (int d = 1; d < D; d++) {
+            lev.push_back((int8_t)Lb[d]);
+            half += std::max(1, Lb[d] - 1);
+        }
+        scale.push_back(std::ldexp(half % 2 ? std::sqrt(2.0) : 1.0, half / 2));
         lmax.push_back(lm);
         base.push_back(numbers);
         const int64_t blocks = ix.lev_cells[b] << (lm - 1);  // finest pieces x cells of the others
@@ -470,6 +478,7 @@ const Pencils& eval_pencils(EvalTables& T) {
     }
     T.lmax = upload(lmax, nullptr);
     T.base = upload(base, nullptr);
+    T.scale = upload(scale, nullptr);
     T.plevels = upload(lev, nullptr);
     T.item = upload(item, nullptr);
     T.plev_off = upload(off, nullptr);
@@ -477,6 +486,7 @@ const Pencils& eval_pencils(EvalTables& T) {
     CK(cudaStreamSynchronize(nullptr));
     P.lmax = T.lmax.as<int32_t>();
     P.base = T.base.as<int64_t>();
+    P.scale = T.scale.as<double>();
     P.levels = T.plevels.as<int8_t>();
     P.item = T.item.as<int64_t>();
     P.lev_off = T.plev_off.as<int32_t>();
