@@ -126,9 +126,10 @@ struct sgdg_op {
     // pruned one (us per application, whole and pruned: Laplacian 2D k=3 n=7, 1.3
     // M entries, 8.3 and 8.9; 4D k=2 n=6, 1.6 M, 10.3 and 8.9; 3D k=3 n=6, 2.2 M,
     // 11.5 and 9.1; 3D k=3 n=7, 8.8 M, 28.3 and 9.0; 3D k=4 n=7, 27.8 M, 82.9 and
-    // 18.5; below 9 the time is the caller's, two launches for one), and where an element of x is not finite through the whole one
-    // after it (k_apply_whole).  Each call leaves its number in a word of its
-    // own among kApplyCalls: calls on other streams may still be in flight.
+    // 18.5; below 9 the time is the caller's, two launches for one), and where
+    // an element of x is not finite through the whole one after it
+    // (k_apply_whole).  Each call leaves its number in a word of its own among
+    // kApplyCalls: calls on other streams may still be in flight.
     static constexpr int64_t kApplyPruned = 3 << 19;
     static constexpr int kApplyCalls = 1024;
     DevBuf apply_seen;

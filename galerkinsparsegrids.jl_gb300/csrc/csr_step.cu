@@ -23,15 +23,15 @@
 // launch's blocks come up and fetch their rows, columns and values while the
 // launch before it still runs, and wait for it only before the vectors.
 //
-// Measured, from host to host: 200 steps of the 2D wave k=3 n=5 6.34 -> 2.0 ms
+// Measured, from host to host: 200 steps of the 2D wave k=3 n=5 6.34 -> 1.84 ms
 // against one solve at a time with the whole operator and plain launches; 60
-// steps of the 4D advection k=2 n=6 5.89 -> 1.5 ms; 3 steps of 48 3D waves k=3
+// steps of the 4D advection k=2 n=6 5.89 -> 1.21 ms; 3 steps of 48 3D waves k=3
 // n=7 11.8 -> 2.6 ms (0.87 ms per step, of which the FP64 pipe needs 0.74).
 // In slices against rows: the single 3D wave 46.9 -> 38.1 us per step, 256 of
 // them 4.80 -> 4.49 ms, the Vlasov step below 810 -> 634 us.  Vlasov 2x2v k=2
-// n=8: 2595 -> 627 us per step against the assembled transforms, of which the
-// FP64 pipe needs 240 (a k_sweep<4> keeps it 78 % busy) and about 150 are the
-// latency of 56 launches; n=5 296 -> 125 us.
+// n=8: 2595 -> 540 us per step against the assembled transforms, of which the
+// FP64 pipe needs 240 and about 150 are the latency of 56 launches; n=5 296 ->
+// 104 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -427,6 +427,16 @@ __device__ __forceinline__ double point_product(const double* __restrict__ v, co
     return __dadd_rn(-c1, c2);
 }
 
+// The row block of one of a sweep's n blocks.  The slices ascend by row length;
+// a grid of more blocks than are resident together takes the long rows first, so
+// that short ones fill its end (8 steps of Vlasov 2x2v k=2 n=8 4885 -> 4511 us,
+// k=3 n=6 4288 -> 4112); a smaller one starts them all at once and is faster in
+// ascending order (k=2 n=7 2529 and 2343 us, n=6 1459 and 1279).
+constexpr unsigned kSweepResident = 152 * (768 / kSliceThreads);  // SMs; threads at 80 registers
+__device__ __forceinline__ int sweep_block(int n) {
+    return gridDim.x * gridDim.y > kSweepResident ? n - 1 - (int)blockIdx.x : (int)blockIdx.x;
+}
+
 // the products of a row's P = NV values
 template <int NV>
 struct PointsOut {
@@ -444,15 +454,16 @@ struct PointsOut {
 template <int NV>
 __global__ void __launch_bounds__(256, 3)
     k_sweep_points(DevSliced A, const double* x, const double* v, const double* F, double* out) {
-    block_rows<NV>(A, blockIdx.x, x, NV, PointsOut<NV>{v, F, out, A.m});
+    block_rows<NV>(A, sweep_block(gridDim.x), x, NV, PointsOut<NV>{v, F, out, A.m});
 }
 
-// One sweep y = T x of a transform along one dimension or a few, for sets of NV of `stride` interleaved vectors; blockIdx.y: the set.
+// One sweep y = T x of a transform along one dimension or a few, for sets of NV
+// of `stride` interleaved vectors; blockIdx.y: the set.
 template <int NV>
 __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
     k_sweep(DevSliced A, const double* x, double* y, int64_t stride, int* nonfinite) {
     const int64_t o = (int64_t)blockIdx.y * NV;
-    block_rows<NV>(A, blockIdx.x, x + o, stride, SweepOut<NV>{y + o, stride, nonfinite});
+    block_rows<NV>(A, sweep_block(gridDim.x), x + o, stride, SweepOut<NV>{y + o, stride, nonfinite});
 }
 
 // One application y = A x with the pruned operator; an element of x that is not
@@ -507,7 +518,7 @@ __global__ void __launch_bounds__(256, 4)
         pdl_wait();
         return;
     }
-    block_rows<1>(A, blockIdx.x, x, 1, SweepOut<1>{y + blockIdx.y, P, nullptr});
+    block_rows<1>(A, sweep_block(A.bin_block[kCsrBins]), x, 1, SweepOut<1>{y + blockIdx.y, P, nullptr});
 }
 
 // the same for P = 2D interleaved vectors pt[i 2D + d]
@@ -543,13 +554,13 @@ static int grid_for(int64_t threads) {
 // a launch that may come up while the one before it in the stream still runs
 // (its kernel calls pdl_wait before it touches what that one writes)
 template <class... P, class... Q>
-static void launch_dependent(void (*kernel)(P...), dim3 grid, cudaStream_t st, Q... args) {
+static void launch_dependent(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, Q... args) {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = grid;
-    c.blockDim = dim3(256);
+    c.blockDim = dim3((unsigned)threads);
     c.stream = st;
     c.attrs = &at;
     c.numAttrs = 1;
@@ -557,13 +568,16 @@ static void launch_dependent(void (*kernel)(P...), dim3 grid, cudaStream_t st, Q
 }
 
 template <class Mat>
+constexpr int block_threads = std::is_same_v<Mat, DevSliced> ? kSliceThreads : 256;
+
+template <class Mat>
 static cudaError_t rk4_one(const Mat& A, const double* uin, double* y, const CsrRK& rk, cudaStream_t st) {
     if (A.bin_block[kCsrBins] > 0)
-        launch_dependent(k_csr_rk<1, Mat>, A.bin_block[kCsrBins], st, A, uin, y, rk, CsrSets{1, 1, 1});
+        launch_dependent(k_csr_rk<1, Mat>, A.bin_block[kCsrBins], block_threads<Mat>, st, A, uin, y, rk, CsrSets{1, 1, 1});
     if constexpr (std::is_same_v<Mat, DevCSR>)
         if (A.nlong > 0) {
-            launch_dependent(k_rk_segments, grid_for(A.nseg * 32), st, A, uin);
-            launch_dependent(k_rk_long_rows, grid_for(A.nlong), st, A, y, rk);
+            launch_dependent(k_rk_segments, grid_for(A.nseg * 32), 256, st, A, uin);
+            launch_dependent(k_rk_long_rows, grid_for(A.nlong), 256, st, A, y, rk);
         }
     return cudaGetLastError();
 }
@@ -606,7 +620,7 @@ static void rk4_sets(const Mat& A, int64_t nb, double* y, double* acc, double* u
     for (int64_t g = 0; g < ng && nrb > 0; g += most) {
         const int64_t n = std::min(most, ng - g), o = g * NV * len;
         const CsrRK rk{acc + o, (stage % 2 ? u1 : u0) + o, dt, 0.5 * dt, dt / 6.0, stage, 1, nonfinite};
-        launch_dependent(k_csr_rk<NV, Mat>, (unsigned)(nrb * n), st, A, uin + o, y + o, rk,
+        launch_dependent(k_csr_rk<NV, Mat>, (unsigned)(nrb * n), block_threads<Mat>, st, A, uin + o, y + o, rk,
                          CsrSets{n, kPlainSetGroup, g + n == ng ? int(nb - (ng - 1) * NV) : NV});
     }
 }
@@ -670,11 +684,11 @@ cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, 
     const unsigned nb = (unsigned)A.bin_block[kCsrBins];
     if (nb == 0) return cudaSuccess;
     if (P % 4 == 0)
-        launch_dependent(k_sweep<4>, dim3(nb, P / 4), st, A, x, y, P, nonfinite);
+        launch_dependent(k_sweep<4>, dim3(nb, P / 4), kSliceThreads, st, A, x, y, P, nonfinite);
     else if (P % 2 == 0)
-        launch_dependent(k_sweep<2>, dim3(nb, P / 2), st, A, x, y, P, nonfinite);
+        launch_dependent(k_sweep<2>, dim3(nb, P / 2), kSliceThreads, st, A, x, y, P, nonfinite);
     else
-        launch_dependent(k_sweep<1>, dim3(nb, P), st, A, x, y, P, nonfinite);
+        launch_dependent(k_sweep<1>, dim3(nb, P), kSliceThreads, st, A, x, y, P, nonfinite);
     return cudaGetLastError();
 }
 
@@ -682,8 +696,8 @@ cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, 
 cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, double* y, int* seen, int call,
                          cudaStream_t st) {
     if (P.bin_block[kCsrBins] == 0) return cudaSuccess;
-    launch_dependent(k_apply, (unsigned)P.bin_block[kCsrBins], st, P, x, y, seen, call);
-    launch_dependent(k_apply_whole, 152u, st, A, x, y, (const int*)seen, call);
+    launch_dependent(k_apply, (unsigned)P.bin_block[kCsrBins], kSliceThreads, st, P, x, y, seen, call);
+    launch_dependent(k_apply_whole, 152u, 256, st, A, x, y, (const int*)seen, call);
     return cudaGetLastError();
 }
 
@@ -696,7 +710,7 @@ cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x
         nb = std::max(nb, D[d]->bin_block[kCsrBins]);
     }
     for (int d = P; d < 8; d++) S.d[d] = *D[0];
-    if (nb > 0) launch_dependent(k_derivatives, dim3((unsigned)nb, P), st, S, x, y, (int64_t)P);
+    if (nb > 0) launch_dependent(k_derivatives, dim3((unsigned)nb, P), kSliceThreads, st, S, x, y, (int64_t)P);
     return cudaGetLastError();
 }
 
@@ -704,7 +718,7 @@ cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x
 cudaError_t launch_sweep_points(const DevSliced& A, int D, const double* x, const double* v, const double* F, double* out,
                                 cudaStream_t st) {
     const unsigned nb = (unsigned)A.bin_block[kCsrBins];
-    if (nb > 0) launch_dependent(D == 1 ? k_sweep_points<2> : k_sweep_points<4>, nb, st, A, x, v, F, out);
+    if (nb > 0) launch_dependent(D == 1 ? k_sweep_points<2> : k_sweep_points<4>, nb, kSliceThreads, st, A, x, v, F, out);
     return cudaGetLastError();
 }
 
@@ -712,7 +726,7 @@ cudaError_t launch_sweep_points(const DevSliced& A, int D, const double* x, cons
 cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                           cudaStream_t st) {
     auto kernel = D == 3 ? k_points<3> : k_points<4>;
-    if (n > 0) launch_dependent(kernel, (unsigned)grid_for(n), st, v, F, pt, n, out);
+    if (n > 0) launch_dependent(kernel, (unsigned)grid_for(n), 256, st, v, F, pt, n, out);
     return cudaGetLastError();
 }
 

@@ -33,13 +33,17 @@ constexpr int64_t kCsrSplit = 2048;  // entries a row group sums directly
 // n=5 (31 K entries) 8.9, 12.0, 17.2, 29.0; 4D advection k=2 n=6 (533 K) 24.4,
 // 21.2, 25.2, 34.3; 3D wave k=3 n=7 (1.9 M) 60.0, 47.8, 46.9, 59.0, and 48 of
 // them sharing it 1446, 1096, 939, 948.  The whole Laplacian of that grid
-// (8.8 M) is applied in 33 us at 16 and 28.5 us at 32.  The nodal transforms,
-// passed over four vectors at once, keep 8 (the Vlasov plain step 2.60 ms
-// against 2.66 at 16 and 2.67 at 32).
+// (8.8 M) is applied in 33 us at 16 and 28.5 us at 32.  The assembled
+// nodal transforms, passed over four vectors at once, keep 8 (a Vlasov step with
+// them 2.60 ms against 2.66 at 16 and 2.67 at 32), the sweeps 6 (8 steps of
+// Vlasov 2x2v k=2 n=8 at 4, 5, 6 and 8: 5227, 4807, 4627 and 4583 us, n=7 2796,
+// 2690, 2726 and 2866, n=6 1581, 1592, 1596 and 1784, k=3 n=6 4702, 4484, 4290
+// and 4353).
 inline int csr_lane_entries(int64_t nnz) {
     return nnz < (128 << 10) ? 4 : nnz < (1 << 20) ? 8 : nnz < (4 << 20) ? 16 : 32;
 }
 constexpr int kCsrLaneEntriesMulti = 8;
+constexpr int kCsrLaneEntriesSweep = 6;
 inline int csr_bin(int64_t L, int per_lane) {
     int b = 0;
     while (b + 1 < kCsrBins && (int64_t(per_lane) << b) < L) b++;

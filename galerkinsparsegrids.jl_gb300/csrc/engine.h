@@ -47,7 +47,13 @@ struct DevSliced {
     const double* val;
     int bin_block[kCsrBins + 1];  // blocks of kSliceWarps slices per bin
 };
-constexpr int kSliceWarps = 8;
+// Small blocks: their ends are less ragged and the next launch's come up sooner.
+// With 8, 4, 2 and 1 warps: 200 steps of the 2D wave k=3 n=5 2006, 1867, 1839 and
+// 1898 us, 60 of the 4D advection k=2 n=6 1307, 1220, 1215 and 1192, 3 of 48 3D
+// waves k=3 n=7 2667, 2624, 2607 and 2595, 8 of Vlasov 2x2v k=2 n=8 4674, 4520,
+// 4512 and 5280 (the last: 32 blocks an SM are its limit).
+constexpr int kSliceWarps = 2;
+constexpr int kSliceThreads = 32 * kSliceWarps;
 
 // ---- chosen form: matrix-free FP32 pencil apply, FP64 RK state --------------
 //

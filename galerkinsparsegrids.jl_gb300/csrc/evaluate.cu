@@ -396,8 +396,8 @@ constexpr int kPencilMaxK = 5;
 // pay for k_lines (us per call, blocks and pencils: 3D k=3 n=7 64 and 69 at 1000
 // points, 90 and 69 at 4000, 3495 and 947 at 2^18; 4D k=3 n=4 90 and 104, 138 and
 // 105, 6579 and 2190; 2D k=2 n=6 39 and 41 at 4000, 64 and 46 at 16000, 524 and
-// 165; 1D k=3 n=8 39 and 45, 55 and 54, 448 and 141; the pencils' since 5 to 25 %
-// less at 2^18 points).
+// 165; 1D k=3 n=8 39 and 45, 55 and 54, 448 and 141.  With the scales in the
+// blocks the pencils take 866, 2126, 124 and 100 at 2^18 points).
 constexpr int64_t kPencilPoints = 4096, kPencilTerms = 1 << 20;
 
 // H_b[i][m] = <child b's Legendre function i, the parent's m>, G_b the same with

@@ -851,13 +851,13 @@ std::unique_ptr<DeviceSliced> gpu_line_operator(const SparseIndex& ix, const Lin
     require_gpu();
     std::vector<int64_t> rp;
     const auto A = line_operator(ix, T, d, st, rp);
-    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesMulti);
+    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesSweep);
 }
 
 std::unique_ptr<DeviceSliced> gpu_partial_transform(const SparseIndex& ix, const CSR& T1, unsigned dims, cudaStream_t st) {
     std::vector<int64_t> rp;
     const auto A = transform_csr(ix, T1, ((1u << ix.D) - 1) & ~dims, st, rp);
-    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesMulti);
+    return to_sliced(*A, rp, ix.N, st, kCsrLaneEntriesSweep);
 }
 
 std::unique_ptr<DeviceAdvection> gpu_advection(const SparseIndex& ix, const DLF1D& dlf, cudaStream_t st) {

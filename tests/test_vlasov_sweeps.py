@@ -54,6 +54,19 @@ def test_right_hand_side_and_steps(sgdg, D, k, n, scheme):
     op.close()
 
 
+# grids whose launches are all resident (ascending rows), partly (the derivatives
+# are more blocks than the sweeps) and all larger (long rows first)
+@pytest.mark.parametrize("D,k,n,scheme", [(2, 2, 5, "sparse"), (2, 2, 7, "sparse"), (1, 2, 7, "full"), (1, 3, 7, "full")])
+def test_right_hand_side_of_small_and_large_launches(sgdg, D, k, n, scheme):
+    # as above: 1e-10 of the result
+    op = sgdg.VlasovOperator(D, k, n, scheme)
+    rng = np.random.default_rng(D + n)
+    F, f = rng.uniform(-1, 1, (D, op.N)), rng.standard_normal(op.N)
+    ref = assembled(sgdg, D, k, n, scheme, F, op.v_point())(f)
+    assert np.linalg.norm(op.rhs(F, f) - ref) <= 1e-10 * np.linalg.norm(ref)
+    op.close()
+
+
 @pytest.mark.parametrize("where,value", [(0, np.nan), (3, np.inf), (-1, -np.inf)])
 def test_what_is_not_finite_spreads_as_the_assembled_operators_spread_it(sgdg, where, value):
     D, k, n = 1, 3, 4
