@@ -232,11 +232,14 @@ CSR add_scaled(const std::vector<const CSR*>& As, const std::vector<double>& s) 
 LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune) {
     const int k = op.k;
     double least = -1.0;  // entries of at most this magnitude are left out
+    std::vector<double> clean;
     if (prune) {
         double top = 0.0;
         for (double v : op.val) top = std::max(top, std::fabs(v));
         least = kPruneRel * top;
+        clean = dlf1d_entries(op, least);
     }
+    const std::vector<double>& val = prune ? clean : op.val;
     LineTables T;
     T.k = k;
     T.levels = levels;
@@ -256,10 +259,10 @@ LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune) {
                     const int cb = op.colblk[p];
                     if (cb >= nrb) continue;
                     for (int mj = 0; mj < k; mj++) {
-                        const double v = op.val[(size_t)p * k * k + (size_t)md * k + mj];
-                        if (prune && !(std::fabs(v) > least)) continue;
+                        const size_t at = (size_t)p * k * k + (size_t)md * k + mj;
+                        if (prune && !(std::fabs(op.val[at]) > least)) continue;
                         lc.push_back(cb * k + mj);
-                        lv.push_back(v);
+                        lv.push_back(val[at]);
                     }
                 }
                 lp[rb * k + md + 1] = (int64_t)lc.size();

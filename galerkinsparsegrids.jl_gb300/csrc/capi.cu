@@ -116,7 +116,15 @@ struct sgdg_op {
     // ones (3D k=3 n=7: 191 entries per row of the Laplacian, 41 of them
     // nonzero).  They do carry NaN and infinities from one row to another, so
     // a run that meets one is repeated with the whole operator (plain_run).
-    bool prunes() const { return basis == SGDG_BASIS_HIER && ix.k <= kPruneMaxK; }
+    // The whole operators' own rounding grows with k and eightfold per level in a
+    // Laplacian (relative L2 of what the two give for sums of Fourier modes: 3D
+    // k=3 n=7 1e-10, 2D k=4 n=7 3e-10, n=9 6e-9; after 200 steps of the wave 2D
+    // k=4 n=7 4e-11, n=9 7e-10; after 200 of the advection at most 5e-13): second
+    // derivatives and applications are pruned where the two agree to 1e-10 or so.
+    static constexpr int kPruneWave = 11, kPruneApply = 10;  // k + n at most
+    bool prunes(bool second, int most) const {
+        return basis == SGDG_BASIS_HIER && ix.k <= kPruneMaxK && (!second || ix.k + ix.n <= most);
+    }
     const DevSliced& stepping(int which) {
         auto it = step_dev.find(which);
         if (it == step_dev.end()) it = step_dev.emplace(which, gpu_step_operator(ix, *dlf, which, stream)).first;
@@ -125,18 +133,18 @@ struct sgdg_op {
     // Applications of an operator of kApplyPruned entries or more go through the
     // pruned one (us per application, whole and pruned: Laplacian 2D k=3 n=7, 1.3
     // M entries, 8.3 and 8.9; 4D k=2 n=6, 1.6 M, 10.3 and 8.9; 3D k=3 n=6, 2.2 M,
-    // 11.5 and 9.1; 3D k=3 n=7, 8.8 M, 28.3 and 9.0; 3D k=4 n=7, 27.8 M, 82.9 and
-    // 18.5; below 9 the time is the caller's, two launches for one), and where
-    // an element of x is not finite through the whole one after it
-    // (k_apply_whole).  Each call leaves its number in a word of its own among
-    // kApplyCalls: calls on other streams may still be in flight.
+    // 11.5 and 9.1; 3D k=3 n=7, 8.8 M, 28.3 and 9.0; below 9 the time is the
+    // caller's, two launches for one), and where an element of x is not finite
+    // through the whole one after it (k_apply_whole).  Each call leaves its number
+    // in a word of its own among kApplyCalls: calls on other streams may still be
+    // in flight.
     static constexpr int64_t kApplyPruned = 3 << 19;
     static constexpr int kApplyCalls = 1024;
     DevBuf apply_seen;
     int apply_call = 0;
     cudaError_t apply(int which, const double* x, double* y, cudaStream_t st) {
         const DevCSR& A = device(which);
-        if (!prunes() || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
+        if (!prunes(true, kPruneApply) || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
         if (!apply_seen.p) {
             stepping(which);
             apply_seen.alloc(sizeof(int) * kApplyCalls);
@@ -746,7 +754,7 @@ static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t
     cudaStream_t st = op_stream(op);
     std::vector<double> s;  // -sum_d a_d D_d
     for (int d = 0; a && d < op->ix.D; d++) s.push_back(-a[d]);
-    if (op->prunes()) {
+    if (op->prunes(a == nullptr, op->kPruneWave)) {
         const DevSliced* A = nullptr;
         if (a) {
             if (!op->adv) op->adv = gpu_advection(op->ix, *op->dlf, st);
@@ -821,7 +829,7 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
     std::unique_ptr<PlainScratch> work;
     DevBuf keep;
     const DevSliced* A = nullptr;
-    if (op->prunes()) {
+    if (op->prunes(which < 1, op->kPruneWave)) {
         try {
             A = &op->stepping(which);
             work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));

@@ -367,6 +367,93 @@ static DLF1D build_dlf(int k, int n) {
     return op;
 }
 
+// One 1D function: on [-1, 1] of y = 2^lev x - (2 cell - 1) the polynomial c[i] +-
+// c[i + k] of its halves, times sqrt(2^lev); positions in units of 2^-F.
+struct Local {
+    int lev, k;
+    int64_t centre, half;
+    const double* c;  // 2k: x^i, sgn(x) x^i
+    double y(int64_t p, double t, int F) const { return std::ldexp((double)(p - centre) + t, lev - F); }
+    double at(int side, double y) const {
+        double s = 0.0;
+        for (int i = k - 1; i >= 0; i--) s = s * y + (side ? c[i] + c[i + k] : c[i] - c[i + k]);
+        return s;
+    }
+    double slope(int side, double y) const {
+        double s = 0.0;
+        for (int i = k - 1; i >= 1; i--) s = s * y + i * (side ? c[i] + c[i + k] : c[i] - c[i + k]);
+        return s;
+    }
+    // limit at position p from the right or the left
+    double limit(int64_t p, bool right, int F) const {
+        for (int side = 0; side < 2; side++) {
+            const int64_t a = centre - (side ? 0 : half), b = a + half;
+            if (right ? p >= a && p < b : p > a && p <= b) return at(side, y(p, 0.0, F));
+        }
+        return 0.0;
+    }
+};
+
+// Entry (i, j) of the derivative with central flux is the integral of f_i f_j'
+// over f_j's pieces plus, at each of f_j's breaks, f_i's mean times f_j's jump.
+std::vector<double> dlf1d_entries(const DLF1D& op, double least) {
+    const int k = op.k;
+    const RefBasis B(k);
+    std::vector<double> X, W, leg((size_t)k * 2 * k, 0.0);
+    gauss_legendre(k, X, W);  // exact to degree 2k - 1
+    for (int m = 0; m < k; m++)
+        for (int i = 0; i < k; i++) leg[(size_t)m * 2 * k + i] = B.legendre(m)[i];
+    auto local = [&](int blk, int mode, int F) {
+        const int L = op.blk_level[blk], lev = std::max(1, L - 1);
+        const int64_t half = int64_t(1) << (F - lev);
+        return Local{lev, k, (2 * (int64_t)op.blk_cell[blk] - 1) * half, half,
+                     (L == 1 ? leg.data() : B.dg) + (size_t)mode * 2 * k};
+    };
+    std::vector<double> out(op.val.size(), 0.0);
+    std::map<std::vector<int64_t>, std::vector<double>> done;  // blocks repeat along the periodic line
+    for (int rb = 0; rb < op.nblocks; rb++)
+        for (int p = op.rowptr[rb]; p < op.rowptr[rb + 1]; p++) {
+            const int cb = op.colblk[p];
+            const size_t first = (size_t)p * k * k;
+            const double* v = &op.val[first];
+            if (std::none_of(v, v + k * k, [&](double e) { return std::fabs(e) > least; })) continue;
+            const int F = std::max({1, op.blk_level[rb] - 1, op.blk_level[cb] - 1});
+            const int64_t period = int64_t(1) << F;
+            const int64_t apart = local(rb, 0, F).centre - local(cb, 0, F).centre;
+            std::vector<double>& block = done[{op.blk_level[rb], op.blk_level[cb], ((apart % period) + period) % period}];
+            if (block.empty()) {
+                block.resize((size_t)k * k);
+                for (int e = 0; e < k * k; e++) {
+                    const Local fi = local(rb, e / k, F), fj = local(cb, e % k, F);
+                    double s = 0.0;
+                    for (int sj = 0; sj < 2; sj++)
+                        for (int si = 0; si < 2; si++) {
+                            const int64_t aj = fj.centre - (sj ? 0 : fj.half), ai = fi.centre - (si ? 0 : fi.half);
+                            const int64_t lo = std::max(ai, aj), len = std::min(ai + fi.half, aj + fj.half) - lo;
+                            if (len <= 0) continue;
+                            double q = 0.0;
+                            for (int g = 0; g < k; g++) {
+                                const double t = 0.5 * (double)len * (1.0 + X[g]);
+                                q += W[g] * fi.at(si, fi.y(lo, t, F)) * fj.slope(sj, fj.y(lo, t, F));
+                            }
+                            s += 0.5 * std::ldexp((double)len, fj.lev - F) * q;
+                        }
+                    int64_t breaks[3] = {fj.centre - fj.half, fj.centre, (fj.centre + fj.half) % period};
+                    for (int b = 0; b < 3; b++) {
+                        if (b == 2 && breaks[2] == breaks[0]) continue;
+                        const int64_t x = breaks[b], xl = x == 0 ? period : x;
+                        s += 0.5 * (fi.limit(x, true, F) + fi.limit(xl, false, F)) *
+                             (fj.limit(x, true, F) - fj.limit(xl, false, F));
+                    }
+                    block[e] = s * std::sqrt(std::ldexp(1.0, fi.lev + fj.lev));
+                }
+            }
+            for (int e = 0; e < k * k; e++)
+                if (std::fabs(v[e]) > least) out[first + e] = block[e];
+        }
+    return out;
+}
+
 static CSR to_csr(const Sp& A) {
     CSR C;
     C.m = A.m;

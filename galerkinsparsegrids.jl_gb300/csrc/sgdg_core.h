@@ -64,6 +64,9 @@ struct DLF1D {
     std::vector<double> val;         // k*k per stored block, [i][j] = D[rb*k+i][cb*k+j]
 };
 std::shared_ptr<const DLF1D> dlf1d(int k, int n);
+// op.val with the entries of more than `least` from their two functions alone
+// (the others 0), rounded to a few units of their own size
+std::vector<double> dlf1d_entries(const DLF1D& op, double least);
 
 // The 1D operator as the matrix-free kernels apply it: block CSR over the
 // blocks that are not zero up to roundoff, each entry as an FP32 (hi, lo)
@@ -212,7 +215,9 @@ void pencil_rows(const Pencil& p, int k, int64_t kD, std::vector<int32_t>& out);
 // largest entry, while the others reach 1e-4 of it and more (k = 1..5,
 // n = 2..10).  The bound is 1e-10, and for the square 1e-10 of the sum of the
 // magnitudes of an entry's terms (rounding leaves at most 1e-11 of it, other
-// entries 8e-4 and more).
+// entries 8e-4 and more).  The entries kept are dlf1d_entries': the route's own
+// hold its rounding too (up to 1e-13 of the largest), which its small entries,
+// left out here, partly undo.
 constexpr int kPruneMaxK = 5;
 constexpr double kPruneRel = 1e-10;
 struct LineTables {

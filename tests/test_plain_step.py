@@ -186,3 +186,45 @@ def test_applications_in_a_graph_and_on_two_streams(sgdg):
         fin = np.isfinite(ref)
         assert np.array_equal(np.isfinite(got), fin)
         assert np.linalg.norm(got[fin] - ref[fin]) <= 1e-10 * np.linalg.norm(ref[fin])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,n", [(2, 5), (3, 5)])
+def test_stepping_against_the_operator_in_plain_numpy(sgdg, k, n):
+    # both operators are within 1e-14 of their largest entry of the true one
+    # (numpy's: rounding of Q' A Q, 4e-15 at k=3 n=5; the wavelets' own, in both,
+    # 2e-15 there, but 2e-13 at k=4 and 8e-13 at k=5; the reference's route is
+    # 6e-14 to 4e-13 away), and what that changes in a step is at most its
+    # share of dt |L| <= 3, with a factor 2 for the norms: 6e-14 in each of 30 steps
+    import importlib.util
+    import pathlib
+    path = pathlib.Path(__file__).resolve().parents[1] / "perf" / "cases.py"
+    spec = importlib.util.spec_from_file_location("perf_cases", path)
+    cases = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(cases)
+    D, _ = cases.derivative_1d(k, n)
+    N = len(D)
+    A = np.block([[np.zeros((N, N)), np.eye(N)], [D @ D, np.zeros((N, N))]])
+    rng = np.random.default_rng(k)
+    y = rng.standard_normal(2 * N)
+    y[N:] *= np.linalg.norm(D, 2)  # velocities of the size the fastest modes have
+    dt = 1.0 / np.linalg.norm(D, 2)
+    _, st = sgdg.wave_evolve(1, k, n, y[:N], y[N:], 0.0, 30 * dt, nsteps=30)
+    ref = rk4(A, y, dt, 30)
+    got = np.asarray(st[-1]).reshape(-1)
+    assert np.linalg.norm(got[:N] - ref[:N]) <= 30 * 6e-14 * np.linalg.norm(ref[:N])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,k,n", [(2, 3, 8), (2, 3, 9), (2, 4, 7), (2, 4, 8)])
+def test_finest_grids_step_with_the_whole_operator(sgdg, D, k, n):
+    # k + n on both sides of the limit of the pruned wave operator: the states are
+    # of the size of the largest entries' results, of which the two operators
+    # differ by at most 1e-11 per step, and with the whole one by roundings
+    op = sgdg.SparseGridOperator(D, k, n)
+    A, N = op.csr(-1), op.N
+    y = np.random.default_rng(n).standard_normal(2 * N)
+    dt = 1.0 / np.sqrt(np.abs(A).sum(1).max())
+    _, st = sgdg.wave_evolve(D, k, n, y[:N], y[N:], 0.0, 3 * dt, nsteps=3, op=op)
+    ref = rk4(A, y, dt, 3)
+    assert np.linalg.norm(st[-1] - ref) <= (1e-10 if k + n <= 11 else 1e-13) * np.linalg.norm(ref)
