@@ -290,7 +290,7 @@ def vlasov_leg(sg, stream, steps, batch=16):
     N = int(f0.size)
     out = {"workload": "Vlasov 2x2v (D=4 phase space), sparse k=2, n=8, RK4", "state_dofs": N,
            "steps": steps, "dt": dt, "unit": UNIT,
-           "plain_fp64": {"form": "FP64 sparse operators (CSR SpMV), graph per RK4 step",
+           "plain_fp64": {"form": "FP64 sparse sweeps along one dimension after another, graph per RK4 step",
                           "value": N * 4.0 / per_step, "ms_per_step": 1e3 * per_step,
                           "wall_s_end_to_end": total, "setup_s": setup},
            "rel_l2_change_of_f": float(np.linalg.norm(st[-1] - f0) / np.linalg.norm(f0))}
@@ -307,7 +307,7 @@ def vlasov_leg(sg, stream, steps, batch=16):
     mf = b.state(i)
     ms_one = timed_steps(b, stream, 20, 3)
     b.close()
-    out["matfree_one"] = {"form": "FP32 pencil sweeps, FP64 RK state, graph per RK4 step",
+    out["matfree_one"] = {"form": "FP32 pencil sweeps, FP64 RK state, one launch per RK4 step",
                           "value": N * 4.0 / (ms_one / 1e3), "ms_per_step": ms_one,
                           "rel_l2_vs_plain_fp64": float(np.linalg.norm(mf - st[-1]) / np.linalg.norm(st[-1]))}
     # matrix-free, a batch of independent solves (different seeded forces and data)
@@ -368,12 +368,11 @@ def evaluate_leg(sg, stream, npts):
     e1.record(stream)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / reps
-    nlev = len({tuple(r) for r in sg.index_map(Dv, kv, nv)[0]})
-    # FP64 operations per point (an FMA counts 2): per level block, with two
-    # dimensions contracted first (D >= 3), k^(D-2) (2k^2 + 2k + D), else
-    # k^(D-1) (2k + D + 1); plus the 1D basis tables
-    per_block = kv ** (Dv - 2) * (2 * kv * kv + 2 * kv + Dv) if Dv >= 3 else kv ** (Dv - 1) * (2 * kv + Dv + 1)
-    flops = npts * (nlev * per_block + Dv * (nv + 1) * 2 * kv * kv)
+    pencils = len({tuple(r[1:]) for r in sg.index_map(Dv, kv, nv)[0]})
+    # FP64 operations per point (an FMA counts 2): per pencil of level blocks
+    # along dimension 1, summed into one before, the contraction of k^3
+    # numbers; plus the 1D basis tables
+    flops = npts * (pencils * 2 * (kv ** 3 + kv ** 2 + kv) + Dv * (nv + 1) * 2 * kv * (kv - 1))
     t0 = time.perf_counter()
     vals = sg.reconstruct_DG(Dv, kv, nv, c, pts)
     e2e = time.perf_counter() - t0
@@ -582,7 +581,7 @@ def run_ours(args):
     # one call per step: host states in, one RK4 step, host states out, with
     # the copies of each pipeline chunk overlapping the other chunks' steps;
     # three repeats of e2e_steps calls, the median reported
-    b.step_host(host.data_ptr(), host.data_ptr(), 1, args.e2e_chunks)  # builds the chunk graphs
+    b.step_host(host.data_ptr(), host.data_ptr(), 1, args.e2e_chunks)  # builds the chunks
     reps = []
     for _ in range(3):
         t0 = time.perf_counter()
@@ -649,7 +648,7 @@ def run_ours(args):
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32 apply / f64 RK state", "data": "synthetic (seeded Fourier ICs)",
         "config": workload_config(args.solves, total // args.solves),
-        "form": "matrix-free FP32 pencil apply, FP64 RK4, CUDA graph per step",
+        "form": "matrix-free FP32 pencil apply, FP64 RK4, one launch per step",
         "working_set_bytes_per_gpu": int(working_set), "tile_shape_wlog_coop": list(tile[:2]),
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(total * 8),
                 "d2h_bytes_per_step": int(total * 8), "steps": args.e2e_steps, "pipeline_chunks": args.e2e_chunks,
@@ -658,8 +657,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": traffic,
                      "bytes_per_dof_update": BYTES_PER_DOF_UPDATE},
-        "plain_fp64_batch": {"form": "FP64 CSR SpMV + FP64 RK4 stage update per solve, all solves of a stage in "
-                                     "one launch, CUDA graph per step (sgdg_op_plain_steps_device)",
+        "plain_fp64_batch": {"form": "FP64 sparse row sums + FP64 RK4 stage update, sets of four solves, all solves "
+                                     "of a stage in one launch (sgdg_op_plain_steps_device)",
                              "value": plain_value, "unit": UNIT, "solves": args.solves, "nnz": int(plain_nnz),
                              "steps": plain_steps, "ms_per_step": 1e3 * plain_s / plain_steps,
                              "chosen_over_plain": value / plain_value,
