@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <mutex>
 #include <queue>
 
@@ -29,13 +30,18 @@ cudaError_t launch_f32_to_f64(const float* a, double* b, int64_t n, cudaStream_t
 
 static constexpr size_t kWaveLag = 3;       // steps between a group's consecutive phases in the work list
 // List order of the work list (mf_work_list): up to these bytes of vectors (L2
-// holds 126 MB, and the list does not keep the groups in flight few), this many
-// items times groups (the host's work), and from these items per phase on: below,
-// every CTA is ahead of the list's end and only waits longer.  us for 20 steps of
-// uneven advection solves (D 2-3, k 2-4, n 4-7), wavefront and list order: 128
-// solves 6614 and 5804, 96 4905 and 4349, 40 3773 and 3469, 20 2750 and 2750, 8
-// 1534 and 1575; eight served requests 7.9 and 8.7 ms.  CTAs it reckons with: all
-// that are resident.
+// holds 126 MB, and the list does not keep the groups in flight few), up to this
+// many items times groups (what was measured), and from these items per phase on:
+// below, every CTA is ahead of the list's end and only waits longer.  us for 20
+// steps of uneven advection solves (D 2-3, k 2-4, n 4-7), wavefront and list
+// order: 128 solves 6614 and 5804, 96 4905 and 4349, 40 3773 and 3469, 20 2750 and
+// 2750, 8 1534 and 1575.  On the host the list order takes about 80 ns an item
+// more: 0.2 to 0.6 ms a plan at 20 to 256 such solves.  A server, which plans again
+// whenever a request ends, keeps the wavefront (set_list_order; the whole stream in
+// wavefront and list order, requests of 20 to 60 steps, D 2-4, k 2-3: 32 live 42
+// and 51 ms, 64 live 77 and 94; of 100 to 400 steps 110 and 125, 188 and 218; eight
+// requests 7.9 and 8.7).  CTAs it reckons with: all that are resident on a GB300 (a
+// list is also built where there is no GPU to ask).
 constexpr double kListBytes = 96e6, kListWork = 4e6, kListItems = 300;
 constexpr int kListCtas = 456;
 static constexpr int kStageKey = 1 << 22;   // counter keys of a whole-step list: key + (stage - 1) * kStageKey
@@ -525,7 +531,7 @@ static int mf_ctas_per_sm(double items_per_phase, int most) {
 // groups in flight (about one per phase) keep their reused vectors in L2.
 size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items, int& nctr, bool pass_only,
                     const std::map<std::pair<int, int>, MFTile>* shapes, int chunk, int nchunks,
-                    std::vector<std::array<int, 3>>* ranges) {
+                    std::vector<std::array<int, 3>>* ranges, bool list_order) {
     struct Phase {
         std::vector<MFItem> items;
         int depth = 0;      // longest chain of phases before it in the group
@@ -533,6 +539,7 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
         int wait_key = -1;  // counter it waits for (-1: none)
         int win_key = -1;   // whole-step list: the counter of the RK phase that wrote its stage input
         int stage = 0;      // RK stage of its items (0: the launch's stage)
+        int ctr[3] = {-1, -1, -1}, need[2] = {0, 0};  // done, wait and win counters; items the two waits are for
     };
     struct Group {
         std::vector<Phase> phases;
@@ -728,27 +735,38 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
             if (!ctr_of[g].count(ph.done_key)) ctr_of[g][ph.done_key] = nctr++;
             items_of[g][ph.done_key] += (int)ph.items.size();
         }
-    auto emit = [&](size_t g, const Phase& ph, MFItem it) {
-        it.done_ctr = ctr_of[g].at(ph.done_key);
-        it.wait_ctr = ph.wait_key >= 0 ? ctr_of[g].at(ph.wait_key) : -1;
-        it.wait_need = ph.wait_key >= 0 ? items_of[g].at(ph.wait_key) : 0;
-        it.win_ctr = ph.win_key >= 0 ? ctr_of[g].at(ph.win_key) : -1;
-        it.win_need = ph.win_key >= 0 ? items_of[g].at(ph.win_key) : 0;
-        items.push_back(it);
-    };
     size_t total = 0;
-    for (auto& g : groups)
-        for (const Phase& ph : g.phases) total += ph.items.size();
-    if (chains && groups.size() > 1 && bytes <= kListBytes && double(total) * double(groups.size()) <= kListWork &&
-        total > kListItems * mf_chain(cls, pass_only)) {
+    for (size_t g = 0; g < groups.size(); g++)
+        for (Phase& ph : groups[g].phases) {
+            total += ph.items.size();
+            ph.ctr[0] = ctr_of[g].at(ph.done_key);
+            if (ph.wait_key >= 0) ph.ctr[1] = ctr_of[g].at(ph.wait_key), ph.need[0] = items_of[g].at(ph.wait_key);
+            if (ph.win_key >= 0) ph.ctr[2] = ctr_of[g].at(ph.win_key), ph.need[1] = items_of[g].at(ph.win_key);
+        }
+    items.reserve(items.size() + total);
+    auto emit = [&](const Phase& ph, const MFItem& from) {
+        items.push_back(from);
+        MFItem& it = items.back();
+        it.done_ctr = ph.ctr[0];
+        it.wait_ctr = ph.ctr[1];
+        it.wait_need = ph.need[0];
+        it.win_ctr = ph.ctr[2];
+        it.win_need = ph.need[1];
+    };
+    if (list_order && chains && groups.size() > 1 && bytes <= kListBytes &&
+        double(total) * double(groups.size()) <= kListWork && total > kListItems * mf_chain(cls, pass_only)) {
         // List order: the items as kListCtas CTAs would take them, each free CTA
         // the item of the group with the most work ahead (its remaining phases)
         // among the groups whose next output would not wait, else of the one whose
         // wait ends first.  An item's cycles are estimated from its elements, and
-        // its output (the last third) waits for the group's previous phase.
+        // its output (the last third) waits for the group's previous phase.  The
+        // CTAs come free in ascending order, so a group that need not wait goes on
+        // so until its item changes: the groups are in two heaps, and a step costs
+        // the replacement of the freed CTA's time.
         struct State {
             size_t phase = 0, item = 0;
             double ready = 0, done = 0;  // end of the previous phase; of this one's items so far
+            double cost = 0, key = 0;    // of its next item; a CTA free by then would not wait
             std::vector<double> ahead;   // per phase: estimated cycles from its start on
         };
         auto cost = [](const Group& g, const MFItem& it) {
@@ -762,43 +780,71 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
             for (size_t p = ph.size(); p-- > 0;) {
                 double sum = 0, most = 0;
                 for (const MFItem& it : ph[p].items) {
-                    sum += cost(groups[g], it);
-                    most = std::max(most, cost(groups[g], it));
+                    const double c = cost(groups[g], it);
+                    sum += c;
+                    most = std::max(most, c);
                 }
                 state[g].ahead[p] = state[g].ahead[p + 1] + std::max(most, sum / kListCtas);
             }
         }
-        std::priority_queue<double, std::vector<double>, std::greater<double>> cta;
-        for (int i = 0; i < kListCtas; i++) cta.push(0.0);
+        auto ahead = [&](size_t g) { return state[g].ahead[state[g].phase]; };
+        auto less_ahead = [&](size_t a, size_t b) { return ahead(a) != ahead(b) ? ahead(a) < ahead(b) : a > b; };
+        auto waits_longer = [&](size_t a, size_t b) {
+            return state[a].key != state[b].key ? state[a].key > state[b].key : less_ahead(a, b);
+        };
+        std::priority_queue<size_t, std::vector<size_t>, decltype(less_ahead)> ready(less_ahead);
+        std::priority_queue<size_t, std::vector<size_t>, decltype(waits_longer)> waiting(waits_longer);
+        // the group's next item, if it has one
+        auto next = [&](size_t g) {
+            State& s = state[g];
+            const auto& ph = groups[g].phases;
+            while (s.phase < ph.size() && s.item == ph[s.phase].items.size()) {
+                s.ready = std::max(s.ready, s.done);
+                s.phase++;
+                s.item = 0;
+            }
+            if (s.phase == ph.size()) return false;
+            s.cost = cost(groups[g], ph[s.phase].items[s.item]);
+            s.key = s.ready - 0.65 * s.cost;
+            return true;
+        };
+        for (size_t g = 0; g < groups.size(); g++)
+            if (next(g)) waiting.push(g);
+        // when each CTA comes free, a binary heap (full: every parent has two children)
+        static_assert(kListCtas % 2 == 0, "one more makes the heap full");
+        std::vector<double> cta(kListCtas + 1, 0.0);
+        cta.back() = std::numeric_limits<double>::infinity();
         for (size_t left = total; left > 0; left--) {
-            const double t = cta.top();
-            cta.pop();
-            size_t best = groups.size();
-            double best_wait = 0;
-            for (size_t g = 0; g < groups.size(); g++) {
-                State& s = state[g];
-                const auto& ph = groups[g].phases;
-                while (s.phase < ph.size() && s.item == ph[s.phase].items.size()) {  // on to the next phase
-                    s.ready = std::max(s.ready, s.done);
-                    s.phase++;
-                    s.item = 0;
-                }
-                if (s.phase == ph.size()) continue;
-                const double c = cost(groups[g], ph[s.phase].items[s.item]);
-                const double wait = std::max(0.0, s.ready - (t + 0.65 * c));
-                if (best == groups.size() || wait < best_wait ||
-                    (wait == best_wait && s.ahead[s.phase] > state[best].ahead[state[best].phase])) {
-                    best = g;
-                    best_wait = wait;
+            const double t = cta[0];
+            for (; !waiting.empty() && state[waiting.top()].key <= t; waiting.pop()) ready.push(waiting.top());
+            const bool waits = ready.empty();
+            const size_t g = waits ? waiting.top() : ready.top();
+            State& s = state[g];
+            const Phase& ph = groups[g].phases[s.phase];
+            emit(ph, ph.items[s.item++]);
+            const double end = std::max(t + 0.65 * s.cost, s.ready) + 0.35 * s.cost;
+            s.done = std::max(s.done, end);
+            size_t i = 0;  // the hole at the top to the bottom, then up to where the end belongs
+            for (size_t c = 1; c < cta.size(); i = c, c = 2 * i + 1) {
+                c += cta[c + 1] < cta[c];
+                cta[i] = cta[c];
+            }
+            for (; i > 0 && cta[(i - 1) / 2] > end; i = (i - 1) / 2) cta[i] = cta[(i - 1) / 2];
+            cta[i] = end;
+            if (s.item < ph.items.size()) {  // it stays where it is in its heap?
+                const double c = cost(groups[g], ph.items[s.item]);
+                if (c == s.cost) continue;
+                if (!waits && s.ready - 0.65 * c <= cta[0]) {
+                    s.cost = c;
+                    s.key = s.ready - 0.65 * c;
+                    continue;
                 }
             }
-            State& s = state[best];
-            const Phase& ph = groups[best].phases[s.phase];
-            const MFItem& it = ph.items[s.item++];
-            const double c = cost(groups[best], it), end = std::max(t + 0.65 * c, s.ready) + 0.35 * c;
-            s.done = std::max(s.done, end);
-            cta.push(end);
-            emit(best, ph, it);
+            if (waits)
+                waiting.pop();
+            else
+                ready.pop();
+            if (next(g)) waiting.push(g);
         }
         return smem;
     }
@@ -826,7 +872,7 @@ size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items,
                 const size_t g = t - t0;
                 for (const Phase& ph : groups[g].phases) {
                     if (ph.depth != (int)pp || std::max(ph.stage, 1) != st + 1) continue;
-                    for (const MFItem& it : ph.items) emit(g, ph, it);
+                    for (const MFItem& it : ph.items) emit(ph, it);
                 }
             }
     return smem;
@@ -846,7 +892,7 @@ void MFEngine::build_items(std::vector<MFItem>& items, int& nctr, bool pass_only
                            const std::map<std::pair<int, int>, MFTile>* shapes, int chunk, int nchunks,
                            std::vector<std::array<int, 3>>* ranges) {
     const std::vector<WLClass> cls = wl_classes();
-    size_t smem = mf_work_list(cls, items, nctr, pass_only, shapes, chunk, nchunks, ranges);
+    size_t smem = mf_work_list(cls, items, nctr, pass_only, shapes, chunk, nchunks, ranges, list_order_);
     int tb = 0;
     for (auto& cp : classes_) {
         const SolveSpec& sp = solves_[cp->slots[0]].spec;

@@ -38,11 +38,12 @@ struct WLClass {
 // Builds the matrix-free work list of the classes -- the whole RK4 step (four
 // stages) for classes that step, one pass per dimension for classes that
 // only apply or when pass_only -- with chunk / nchunks and ranges as for
-// MFEngine::step_host; nctr receives the number of counters.  Returns the
-// shared memory a tile needs (without the operator table).
+// MFEngine::step_host; nctr receives the number of counters.  list_order: in
+// list order where that pays for steps enough.  Returns the shared memory a tile
+// needs (without the operator table).
 size_t mf_work_list(const std::vector<WLClass>& cls, std::vector<MFItem>& items, int& nctr, bool pass_only,
                     const std::map<std::pair<int, int>, MFTile>* shapes, int chunk, int nchunks,
-                    std::vector<std::array<int, 3>>* ranges);
+                    std::vector<std::array<int, 3>>* ranges, bool list_order = true);
 
 class MFEngine {
    public:
@@ -53,6 +54,8 @@ class MFEngine {
 
     void set_stream(cudaStream_t st);
     cudaStream_t stream() const { return stream_; }
+    // false for an engine that is stepped a few times only between its re-plans
+    void set_list_order(bool on) { list_order_ = on; }
 
     // Adds a solve; y0 (host, Ns values) may be null (zero state).  A Vlasov
     // solve also takes its point weights: 2 x D x N floats (hi block, lo block)
@@ -155,6 +158,7 @@ class MFEngine {
     size_t smem_ = 0;
     int table_bytes_ = 0;  // shared-memory operator table reserved ahead of the tile
     bool dirty_ = true;
+    bool list_order_ = true;
     struct Chunk {  // step_host's pipeline stage
         DevBuf items, ctr;
         int nitems = 0, nctr = 0;

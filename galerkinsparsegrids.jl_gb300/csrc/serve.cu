@@ -45,7 +45,9 @@ class Server {
         double t_arrival = 0, t_admit = -1, t_done = -1;
     };
 
-    Server(int max_chunk, cudaStream_t st) : max_chunk_(max_chunk), eng_(st), t0_(Clock::now()) {}
+    Server(int max_chunk, cudaStream_t st) : max_chunk_(max_chunk), eng_(st), t0_(Clock::now()) {
+        eng_.set_list_order(false);
+    }
 
     double now() const { return std::chrono::duration<double>(Clock::now() - t0_).count(); }
 
