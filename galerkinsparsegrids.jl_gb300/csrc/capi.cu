@@ -60,7 +60,7 @@ void set_error(const std::string& msg) { g_err = msg; }
 using namespace sgdg;
 
 // ------------------------------------------------------------ handles ----
-struct sgdg_op {
+struct sgdg_op : Spare {
     SparseIndex ix;
     std::shared_ptr<const DLF1D> dlf;
     int basis = SGDG_BASIS_HIER;  // SGDG_BASIS_POS: the 1D position-basis operators
@@ -69,6 +69,8 @@ struct sgdg_op {
     std::map<int, std::unique_ptr<DeviceCSR>> dev;  // plain-form device copies by `which`
     std::map<int, std::unique_ptr<DeviceSliced>> step_dev;  // without the rounding of zeros (stepping)
     std::unique_ptr<DeviceAdvection> adv;
+    std::map<int, int> refused;  // `which`: the budget (g_budget_set) that had no room for its pruned form
+    static constexpr int kAdvection = INT32_MIN;  // adv, beside the selectors
     std::map<int, std::unique_ptr<MFEngine>> mf_apply;
     cudaStream_t stream = nullptr;
 
@@ -125,10 +127,45 @@ struct sgdg_op {
     bool prunes(bool second, int most) const {
         return basis == SGDG_BASIS_HIER && ix.k <= kPruneMaxK && (!second || ix.k + ix.n <= most);
     }
-    const DevSliced& stepping(int which) {
+    // Without room for it, now or earlier under the same budget: null, and the
+    // caller goes on with the whole operator.  The caller holds a Use.
+    const DevSliced* stepping(int which) {
         auto it = step_dev.find(which);
-        if (it == step_dev.end()) it = step_dev.emplace(which, gpu_step_operator(ix, *dlf, which, stream)).first;
-        return it->second->d;
+        if (it == step_dev.end()) {
+            std::unique_ptr<DeviceSliced> S;
+            if (!build_pruned(which, [&] { S = gpu_step_operator(ix, *dlf, which, stream); })) return nullptr;
+            it = step_dev.emplace(which, std::move(S)).first;
+        }
+        return &it->second->d;
+    }
+    template <class Build>
+    bool build_pruned(int which, Build&& build) {
+        const auto f = refused.find(which);
+        if (f != refused.end() && f->second == g_budget_set.load()) return false;
+        try {
+            build();
+            return true;
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET) throw;
+            refused[which] = g_budget_set.load();
+            return false;
+        }
+    }
+    // what is there beside the whole operators
+    bool drop_spare() override {
+        bool any = adv != nullptr;
+        if (adv) refused[kAdvection] = g_budget_set.load();
+        adv.reset();
+        for (auto it = step_dev.begin(); it != step_dev.end();) {
+            if (!dev.count(it->first)) {
+                ++it;
+                continue;
+            }
+            refused[it->first] = g_budget_set.load();
+            it = step_dev.erase(it);
+            any = true;
+        }
+        return any;
     }
     // Applications of an operator of kApplyPruned entries or more go through the
     // pruned one (us per application, whole and pruned: Laplacian 2D k=3 n=7, 1.3
@@ -143,28 +180,36 @@ struct sgdg_op {
     DevBuf apply_seen;
     int apply_call = 0;
     cudaError_t apply(int which, const double* x, double* y, cudaStream_t st) {
-        const DevCSR& A = device(which);
+        const DevCSR& A = whole(which);
         if (!prunes(true, kPruneApply) || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
-        if (!apply_seen.p) {
-            stepping(which);
-            apply_seen.alloc(sizeof(int) * kApplyCalls);
-            CK(cudaMemsetAsync(apply_seen.p, 0, apply_seen.bytes, stream));
-            CK(cudaStreamSynchronize(stream));
-        }
-        const DevSliced& P = stepping(which);
+        Use use(*this);
+        const DevSliced* P = stepping(which);
+        if (P && !apply_seen.p && !build_pruned(which, [&] {
+                DevBuf seen(sizeof(int) * kApplyCalls);
+                CK(cudaMemsetAsync(seen.p, 0, seen.bytes, stream));
+                CK(cudaStreamSynchronize(stream));
+                apply_seen = std::move(seen);
+            }))
+            P = nullptr;
+        if (!P) return launch_csr_spmv(A, x, y, st);
         apply_call = apply_call == INT32_MAX ? 1 : apply_call + 1;
-        return launch_apply(P, A, x, y, apply_seen.as<int>() + apply_call % kApplyCalls, apply_call, st);
+        return launch_apply(*P, A, x, y, apply_seen.as<int>() + apply_call % kApplyCalls, apply_call, st);
     }
     // the whole operator, the pruned one making room for it where there is none
     const DevCSR& whole(int which) {
+        const auto it = dev.find(which);
+        if (it != dev.end()) return it->second->d;
+        Use use(*this);
         try {
             return device(which);
         } catch (const Error& e) {
-            if (e.code != SGDG_ENOMEM_BUDGET || step_dev.erase(which) == 0) throw;
+            if (e.code != SGDG_ENOMEM_BUDGET) throw;
+            if (step_dev.erase(which) + drop_spare() == 0) throw;
         }
         return device(which);
     }
     ~sgdg_op() {
+        retire();
         dev.clear();
         step_dev.clear();
         adv.reset();
@@ -623,7 +668,7 @@ int sgdg_op_device_nnz(sgdg_op* op, int which, int64_t* nnz) {
     NEED(op);
     NEED(nnz);
     op_stream(op);
-    *nnz = op->device(which).nnz;
+    *nnz = op->whole(which).nnz;
     API_END
 }
 
@@ -634,7 +679,7 @@ int sgdg_op_export_device_csr(sgdg_op* op, int which, int64_t* rowptr, int32_t* 
     NEED(col);
     NEED(val);
     cudaStream_t st = op_stream(op);
-    op->device(which);
+    op->whole(which);
     const CSR A = download_csr(*op->dev.at(which), st);
     std::memcpy(rowptr, A.rowptr.data(), sizeof(int64_t) * A.rowptr.size());
     std::memcpy(col, A.col.data(), sizeof(int32_t) * A.col.size());
@@ -752,6 +797,7 @@ static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, do
 static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t len, double t0, double t1,
                          int64_t nsteps, int nout, double* times, double* states) {
     cudaStream_t st = op_stream(op);
+    Spare::Use use(*op);
     std::vector<double> s;  // -sum_d a_d D_d
     for (int d = 0; a && d < op->ix.D; d++) s.push_back(-a[d]);
     if (op->prunes(a == nullptr, op->kPruneWave)) {
@@ -761,7 +807,8 @@ static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t
             CK(op->adv->scale(op->ix.D, s.data(), st));
             A = &op->adv->A.d;
         } else {
-            A = &op->stepping(SGDG_OP_WAVE_RHS);
+            A = op->stepping(SGDG_OP_WAVE_RHS);
+            if (!A) throw Error(SGDG_ENOMEM_BUDGET, "no room");
         }
         if (!plain_run(*A, y0, len, t0, t1, nsteps, nout, times, states, st)) return;
     }
@@ -828,16 +875,15 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
     }
     std::unique_ptr<PlainScratch> work;
     DevBuf keep;
-    const DevSliced* A = nullptr;
-    if (op->prunes(which < 1, op->kPruneWave)) {
+    Spare::Use use(*op);
+    const DevSliced* A = op->prunes(which < 1, op->kPruneWave) ? op->stepping(which) : nullptr;
+    if (A) {
         try {
-            A = &op->stepping(which);
             work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));
             keep.alloc(sizeof(double) * (size_t)(nsolves * A->m));
         } catch (const Error& e) {
             if (e.code != SGDG_ENOMEM_BUDGET) throw;
             work.reset();
-            op->step_dev.erase(which);
         }
     }
     if (keep.p) {
@@ -853,10 +899,13 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
         work.reset();
     }
     const DevCSR& W = op->whole(which);
-    try {
-        work.reset(new PlainScratch(W, nsolves, plain_set_size(W, nsolves)));
-    } catch (const Error&) {
-        work.reset(new PlainScratch(W, nsolves, 1));
+    for (int nv = plain_set_size(W, nsolves); !work;) {
+        try {
+            work.reset(new PlainScratch(W, nsolves, nv));
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET || (nv == 1 && !op->drop_spare())) throw;
+            nv = 1;
+        }
     }
     work->run(W, nsolves, y, dt, nsteps, cs);
     work->recycle();
@@ -1554,6 +1603,7 @@ int sgdg_set_hbm_budget(int64_t bytes) {
     API_BEGIN
     if (bytes < 0) throw Error(SGDG_EINVAL, "budget must be >= 0");
     g_budget = bytes;
+    g_budget_set++;
     if (bytes > 0) device_pool().trim((size_t)std::max<int64_t>(0, bytes - g_in_use.load()));
     API_END
 }

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <iterator>
 #include <map>
@@ -24,6 +25,7 @@ namespace sgdg {
     } while (0)
 
 inline std::atomic<int64_t> g_budget{0};
+inline std::atomic<int> g_budget_set{0};  // counts the calls that set it
 inline std::atomic<int64_t> g_in_use{0};
 
 inline void require_gpu() {
@@ -109,6 +111,62 @@ inline DevPool& device_pool() {
     return *p;
 }
 
+// Device memory that its owner, a handle, can do without (an operator's second,
+// faster form): given back where an allocation or the budget needs the room, so
+// that holding it never refuses a call.  The owner holds a Use while it looks at
+// that memory, changes it or launches with it; between its calls any thread may
+// take it (its destructor calls retire() before anything else).
+class Spare {
+   public:
+    // frees what idle handles can do without; false: there was nothing
+    static bool give_back() {
+        std::lock_guard<std::mutex> g(mutex());
+        bool any = false;
+        for (Spare* s : all())
+            if (s->users_ == 0) any = s->drop_spare() || any;
+        return any;
+    }
+    struct Use {
+        explicit Use(Spare& s) : s_(s) {
+            std::lock_guard<std::mutex> g(mutex());
+            s_.users_++;
+        }
+        ~Use() { s_.users_--; }
+        Use(const Use&) = delete;
+        Use& operator=(const Use&) = delete;
+
+       private:
+        Spare& s_;
+    };
+
+   protected:
+    Spare() {
+        std::lock_guard<std::mutex> g(mutex());
+        all().push_back(this);
+    }
+    Spare(const Spare&) = delete;
+    Spare& operator=(const Spare&) = delete;
+    virtual ~Spare() { retire(); }
+    void retire() {
+        std::lock_guard<std::mutex> g(mutex());
+        auto& a = all();
+        a.erase(std::remove(a.begin(), a.end(), this), a.end());
+    }
+    // frees it (cudaFree waits for the launches that use it); whether there was any
+    virtual bool drop_spare() = 0;
+
+   private:
+    static std::mutex& mutex() {
+        static std::mutex* m = new std::mutex;
+        return *m;
+    }
+    static std::vector<Spare*>& all() {
+        static std::vector<Spare*>* a = new std::vector<Spare*>;
+        return *a;
+    }
+    std::atomic<int> users_{0};
+};
+
 // Device allocation counted against the HBM budget (sgdg_set_hbm_budget).
 struct DevBuf {
     void* p = nullptr;
@@ -138,17 +196,19 @@ struct DevBuf {
         release();
         if (n == 0) n = 16;
         const int64_t b = g_budget.load();
-        if (b > 0 && g_in_use.load() + (int64_t)n > b)
+        auto over = [&] { return b > 0 && g_in_use.load() + (int64_t)n > b; };
+        if (over() && !(Spare::give_back() && !over()))
             throw Error(SGDG_ENOMEM_BUDGET, "HBM budget exceeded: requested " + std::to_string(n) + " bytes, " +
                                                 std::to_string(g_in_use.load()) + " of " + std::to_string(b) +
                                                 " in use");
         p = device_pool().take(n, b > 0, size);
         if (!p) {
             size = DevPool::rounded(n);
-            if (b > 0) device_pool().trim((size_t)(b - g_in_use.load() - (int64_t)n));
+            if (b > 0) device_pool().trim((size_t)std::max<int64_t>(0, b - g_in_use.load() - (int64_t)n));
             cudaError_t e = cudaMalloc(&p, size);
-            if (e == cudaErrorMemoryAllocation && device_pool().held() > 0) {
+            for (int more = 0; e == cudaErrorMemoryAllocation && more < 2; more++) {
                 cudaGetLastError();
+                if (more == 0 ? device_pool().held() == 0 : !Spare::give_back()) continue;
                 device_pool().trim(0);
                 e = cudaMalloc(&p, size);
             }

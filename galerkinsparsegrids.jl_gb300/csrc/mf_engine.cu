@@ -130,8 +130,9 @@ int MFEngine::add(const SolveSpec& sp, const double* y0, const float* weights) {
     // admission: the solve's arena share must fit the HBM budget now
     const int64_t need = solve_bytes(s.N, s.Ns, sp.kind, sp.D);
     const int64_t budget = g_budget.load();
-    const int64_t held = g_in_use.load() - dead_bytes() + pending_bytes_;
-    if (budget > 0 && held + need > budget)
+    int64_t held = 0;
+    auto over = [&] { return (held = g_in_use.load() - dead_bytes() + pending_bytes_) + need > budget; };
+    if (budget > 0 && over() && !(Spare::give_back() && !over()))
         throw Error(SGDG_ENOMEM_BUDGET, "HBM budget: solve needs " + std::to_string(need) + " bytes, " +
                                             std::to_string(held) + " of " + std::to_string(budget) + " committed");
     if (y0) s.pending.assign(y0, y0 + s.Ns);

@@ -210,8 +210,12 @@ class Server {
             const int64_t budget = g_budget.load();
             if (budget > 0) {
                 // bytes held once removed solves are freed, plus what a re-plan holds on top
-                const int64_t held = g_in_use.load() - eng_.dead_bytes() + eng_.pending_bytes();
-                if (held + eng_.replan_reserve() + need > budget) {
+                int64_t held = 0;
+                auto over = [&] {
+                    held = g_in_use.load() - eng_.dead_bytes() + eng_.pending_bytes();
+                    return held + eng_.replan_reserve() + need > budget;
+                };
+                if (over() && !(Spare::give_back() && !over())) {
                     // the head of the line waits for memory, unless nothing is left to free
                     if (!running_.empty() || eng_.pending_bytes() > 0) break;
                     if (eng_.dead_bytes() > 0) {  // free the finished solves' arenas and look again
