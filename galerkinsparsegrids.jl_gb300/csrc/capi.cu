@@ -138,6 +138,12 @@ struct sgdg_op : Spare {
         }
         return &it->second->d;
     }
+    // sum_d s[d] D_d, as stepping()
+    const DevSliced* advection(const double* s) {
+        if (!adv && !build_pruned(kAdvection, [&] { adv = gpu_advection(ix, *dlf, stream); })) return nullptr;
+        CK(adv->scale(ix.D, s, stream));
+        return &adv->A.d;
+    }
     template <class Build>
     bool build_pruned(int which, Build&& build) {
         const auto f = refused.find(which);
@@ -769,11 +775,12 @@ template <class Mat>
 static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, double t1, int64_t nsteps, int nout,
                       double* times, double* states, cudaStream_t st) {
     const size_t b = sizeof(double) * (size_t)len;
-    DevBuf work(4 * b + sizeof(int));
+    constexpr bool pruned = std::is_same_v<Mat, DevSliced>;  // to be repeated where a result is not finite
+    DevBuf work(4 * b + (pruned ? sizeof(int) : 0));
     double* y = work.as<double>();
     double *acc = y + len, *u0 = y + 2 * len, *u1 = y + 3 * len;
-    int* flag = reinterpret_cast<int*>(y + 4 * len);
-    CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    int* flag = pruned ? reinterpret_cast<int*>(y + 4 * len) : nullptr;
+    if (flag) CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
     CK(cudaMemcpyAsync(y, y0, b, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
     const auto steps = out_steps(nsteps, nout);
@@ -786,40 +793,45 @@ static bool plain_run(const Mat& A, const double* y0, int64_t len, double t0, do
         CK(cudaMemcpyAsync(states + (size_t)i * len, y, b, cudaMemcpyDeviceToHost, st));
         if (times) times[i] = t0 + (t1 - t0) * double(steps[i]) / double(nsteps);
     }
-    CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (flag) CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     work.recycle();
     return bad != 0;
 }
 
 // The wave (a = null) or advection with velocity a, stepped with the pruned
-// operator; again with the whole one if a stage was not finite.
+// operator; with the whole one if a stage was not finite, or where there is no
+// room for the pruned one and the vectors.
 static void plain_evolve(sgdg_op* op, const double* a, const double* y0, int64_t len, double t0, double t1,
                          int64_t nsteps, int nout, double* times, double* states) {
     cudaStream_t st = op_stream(op);
     Spare::Use use(*op);
     std::vector<double> s;  // -sum_d a_d D_d
     for (int d = 0; a && d < op->ix.D; d++) s.push_back(-a[d]);
-    if (op->prunes(a == nullptr, op->kPruneWave)) {
-        const DevSliced* A = nullptr;
+    const DevSliced* P = nullptr;
+    if (op->prunes(a == nullptr, op->kPruneWave)) P = a ? op->advection(s.data()) : op->stepping(SGDG_OP_WAVE_RHS);
+    try {
+        if (P && !plain_run(*P, y0, len, t0, t1, nsteps, nout, times, states, st)) return;
+    } catch (const Error& e) {
+        if (e.code != SGDG_ENOMEM_BUDGET) throw;
+    }
+    auto run = [&] {
         if (a) {
-            if (!op->adv) op->adv = gpu_advection(op->ix, *op->dlf, st);
-            CK(op->adv->scale(op->ix.D, s.data(), st));
-            A = &op->adv->A.d;
+            op->adv.reset();
+            // assembled on the GPU (the same entries as add_scaled)
+            const auto A = gpu_scaled_sum(op->ix, *op->dlf, s.data(), st);
+            plain_run(A->d, y0, len, t0, t1, nsteps, nout, times, states, st);
         } else {
-            A = op->stepping(SGDG_OP_WAVE_RHS);
-            if (!A) throw Error(SGDG_ENOMEM_BUDGET, "no room");
+            plain_run(op->whole(SGDG_OP_WAVE_RHS), y0, len, t0, t1, nsteps, nout, times, states, st);
         }
-        if (!plain_run(*A, y0, len, t0, t1, nsteps, nout, times, states, st)) return;
+    };
+    try {
+        run();
+        return;
+    } catch (const Error& e) {
+        if (e.code != SGDG_ENOMEM_BUDGET || !op->drop_spare()) throw;
     }
-    if (a) {
-        op->adv.reset();
-        // assembled on the GPU (the same entries as add_scaled)
-        const auto A = gpu_scaled_sum(op->ix, *op->dlf, s.data(), st);
-        plain_run(A->d, y0, len, t0, t1, nsteps, nout, times, states, st);
-    } else {
-        plain_run(op->whole(SGDG_OP_WAVE_RHS), y0, len, t0, t1, nsteps, nout, times, states, st);
-    }
+    run();
 }
 
 // The scratch of nsteps RK4 steps of nb solves sharing A.

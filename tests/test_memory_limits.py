@@ -55,3 +55,88 @@ def test_application_gives_the_pruned_operator_back(sgdg, budget):
     assert np.linalg.norm(big.apply(x, 0) - first) <= 1e-10 * np.linalg.norm(first)
     big.close()
     small.close()
+
+
+def rk4(A, y, dt, nsteps):
+    for _ in range(nsteps):
+        k1 = A @ y
+        k2 = A @ (y + 0.5 * dt * k1)
+        k3 = A @ (y + 0.5 * dt * k2)
+        y = y + dt / 6 * (k1 + 2 * k2 + 2 * k3 + A @ (y + dt * k3))
+    return y
+
+
+def wave(sgdg, op, y, dt=1e-4, steps=3):
+    _, st = sgdg.wave_evolve(op.D, op.k, op.n, y[:op.N], y[op.N:], 0.0, steps * dt, nsteps=steps, op=op)
+    return st[-1]
+
+
+def advect(sgdg, op, y, dt=1e-4, steps=3):
+    a = np.linspace(0.5, 1.0, op.D)
+    _, st = sgdg.advect_evolve(op.D, op.k, op.n, a, y[:op.N], 0.0, steps * dt, nsteps=steps, op=op)
+    return st[-1]
+
+
+def vectors(op):  # of a wave's evolution
+    return 4 * 8 * 2 * op.N + 64
+
+
+def test_wave_without_room_for_the_pruned_operator(sgdg, budget):
+    # the whole operator is there, or a run that was not finite has built it
+    op = sgdg.SparseGridOperator(3, 3, 5)
+    y = np.random.default_rng(0).standard_normal(2 * op.N)
+    ref = rk4(op.csr(-1), y, 1e-4, 3)
+    op.device_csr(-1)
+    budget(vectors(op))
+    for _ in range(2):
+        assert np.linalg.norm(wave(sgdg, op, y) - ref) <= 1e-10 * np.linalg.norm(ref)
+    sgdg.set_hbm_budget(0)
+    got = wave(sgdg, op, y)  # with the pruned one again
+    bad = y.copy()
+    bad[3] = np.nan
+    assert not np.all(np.isfinite(wave(sgdg, op, bad)))
+    budget(0)  # the pruned one makes room for the vectors
+    assert np.linalg.norm(wave(sgdg, op, y) - got) <= 1e-10 * np.linalg.norm(got)
+    op.close()
+
+
+def test_advection_gives_its_operator_back(sgdg, budget):
+    op, other = sgdg.SparseGridOperator(3, 3, 6), sgdg.SparseGridOperator(3, 2, 4)
+    y = np.random.default_rng(1).standard_normal(op.N)
+    before = sgdg.hbm_in_use()
+    first = advect(sgdg, op, y)
+    assert sgdg.hbm_in_use() > before + (1 << 20)  # kept for the next call
+    budget(0)
+    z = np.random.default_rng(2).standard_normal(2 * other.N)
+    ref = rk4(other.csr(-1), z, 1e-4, 3)
+    assert np.linalg.norm(wave(sgdg, other, z) - ref) <= 1e-10 * np.linalg.norm(ref)
+    # and back again, whichever operator fits now
+    sgdg.set_hbm_budget(0)
+    assert np.array_equal(advect(sgdg, op, y), first)
+    op.close()
+    other.close()
+
+
+@pytest.mark.parametrize("evolve", [wave, advect])
+def test_a_run_after_one_that_was_not_finite(sgdg, budget, evolve):
+    # at every budget under which a run that is not finite fits, on a fresh handle
+    # as in a sequence, a finite one does as well
+    y = np.random.default_rng(3).standard_normal(2 * sgdg.get_size(3, 3, 5))
+    bad = y.copy()
+    bad[3] = np.inf
+    ran = 0
+    for extra in np.geomspace(1 << 20, 64 << 20, 13):
+        op = sgdg.SparseGridOperator(3, 3, 5)
+        budget(int(extra))
+        try:
+            evolve(sgdg, op, bad)
+        except sgdg.SGDGError as e:
+            assert e.code == 2
+        else:
+            ran += 1
+            assert np.all(np.isfinite(evolve(sgdg, op, y)))
+            assert not np.all(np.isfinite(evolve(sgdg, op, bad)))
+            assert np.all(np.isfinite(evolve(sgdg, op, y)))
+        sgdg.set_hbm_budget(0)
+        op.close()
+    assert 0 < ran < 13
