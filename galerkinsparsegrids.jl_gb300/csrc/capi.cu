@@ -240,8 +240,9 @@ struct sgdg_op : Spare {
 // where the assembled transforms hold 147 + 120 + 12 + 244, and the derivatives
 // go without the rounding of zeros (22 entries instead of 50).  The assembled
 // operators (whole_rhs) are built and used when a run meets a value that is not
-// finite, which they spread over more rows.
-struct sgdg_vlasov {
+// finite, which they spread over more rows, or where the sweeps have no room;
+// once they are there, the sweeps give way to an allocation that needs theirs.
+struct sgdg_vlasov : Spare {
     int D = 0, P = 0, k = 0, n = 0;
     SparseIndex ix;
     std::shared_ptr<const DLF1D> dlf;
@@ -258,7 +259,9 @@ struct sgdg_vlasov {
     DevBuf p;                   // P vectors for the assembled operators
     DevBuf flag;                // a result was not finite
     cudaStream_t stream = nullptr;
+    int refused = -1;           // the budget (g_budget_set) that had no room for the sweeps
     ~sgdg_vlasov() {
+        retire();
         if (stream) cudaStreamDestroy(stream);
     }
     const CSR& host_transform(int w) const {
@@ -290,11 +293,12 @@ struct sgdg_vlasov {
         }
         have_vpoint = true;
     }
-    void to_gpu() {
+    void to_gpu() {  // the caller holds a Use
         if (flag.p) return;
         require_gpu();
         if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        build_sweeps();
+        const bool sweeps = have_sweeps();
+        if (!sweeps) build_whole();
         const size_t b = sizeof(double) * (size_t)ix.N;
         if (!have_vpoint) {  // n2p m2n with the device transforms
             DevBuf x(b), y(b);
@@ -303,7 +307,14 @@ struct sgdg_vlasov {
                 const std::vector<double> vm = v_modal(d);
                 CK(cudaMemcpyAsync(x.p, vm.data(), b, cudaMemcpyHostToDevice, stream));
                 double *from = x.as<double>(), *to = y.as<double>();
-                for (int w : {0, 1}) CK(transform(w, sweep[w].size(), 1, from, to));
+                for (int w : {0, 1}) {
+                    if (sweeps) {
+                        CK(transform(w, sweep[w].size(), 1, from, to));
+                    } else {
+                        CK(launch_csr_spmv(dT[w]->d, from, to, stream));
+                        std::swap(from, to);
+                    }
+                }
                 CK(cudaMemcpyAsync(v_point.data() + (size_t)d * ix.N, from, b, cudaMemcpyDeviceToHost, stream));
                 CK(cudaStreamSynchronize(stream));
             }
@@ -315,8 +326,8 @@ struct sgdg_vlasov {
         s.alloc(b * P);
         c.alloc(b);
         z.alloc(b);
-        flag.alloc(sizeof(int));
         CK(cudaStreamSynchronize(stream));
+        flag.alloc(sizeof(int));
     }
     // Dimensions a sweep of transform w takes at once.  More at once multiply
     // more entries (the product of the dimensions' rows instead of their sum) in
@@ -352,6 +363,27 @@ struct sgdg_vlasov {
     void drop_sweeps() {
         for (auto& d : deriv) d.reset();
         for (auto& s : sweep) s.clear();
+    }
+    // builds the sweeps where there is room for them; false: the assembled
+    // operators are to be used
+    bool have_sweeps() {
+        if (!sweep[3].empty()) return true;
+        if (refused == g_budget_set.load()) return false;
+        try {
+            build_sweeps();
+            return true;
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET) throw;
+        }
+        drop_sweeps();
+        refused = g_budget_set.load();
+        return false;
+    }
+    bool drop_spare() override {
+        if (!p.p || sweep[3].empty()) return false;
+        drop_sweeps();
+        refused = g_budget_set.load();
+        return true;
     }
     // the first `count` sweeps of transform w of nv interleaved vectors, from x;
     // the result is in x, y is scratch (the two pointers change places)
@@ -401,6 +433,7 @@ struct sgdg_vlasov {
         } catch (const Error& e) {
             if (e.code != SGDG_ENOMEM_BUDGET || sweep[3].empty()) throw;
             drop_sweeps();
+            refused = g_budget_set.load();
             build();
         }
     }
@@ -1122,9 +1155,11 @@ int sgdg_vlasov_v_point(const sgdg_vlasov* v, double* out) {
     NEED(out);
     if (!v->have_vpoint) {
         int ndev = 0;
-        if (cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0)
-            const_cast<sgdg_vlasov*>(v)->to_gpu();
-        else {
+        if (cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0) {
+            sgdg_vlasov* m = const_cast<sgdg_vlasov*>(v);
+            Spare::Use use(*m);
+            m->to_gpu();
+        } else {
             cudaGetLastError();
             v->vpoint_host();
         }
@@ -1188,22 +1223,27 @@ int sgdg_vlasov_rhs(sgdg_vlasov* v, const double* F_point, const double* f, doub
     NEED(F_point);
     NEED(f);
     NEED(out);
-    v->to_gpu();
     const int64_t N = v->ix.N;
     const size_t b = sizeof(double) * (size_t)N;
-    DevBuf u(b), r(b);
-    int bad = 0;
+    {
+        Spare::Use use(*v);
+        v->to_gpu();
+    }
+    DevBuf u(b), r(b);  // the sweeps may give way to them
+    Spare::Use use(*v);
     CK(cudaMemcpyAsync(v->F.p, F_point, b * v->D, cudaMemcpyHostToDevice, v->stream));
     CK(cudaMemcpyAsync(u.p, f, b, cudaMemcpyHostToDevice, v->stream));
-    CK(cudaMemsetAsync(v->flag.p, 0, sizeof(int), v->stream));
-    v->build_sweeps();
-    CK(launch_check_finite(u.as<double>(), N, v->flag.as<int>(), v->stream));
-    double* last = nullptr;
-    CK(v->sweep_rhs(u.as<double>(), &last));
-    CK(launch_sweep(v->last_sweep(), 1, last, r.as<double>(), v->flag.as<int>(), v->stream));
-    CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
-    CK(cudaMemcpyAsync(&bad, v->flag.p, sizeof(int), cudaMemcpyDeviceToHost, v->stream));
-    CK(cudaStreamSynchronize(v->stream));
+    int bad = 1;
+    if (v->have_sweeps()) {
+        CK(cudaMemsetAsync(v->flag.p, 0, sizeof(int), v->stream));
+        CK(launch_check_finite(u.as<double>(), N, v->flag.as<int>(), v->stream));
+        double* last = nullptr;
+        CK(v->sweep_rhs(u.as<double>(), &last));
+        CK(launch_sweep(v->last_sweep(), 1, last, r.as<double>(), v->flag.as<int>(), v->stream));
+        CK(cudaMemcpyAsync(out, r.p, b, cudaMemcpyDeviceToHost, v->stream));
+        CK(cudaMemcpyAsync(&bad, v->flag.p, sizeof(int), cudaMemcpyDeviceToHost, v->stream));
+        CK(cudaStreamSynchronize(v->stream));
+    }
     if (bad) {
         v->build_whole();
         CK(v->whole_rhs(u.as<double>()));
@@ -1252,11 +1292,15 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
         return SGDG_OK;
     }
     if (method != SGDG_METHOD_PLAIN) throw Error(SGDG_EINVAL, "method must be PLAIN (0) or MATFREE (1)");
-    v->to_gpu();
+    {
+        Spare::Use use(*v);
+        v->to_gpu();
+    }
     cudaStream_t st = v->stream;
     const int64_t N = v->ix.N;
     const size_t b = sizeof(double) * (size_t)N;
-    DevBuf y(b), acc(b), u0(b), u1(b);
+    DevBuf y(b), acc(b), u0(b), u1(b);  // the sweeps may give way to them
+    Spare::Use use(*v);
     CK(cudaMemcpyAsync(v->F.p, F_point, b * v->D, cudaMemcpyHostToDevice, st));
     const double dt = (t1 - t0) / double(nsteps);
     const double* in[4] = {y.as<double>(), u0.as<double>(), u1.as<double>(), u0.as<double>()};
@@ -1296,8 +1340,7 @@ int sgdg_vlasov_evolve(sgdg_vlasov* v, const double* F_point, const double* f0, 
         CK(cudaStreamSynchronize(st));
         return bad != 0;
     };
-    v->build_sweeps();
-    if (run(false)) {
+    if (!v->have_sweeps() || run(false)) {
         v->build_whole();
         run(true);
     }

@@ -140,3 +140,52 @@ def test_a_run_after_one_that_was_not_finite(sgdg, budget, evolve):
         sgdg.set_hbm_budget(0)
         op.close()
     assert 0 < ran < 13
+
+
+def vlasov(sgdg, seed=5):
+    v = sgdg.VlasovOperator(2, 2, 4)
+    rng = np.random.default_rng(seed)
+    return v, rng.standard_normal((2, v.N)), rng.standard_normal(v.N)
+
+
+def test_vlasov_without_room_for_the_sweeps(sgdg, budget):
+    v, F, f = vlasov(sgdg)
+    ref = v.rhs(F, f)
+    bad = f.copy()
+    bad[3] = np.nan
+    assert not np.all(np.isfinite(v.rhs(F, bad)))  # builds the assembled operators
+
+    def evolve():
+        return sgdg.vlasov_evolve(2, 2, 4, F, f, 0.0, 3e-4, nsteps=3, op=v)[1][-1]
+    evolved = evolve()
+    for call in range(2):
+        budget(0)  # the sweeps make room for the vectors
+        got = evolve() if call else v.rhs(F, f)
+        want = evolved if call else ref
+        # the same right-hand side in another order of its sums (at most 1e4 terms of the
+        # size of the largest, which a transform grows by less than 100)
+        assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want)
+        sgdg.set_hbm_budget(0)
+        assert np.array_equal(v.rhs(F, f), ref)  # with the sweeps again
+    v.close()
+
+
+def test_vlasov_run_after_one_that_was_not_finite(sgdg, budget):
+    ran = 0
+    for extra in np.geomspace(1 << 18, 256 << 20, 21):
+        v, F, f = vlasov(sgdg)
+        bad = f.copy()
+        bad[3] = np.inf
+        budget(int(extra))
+        try:
+            v.rhs(F, bad)
+        except sgdg.SGDGError as e:
+            assert e.code == 2
+        else:
+            ran += 1
+            assert np.all(np.isfinite(v.rhs(F, f)))
+            assert not np.all(np.isfinite(v.rhs(F, bad)))
+            assert np.all(np.isfinite(v.rhs(F, f)))
+        sgdg.set_hbm_budget(0)
+        v.close()
+    assert 0 < ran < 21
