@@ -389,6 +389,7 @@ struct EvalTables {
     Pencils P{};
     int64_t items = 0, numbers = 0;  // of k_lines; of its output
     size_t psmem = 0;
+    int refused = -1;  // the budget (g_budget_set) that had no room for them
 };
 
 constexpr int kPencilMaxK = 5;
@@ -432,9 +433,7 @@ std::vector<double> two_scale(int k) {
     return out;
 }
 
-const Pencils& eval_pencils(EvalTables& T) {
-    std::lock_guard<std::mutex> g(T.mu);
-    if (T.P.np > 0) return T.P;
+void build_pencils(EvalTables& T) {
     const SparseIndex& ix = T.ix;
     const int D = ix.D, k = ix.k, n = ix.n;
     Pencils P{};
@@ -497,7 +496,22 @@ const Pencils& eval_pencils(EvalTables& T) {
     T.psmem = sizeof(double) * kPencilPts * ((size_t)D * (n + 1) * k + kPencilParts) + sizeof(int) * kPencilPts * D;
     P.np = (int)lmax.size();
     T.P = P;
-    return T.P;
+}
+
+// null where there is no room for them, now or earlier under the same budget
+const Pencils* eval_pencils(EvalTables& T) {
+    std::lock_guard<std::mutex> g(T.mu);
+    if (T.P.np > 0) return &T.P;
+    if (T.refused == g_budget_set.load()) return nullptr;
+    try {
+        build_pencils(T);
+        return &T.P;
+    } catch (const Error& e) {
+        if (e.code != SGDG_ENOMEM_BUDGET) throw;
+    }
+    for (DevBuf* b : {&T.lmax, &T.base, &T.scale, &T.plevels, &T.item, &T.plev_off, &T.two}) b->release();
+    T.refused = g_budget_set.load();
+    return nullptr;
 }
 
 template <int K>
@@ -552,9 +566,9 @@ void evaluate_impl(int D, int k, int n, int scheme, const double* coeffs, int64_
     if (npts == 0) return;
     if (k <= kPencilMaxK && npts >= kPencilPoints && npts * T.ix.nlev * T.ix.kD >= kPencilTerms &&
         npts < (int64_t(1) << 31) * kPencilPts) {
-        const Pencils& P = eval_pencils(T);
+        const Pencils* P = eval_pencils(T);
         DevBuf work;
-        if (T.psmem <= 200 * 1024) try {
+        if (P && T.psmem <= 200 * 1024) try {
                 work.alloc(sizeof(double) * (size_t)T.numbers + 2 * sizeof(int));
             } catch (const Error&) {  // no room: k_evaluate needs none
             }
@@ -563,7 +577,7 @@ void evaluate_impl(int D, int k, int n, int scheme, const double* coeffs, int64_
             CK(cudaMemsetAsync(err, 0, 2 * sizeof(int), st));
             auto launch = k == 1 ? launch_pencils<1> : k == 2 ? launch_pencils<2> : k == 3 ? launch_pencils<3>
                         : k == 4 ? launch_pencils<4> : launch_pencils<5>;
-            CK(launch(T, P, coeffs, npts, xs, out, work.as<double>(), err, st));
+            CK(launch(T, *P, coeffs, npts, xs, out, work.as<double>(), err, st));
             int h[2] = {0, 0};
             CK(cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));

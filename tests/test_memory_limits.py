@@ -189,3 +189,17 @@ def test_vlasov_run_after_one_that_was_not_finite(sgdg, budget):
         sgdg.set_hbm_budget(0)
         v.close()
     assert 0 < ran < 21
+
+
+def test_many_points_without_room_for_the_pencils(sgdg, budget):
+    D, k, n, points = 3, 4, 3, 1 << 15
+    rng = np.random.default_rng(7)
+    c = rng.standard_normal(sgdg.get_size(D, k, n))
+    x = rng.uniform(0, 1, (points, D))
+    few = [sgdg.reconstruct_DG(D, k, n, c, part) for part in np.array_split(x, 16)]  # block by block
+    budget(8 * (c.size + points * (D + 1)) + 64)
+    for _ in range(2):
+        assert np.array_equal(sgdg.reconstruct_DG(D, k, n, c, x), np.concatenate(few))
+    sgdg.set_hbm_budget(0)
+    # the sums in another order: 1e3 terms a point at most, none above |c| 8^1.5 k^1.5 = 500
+    assert np.allclose(sgdg.reconstruct_DG(D, k, n, c, x), np.concatenate(few), rtol=0, atol=1e-10)
