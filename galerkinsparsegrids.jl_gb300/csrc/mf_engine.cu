@@ -70,7 +70,9 @@ static int mf_ctas_per_sm(double items_per_phase, int most);
 MFEngine::~MFEngine() { drop_chunks(); }
 
 void MFEngine::set_stream(cudaStream_t st) {
-    if (st != stream_) drop_chunks();
+    if (st == stream_) return;
+    drop_chunks();
+    moved_ = moved_ || !classes_.empty();
     stream_ = st;
 }
 
@@ -248,7 +250,12 @@ const MFEngine::QTable& MFEngine::qtab(int k, int n) {
 void MFEngine::plan() {
     if (!dirty_) return;
     drop_chunks();
-    CK(cudaStreamSynchronize(stream_));  // the old arenas' work: their blocks are reused below
+    // The old arenas' work has to end: their blocks are reused below.  It may be on
+    // other streams than this one, which may be gone by now, or in replays of a
+    // captured step: then as the destructor, by cudaFree, which waits for all.
+    if (moved_ || captured_) ctr_d_.release();
+    moved_ = false;
+    CK(cudaStreamSynchronize(stream_));
     if (!err_d_.p) {
         err_d_.alloc(sizeof(int));
         CK(cudaMemsetAsync(err_d_.p, 0, sizeof(int), stream_));
@@ -1107,6 +1114,9 @@ void MFEngine::step_host(const double* in, double* out, int64_t nsteps, int nchu
 void MFEngine::step(int64_t nsteps) {
     plan();
     if (nitems_ == 0 || nsteps <= 0) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream_, &cap) != cudaSuccess) cudaGetLastError();
+    captured_ = captured_ || cap != cudaStreamCaptureStatusNone;
     for (int64_t i = 0; i < nsteps; i++)
         CK(launch_mf_step(items_d_.as<MFItem>(), nitems_, classes_d_.as<MFClass>(), ctr_d_.as<int>(), nctr_,
                           err_d_.as<int>(), smem_, table_bytes_, grid_, stream_));

@@ -52,6 +52,8 @@ class MFEngine {
     MFEngine(const MFEngine&) = delete;
     MFEngine& operator=(const MFEngine&) = delete;
 
+    // The work that comes is on st; the caller orders it after what the old stream
+    // still runs, except where a re-plan comes first, which waits for that.
     void set_stream(cudaStream_t st);
     cudaStream_t stream() const { return stream_; }
     // false for an engine that is stepped a few times only between its re-plans
@@ -159,6 +161,8 @@ class MFEngine {
     int table_bytes_ = 0;  // shared-memory operator table reserved ahead of the tile
     bool dirty_ = true;
     bool list_order_ = true;
+    bool moved_ = false;     // the stream was changed since the plan
+    bool captured_ = false;  // a step was captured: its replays may be on any stream
     struct Chunk {  // step_host's pipeline stage
         DevBuf items, ctr;
         int nitems = 0, nctr = 0;
