@@ -6,6 +6,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -157,13 +158,13 @@ struct sgdg_op : Spare {
             return false;
         }
     }
-    // what is there beside the whole operators
+    // what is there beside the whole operators, but for captured calls'
     bool drop_spare() override {
         bool any = adv != nullptr;
         if (adv) refused[kAdvection] = g_budget_set.load();
         adv.reset();
         for (auto it = step_dev.begin(); it != step_dev.end();) {
-            if (!dev.count(it->first)) {
+            if (!dev.count(it->first) || in_graphs.count(it->first)) {
                 ++it;
                 continue;
             }
@@ -180,18 +181,33 @@ struct sgdg_op : Spare {
     // caller's, two launches for one), and where an element of x is not finite
     // through the whole one after it (k_apply_whole).  Each call leaves its number
     // in a word of its own among kApplyCalls: calls on other streams may still be
-    // in flight.
+    // in flight.  A captured call, whose number is the same in every replay, has a
+    // word for good, cleared in the graph, and keeps the pruned operator there; with
+    // a budget set, without the operator, or after kApplyCalls of them, it is
+    // captured with the whole one.
     static constexpr int64_t kApplyPruned = 3 << 19;
     static constexpr int kApplyCalls = 1024;
-    DevBuf apply_seen;
-    int apply_call = 0;
+    DevBuf apply_seen;  // the calls' words, then those of captured calls
+    int apply_call = 0, apply_captured = 0;
+    std::set<int> in_graphs;  // `which` of pruned operators that captured calls use
     cudaError_t apply(int which, const double* x, double* y, cudaStream_t st) {
         const DevCSR& A = whole(which);
         if (!prunes(true, kPruneApply) || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(st, &cap);
+        if (e != cudaSuccess) return e;
         Use use(*this);
+        if (cap != cudaStreamCaptureStatusNone) {
+            if (g_budget.load() > 0 || !apply_seen.p || !step_dev.count(which) || apply_captured == kApplyCalls)
+                return launch_csr_spmv(A, x, y, st);
+            in_graphs.insert(which);
+            int* seen = apply_seen.as<int>() + kApplyCalls + apply_captured++;
+            const cudaError_t m = cudaMemsetAsync(seen, 0, sizeof(int), st);
+            return m != cudaSuccess ? m : launch_apply(step_dev.at(which)->d, A, x, y, seen, 1, st);
+        }
         const DevSliced* P = stepping(which);
         if (P && !apply_seen.p && !build_pruned(which, [&] {
-                DevBuf seen(sizeof(int) * kApplyCalls);
+                DevBuf seen(2 * sizeof(int) * kApplyCalls);
                 CK(cudaMemsetAsync(seen.p, 0, seen.bytes, stream));
                 CK(cudaStreamSynchronize(stream));
                 apply_seen = std::move(seen);
@@ -210,7 +226,7 @@ struct sgdg_op : Spare {
             return device(which);
         } catch (const Error& e) {
             if (e.code != SGDG_ENOMEM_BUDGET) throw;
-            if (step_dev.erase(which) + drop_spare() == 0) throw;
+            if (step_dev.erase(which) + drop_spare() == 0) throw;  // (no call of it was captured without the whole one)
         }
         return device(which);
     }
