@@ -888,8 +888,9 @@ struct PlainScratch {
     DevBuf acc, u0, u1, flag;
     int nv;
     template <class Mat>
-    PlainScratch(const Mat& A, int64_t nb, int nv_) : flag(sizeof(int)), nv(nv_) {
+    PlainScratch(const Mat& A, int64_t nb, int nv_) : nv(nv_) {
         const size_t b = sizeof(double) * (size_t)((nb + nv - 1) / nv * nv * A.m);
+        if (std::is_same_v<Mat, DevSliced>) flag.alloc(sizeof(int) * (size_t)nb);
         acc.alloc(b);
         u0.alloc(b);
         u1.alloc(b);
@@ -897,28 +898,47 @@ struct PlainScratch {
     void recycle() {  // after run
         for (DevBuf* b : {&acc, &u0, &u1, &flag}) b->recycle();
     }
-    // returns whether a stage result was not finite; waits for the steps
+    // waits for the steps; with the pruned operator, which solves had a stage result
+    // that was not finite (one int each)
     template <class Mat>
-    bool run(const Mat& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
-        int bad = 0;
+    std::vector<int> run(const Mat& A, int64_t nb, double* y, double dt, int64_t nsteps, cudaStream_t st) {
+        std::vector<int> bad(flag.p ? (size_t)nb : 0);
         StepGraph graph(8, nsteps >= kGraphSteps);
-        CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
+        if (flag.p) CK(cudaMemsetAsync(flag.p, 0, sizeof(int) * bad.size(), st));
         CK(launch_plain_interleave(A.m, nv, nb, y, u0.as<double>(), st));
         graph.run(nsteps, st, [&](int64_t n) {
             return launch_plain_steps(A, nv, nb, y, acc.as<double>(), u0.as<double>(), u1.as<double>(), dt, n,
                                       flag.as<int>(), st);
         });
-        CK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (flag.p) CK(cudaMemcpyAsync(bad.data(), flag.p, sizeof(int) * bad.size(), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        return bad != 0;
+        return bad;
     }
 };
+
+// Steps solves with the whole operator, in its own scratch.
+static void plain_whole_steps(sgdg_op* op, int which, int64_t nsolves, double* y, double dt, int64_t nsteps,
+                              cudaStream_t st) {
+    const DevCSR& W = op->whole(which);
+    std::unique_ptr<PlainScratch> work;
+    for (int nv = plain_set_size(W, nsolves); !work;) {
+        try {
+            work.reset(new PlainScratch(W, nsolves, nv));
+        } catch (const Error& e) {
+            if (e.code != SGDG_ENOMEM_BUDGET || (nv == 1 && !op->drop_spare())) throw;
+            nv = 1;
+        }
+    }
+    work->run(W, nsolves, y, dt, nsteps, st);
+    work->recycle();
+}
 
 // nsteps plain FP64 RK4 steps of nsolves solves y' = A y sharing operator
 // `which`, states device-resident one after another.  The pruned operator
 // needs the states of the call's start beside the scratch vectors, to repeat
-// the steps with the whole one if a stage was not finite; without room for
-// them, or for sets padded to whole ones, the whole operator steps the solves
+// the steps of a solve with the whole one if a stage of its was not finite (the
+// others' results stand: a solve's do not depend on its neighbours); without room
+// for them, or for sets padded to whole ones, the whole operator steps the solves
 // one by one from the start.
 static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y, double dt, int64_t nsteps,
                               cudaStream_t st) {
@@ -934,42 +954,42 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
         cs = own.s;
         CK(cudaStreamSynchronize(nullptr));
     }
-    std::unique_ptr<PlainScratch> work;
-    DevBuf keep;
     Spare::Use use(*op);
     const DevSliced* A = op->prunes(which < 1, op->kPruneWave) ? op->stepping(which) : nullptr;
-    if (A) {
-        try {
+    std::unique_ptr<PlainScratch> work;
+    DevBuf keep;
+    if (A) try {
             work.reset(new PlainScratch(*A, nsolves, plain_set_size(*A, nsolves)));
             keep.alloc(sizeof(double) * (size_t)(nsolves * A->m));
         } catch (const Error& e) {
             if (e.code != SGDG_ENOMEM_BUDGET) throw;
             work.reset();
         }
-    }
-    if (keep.p) {
-        CK(cudaMemcpyAsync(keep.p, y, keep.bytes, cudaMemcpyDeviceToDevice, cs));
-        const bool bad = work->run(*A, nsolves, y, dt, nsteps, cs);
-        if (bad) {
-            CK(cudaMemcpyAsync(y, keep.p, keep.bytes, cudaMemcpyDeviceToDevice, cs));
-            CK(cudaStreamSynchronize(cs));
-        }
-        work->recycle();
-        keep.recycle();
-        if (!bad) return;
-        work.reset();
-    }
-    const DevCSR& W = op->whole(which);
-    for (int nv = plain_set_size(W, nsolves); !work;) {
-        try {
-            work.reset(new PlainScratch(W, nsolves, nv));
-        } catch (const Error& e) {
-            if (e.code != SGDG_ENOMEM_BUDGET || (nv == 1 && !op->drop_spare())) throw;
-            nv = 1;
-        }
-    }
-    work->run(W, nsolves, y, dt, nsteps, cs);
+    if (!keep.p) return plain_whole_steps(op, which, nsolves, y, dt, nsteps, cs);
+    CK(cudaMemcpyAsync(keep.p, y, keep.bytes, cudaMemcpyDeviceToDevice, cs));
+    const std::vector<int> bad = work->run(*A, nsolves, y, dt, nsteps, cs);
     work->recycle();
+    const int64_t len = A->m;
+    auto restore = [&](int64_t first, int64_t n) {
+        CK(cudaMemcpyAsync(y + first * len, keep.as<double>() + first * len, sizeof(double) * (size_t)(n * len),
+                           cudaMemcpyDeviceToDevice, cs));
+    };
+    bool fits = true;
+    try {
+        for (int64_t i = 0, n; i < nsolves; i += n) {
+            for (n = 1; i + n < nsolves && bad[i + n] == bad[i];) n++;
+            if (!bad[i]) continue;
+            restore(i, n);
+            plain_whole_steps(op, which, n, y + i * len, dt, nsteps, cs);
+        }
+    } catch (const Error& e) {
+        if (e.code != SGDG_ENOMEM_BUDGET) throw;
+        fits = false;  // beside the states of the call's start
+    }
+    if (!fits) restore(0, nsolves);
+    CK(cudaStreamSynchronize(cs));
+    keep.recycle();
+    if (!fits) plain_whole_steps(op, which, nsolves, y, dt, nsteps, cs);
 }
 
 extern "C" {

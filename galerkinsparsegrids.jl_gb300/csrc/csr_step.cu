@@ -51,7 +51,7 @@ struct CsrRK {  // stage update of the RK4 epilogue: k = A uin, then rk_stage
     double dt, hdt, dt6;
     int stage;
     int write_u;     // stage 4 also stores the new state to uout (the next step's input when it is not y)
-    int* nonfinite;  // set to 1 when a stage result is not finite (may be null)
+    int* nonfinite;  // one per solve: set to 1 when a stage result of its is not finite (may be null)
 };
 
 // Programmatic dependent launch: waits until the launches this one depends on
@@ -144,8 +144,10 @@ __device__ __forceinline__ void row_sum(const DevCSR& A, int64_t b, int64_t e, C
 __device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
 
 // RK4 stage update of one element: k its right-hand side, yy its state and aa its
-// accumulator (from y and acc[o]), which go back there and uout[o]
-__device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double yy, double aa, double* y, int64_t o) {
+// accumulator (from y and acc[o]), which go back there and uout[o]; its solve's flag
+// is rk.nonfinite[j]
+__device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double yy, double aa, double* y, int64_t o,
+                                              int j) {
     double un;
     rk_stage(rk.stage, rk.dt, rk.hdt, rk.dt6, k, yy, aa, un);
     if (rk.stage == 4)
@@ -153,7 +155,7 @@ __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double 
     else
         rk.acc[o] = aa;
     if (rk.stage != 4 || rk.write_u) rk.uout[o] = un;
-    if (rk.nonfinite && not_finite(un)) *rk.nonfinite = 1;
+    if (rk.nonfinite && not_finite(un)) rk.nonfinite[j] = 1;
 }
 
 // Block rb's rows, 2^bin lanes each: out.one(row, j, sum) by the lane that
@@ -312,7 +314,7 @@ struct RkOut {
     __device__ __forceinline__ void one(int64_t row, int j, double s, Fetched& f) const {
         if (j >= nv) return;
         if constexpr (NV > 1) load(row, j, f);
-        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j);
+        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j, NV == 1 ? 0 : j);
     }
     __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], Fetched& f) const {
 #pragma unroll
@@ -352,6 +354,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
         y += o;
         rk.acc += o;
         rk.uout += o;
+        if (NV > 1 && rk.nonfinite) rk.nonfinite += g * NV;  // (one solve at a time for NV = 1)
     }
     block_rows<NV>(A, rb, x, NV, RkOut<NV>{rk, y, A.m, g + 1 == q.count ? q.last : NV});
 }
@@ -382,7 +385,7 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
     for (int q = A.long_seg[i]; q < A.long_seg[i + 1]; q++) s += A.partial[q];
     const int64_t row = A.long_row[i];
     if (!SGDG_IN(row, A.m)) return;
-    csr_rk_update(rk, s, y[row], rk.stage == 1 ? 0.0 : rk.acc[row], y + row, row);
+    csr_rk_update(rk, s, y[row], rk.stage == 1 ? 0.0 : rk.acc[row], y + row, row, 0);
 }
 
 // NV adjacent vectors of an interleaved set (element i of vector j at
@@ -619,7 +622,8 @@ static void rk4_sets(const Mat& A, int64_t nb, double* y, double* acc, double* u
     const int64_t most = std::max<int64_t>(1, ((int64_t(1) << 31) - 1) / std::max<int64_t>(nrb, 1));
     for (int64_t g = 0; g < ng && nrb > 0; g += most) {
         const int64_t n = std::min(most, ng - g), o = g * NV * len;
-        const CsrRK rk{acc + o, (stage % 2 ? u1 : u0) + o, dt, 0.5 * dt, dt / 6.0, stage, 1, nonfinite};
+        const CsrRK rk{acc + o, (stage % 2 ? u1 : u0) + o, dt, 0.5 * dt, dt / 6.0, stage, 1,
+                       nonfinite ? nonfinite + g * NV : nullptr};
         launch_dependent(k_csr_rk<NV, Mat>, (unsigned)(nrb * n), block_threads<Mat>, st, A, uin + o, y + o, rk,
                          CsrSets{n, kPlainSetGroup, g + n == ng ? int(nb - (ng - 1) * NV) : NV});
     }
@@ -630,7 +634,7 @@ static void rk4_sets(const Mat& A, int64_t nb, double* y, double* acc, double* u
 // a row together: the stage inputs and accumulators are interleaved, so a
 // matrix entry is loaded once per set and meets a column's values in one
 // load.  nv is plain_set_size or 1; acc, u0 and u1 hold whole sets of A.m
-// numbers a solve, and with nv > 1 u0 holds the interleaved states on entry
+// numbers a solve, nonfinite (or null) one flag a solve, and with nv > 1 u0 holds the interleaved states on entry
 // (launch_plain_interleave) and on return.
 template <class Mat>
 static cudaError_t plain_steps(const Mat& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
@@ -642,7 +646,8 @@ static cudaError_t plain_steps(const Mat& A, int nv, int64_t nb, double* y, doub
                 for (int64_t s = 0; s < nb && e == cudaSuccess; s++) {
                     const int64_t o = s * A.m;
                     const double* in = stage == 1 ? y : stage == 3 ? u1 : u0;
-                    e = launch_csr_rk4(A, in + o, y + o, acc + o, (stage == 2 ? u1 : u0) + o, dt, stage, nonfinite, st);
+                    e = launch_csr_rk4(A, in + o, y + o, acc + o, (stage == 2 ? u1 : u0) + o, dt, stage,
+                                       nonfinite ? nonfinite + s : nullptr, st);
                 }
                 continue;
             }
