@@ -41,7 +41,7 @@ cudaError_t launch_csr_spmv_multi(const DevCSR& A, int nv, const double* x, int6
 cudaError_t launch_vlasov_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
                                  cudaStream_t st);
 cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, int* nonfinite, cudaStream_t st);
-cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, double* y, int* seen, int call,
+cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, double* y, int* seen, int call, int* left,
                          cudaStream_t st);
 cudaError_t launch_derivatives(const DevSliced* const* D, int P, const double* x, double* y, cudaStream_t st);
 cudaError_t launch_points(const double* v, const double* F, const double* pt, int D, int64_t n, double* out,
@@ -181,33 +181,32 @@ struct sgdg_op : Spare {
     // caller's, two launches for one), and where an element of x is not finite
     // through the whole one after it (k_apply_whole).  Each call leaves its number
     // in a word of its own among kApplyCalls: calls on other streams may still be
-    // in flight.  A captured call, whose number is the same in every replay, has a
-    // word for good, cleared in the graph, and keeps the pruned operator there; with
-    // a budget set, without the operator, or after kApplyCalls of them, it is
-    // captured with the whole one.
+    // in flight.  A captured call, whose number is the same in every replay, has two
+    // words for good (the second for k_apply_whole to clear the first) and keeps the
+    // pruned operator there; with a budget set, without the operator, or after
+    // kApplyCalls of them, it is captured with the whole one.
     static constexpr int64_t kApplyPruned = 3 << 19;
     static constexpr int kApplyCalls = 1024;
-    DevBuf apply_seen;  // the calls' words, then those of captured calls
+    DevBuf apply_seen;  // the calls' words, then the pairs of captured calls
     int apply_call = 0, apply_captured = 0;
     std::set<int> in_graphs;  // `which` of pruned operators that captured calls use
     cudaError_t apply(int which, const double* x, double* y, cudaStream_t st) {
         const DevCSR& A = whole(which);
         if (!prunes(true, kPruneApply) || A.nnz < kApplyPruned) return launch_csr_spmv(A, x, y, st);
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        const cudaError_t e = cudaStreamIsCapturing(st, &cap);
+        const cudaError_t e = st ? cudaStreamIsCapturing(st, &cap) : cudaSuccess;  // (the legacy stream never is)
         if (e != cudaSuccess) return e;
         Use use(*this);
         if (cap != cudaStreamCaptureStatusNone) {
             if (g_budget.load() > 0 || !apply_seen.p || !step_dev.count(which) || apply_captured == kApplyCalls)
                 return launch_csr_spmv(A, x, y, st);
             in_graphs.insert(which);
-            int* seen = apply_seen.as<int>() + kApplyCalls + apply_captured++;
-            const cudaError_t m = cudaMemsetAsync(seen, 0, sizeof(int), st);
-            return m != cudaSuccess ? m : launch_apply(step_dev.at(which)->d, A, x, y, seen, 1, st);
+            int* seen = apply_seen.as<int>() + kApplyCalls + 2 * apply_captured++;
+            return launch_apply(step_dev.at(which)->d, A, x, y, seen, 1, seen + 1, st);
         }
         const DevSliced* P = stepping(which);
         if (P && !apply_seen.p && !build_pruned(which, [&] {
-                DevBuf seen(2 * sizeof(int) * kApplyCalls);
+                DevBuf seen(3 * sizeof(int) * kApplyCalls);
                 CK(cudaMemsetAsync(seen.p, 0, seen.bytes, stream));
                 CK(cudaStreamSynchronize(stream));
                 apply_seen = std::move(seen);
@@ -215,7 +214,7 @@ struct sgdg_op : Spare {
             P = nullptr;
         if (!P) return launch_csr_spmv(A, x, y, st);
         apply_call = apply_call == INT32_MAX ? 1 : apply_call + 1;
-        return launch_apply(*P, A, x, y, apply_seen.as<int>() + apply_call % kApplyCalls, apply_call, st);
+        return launch_apply(*P, A, x, y, apply_seen.as<int>() + apply_call % kApplyCalls, apply_call, nullptr, st);
     }
     // the whole operator, the pruned one making room for it where there is none
     const DevCSR& whole(int which) {

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/sgdg.h"
@@ -122,14 +123,24 @@ class Spare {
     static bool give_back() {
         std::lock_guard<std::mutex> g(mutex());
         bool any = false;
-        for (Spare* s : all())
-            if (s->users_ == 0) any = s->drop_spare() || any;
+        for (Spare* s : all()) {
+            int idle = 0;
+            if (!s->users_.compare_exchange_strong(idle, -1)) continue;
+            any = s->drop_spare() || any;
+            s->users_ = 0;
+        }
         return any;
     }
     struct Use {
         explicit Use(Spare& s) : s_(s) {
-            std::lock_guard<std::mutex> g(mutex());
-            s_.users_++;
+            for (int u = s_.users_.load();;) {  // -1: being freed
+                if (u < 0) {
+                    std::this_thread::yield();
+                    u = s_.users_.load();
+                } else if (s_.users_.compare_exchange_weak(u, u + 1)) {
+                    break;
+                }
+            }
         }
         ~Use() { s_.users_--; }
         Use(const Use&) = delete;
@@ -164,7 +175,7 @@ class Spare {
         static std::vector<Spare*>* a = new std::vector<Spare*>;
         return *a;
     }
-    std::atomic<int> users_{0};
+    std::atomic<int> users_{0};  // -1 while give_back frees it
 };
 
 // Device allocation counted against the HBM budget (sgdg_set_hbm_budget).
