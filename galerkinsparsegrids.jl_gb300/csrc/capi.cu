@@ -61,7 +61,7 @@ void set_error(const std::string& msg) { g_err = msg; }
 using namespace sgdg;
 
 // ------------------------------------------------------------ handles ----
-struct sgdg_op : Spare {
+struct sgdg_op : LiveHandle, Spare {
     SparseIndex ix;
     std::shared_ptr<const DLF1D> dlf;
     int basis = SGDG_BASIS_HIER;  // SGDG_BASIS_POS: the 1D position-basis operators
@@ -257,7 +257,7 @@ struct sgdg_op : Spare {
 // operators (whole_rhs) are built and used when a run meets a value that is not
 // finite, which they spread over more rows, or where the sweeps have no room;
 // once they are there, the sweeps give way to an allocation that needs theirs.
-struct sgdg_vlasov : Spare {
+struct sgdg_vlasov : LiveHandle, Spare {
     int D = 0, P = 0, k = 0, n = 0;
     SparseIndex ix;
     std::shared_ptr<const DLF1D> dlf;
@@ -518,7 +518,7 @@ class StepGraph {
     cudaGraphExec_t exec_ = nullptr;
 };
 
-struct sgdg_batch {
+struct sgdg_batch : LiveHandle {
     MFEngine eng;  // its destructor frees device memory only, never touches a stream
     cudaStream_t own = nullptr;
     ~sgdg_batch() {
@@ -1694,7 +1694,7 @@ int sgdg_set_hbm_budget(int64_t bytes) {
     if (bytes < 0) throw Error(SGDG_EINVAL, "budget must be >= 0");
     g_budget = bytes;
     g_budget_set++;
-    if (bytes > 0) device_pool().trim((size_t)std::max<int64_t>(0, bytes - g_in_use.load()));
+    device_pool().trim(bytes > 0 ? (size_t)std::max<int64_t>(0, bytes - g_in_use.load()) : 0);
     API_END
 }
 

@@ -49,8 +49,9 @@ inline void require_gpu() {
 // ms).  Only a block whose work has finished is recycled (its owner has waited
 // for every stream that used it), so any stream or thread may take it; the others
 // are freed, and cudaFree waits.  At most kPoolBytes are kept; they count against
-// the HBM budget, and are given back where an allocation or the budget needs them
-// and when the library holds nothing else.
+// the HBM budget, and are given back where an allocation or the budget needs them,
+// when the last handle is destroyed (LiveHandle) or nothing else is held, and with
+// every call of sgdg_set_hbm_budget.
 class DevPool {
    public:
     static constexpr size_t kPoolBytes = size_t(1) << 30;
@@ -111,6 +112,24 @@ inline DevPool& device_pool() {
     static DevPool* p = new DevPool;  // outlives the buffers of static objects
     return *p;
 }
+
+// Base of the handles: the blocks kept for reuse go with the last of them (tables
+// kept for the process, of the point evaluation, may still be held then).
+class LiveHandle {
+   protected:
+    LiveHandle() { count()++; }
+    LiveHandle(const LiveHandle&) = delete;
+    LiveHandle& operator=(const LiveHandle&) = delete;
+    ~LiveHandle() {  // the last part of a handle to go: its own blocks are freed
+        if (--count() == 0) device_pool().trim(0);
+    }
+
+   private:
+    static std::atomic<int64_t>& count() {
+        static std::atomic<int64_t> n{0};
+        return n;
+    }
+};
 
 // Device memory that its owner, a handle, can do without (an operator's second,
 // faster form): given back where an allocation or the budget needs the room, so

@@ -254,7 +254,7 @@ class Server {
 
 using namespace sgdg;
 
-struct sgdg_server {
+struct sgdg_server : LiveHandle {
     std::unique_ptr<Server> srv;
     cudaStream_t own = nullptr;
     ~sgdg_server() {

@@ -392,7 +392,10 @@ int sgdg_worklist_dryrun(int nclasses, const int *spec, int pass_only, int chunk
 int sgdg_selftest_convert(const double *x, int64_t n, int64_t *mismatches, int64_t *first);
 
 /* ---- resources ---------------------------------------------------------- */
-/* Upper bound on device bytes the library may hold (0 = no limit). */
+/* Upper bound on device bytes the library may hold (0 = no limit).  Also gives
+ * back device blocks that it keeps between calls for reuse (at most 1 GiB):
+ * all of them for 0, else those beyond the bound.  The rest is given back when
+ * the last handle is destroyed. */
 int sgdg_set_hbm_budget(int64_t bytes);
 int sgdg_hbm_in_use(int64_t *bytes);
 /* Blocks until all library work on the device has finished. */
