@@ -160,13 +160,13 @@ struct Pencils {
     int inner, pad, outer;   // k^min(D,3), the same rounded up to 4, k^(D-3) (1 for D <= 3)
     const int32_t* lmax;     // per pencil: levels along dimension 1
     const int64_t* base;     // first number of its blocks
-    const double* scale;     // product of the scales of its 1D functions (2^(1/2) at level 0, 2^(l/2) at l,
-                             // 2^((lmax)/2) on the pieces), which k_lines puts into the blocks
+    const double* scale;     // product of the scales of its 1D functions (2^(1/2) at level 0 and on the
+                             // pieces, 2^(l/2) at l), which k_lines puts into the blocks
     const int8_t* levels;    // D - 1 levels of the other dimensions, 1-based
     const int64_t* item;     // first item (piece, cell and mode of the others) of k_lines; np + 1
     const int32_t* lev_off;  // per pencil n + 1 offsets of its level blocks
-    const double* two;       // H_0, G_0, H_1, G_1 (k x k each): child b's Legendre coefficients from the
-                             // parent's and its wavelets'
+    const double* two;       // H_0, H_1, then G_0, G_1 of levels 1..n (k x k each): child b's Legendre
+                             // coefficients from the parent's and its wavelets' (two_scale)
     const double* pieces;    // as EvalShape
 };
 
@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(256)
     for (int t = 1; t < lmax; t++) {
         const int64_t ct = t > 1 ? j >> (lmax - t) : 0;
         const double* d = c + off[t] + kD * (ct + (cl << (t > 1 ? t - 1 : 0))) + K * mo;
-        const double* H = S.two + ((j >> (lmax - 1 - t)) & 1) * 2 * K * K;
+        const int b = (j >> (lmax - 1 - t)) & 1;
+        const double *H = S.two + b * K * K, *G = S.two + (2 * t + b) * K * K;
         double w[K], x[K];
 #pragma unroll
         for (int m = 0; m < K; m++) w[m] = d[m];
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(256)
         for (int i = 0; i < K; i++) {
             double v = 0.0;
 #pragma unroll
-            for (int m = 0; m < K; m++) v = fma(__ldg(H + i * K + m), s[m], fma(__ldg(H + K * K + i * K + m), w[m], v));
+            for (int m = 0; m < K; m++) v = fma(__ldg(H + i * K + m), s[m], fma(__ldg(G + i * K + m), w[m], v));
             x[i] = v;
         }
 #pragma unroll
@@ -401,33 +402,52 @@ constexpr int kPencilMaxK = 5;
 // blocks the pencils take 866, 2126, 124 and 100 at 2^18 points).
 constexpr int64_t kPencilPoints = 4096, kPencilTerms = 1 << 20;
 
-// H_b[i][m] = <child b's Legendre function i, the parent's m>, G_b the same with
-// the wavelets: 2^(-1/2) int leg_i(z) p_m((z + s) / 2) dz, s = 2b - 1, over
-// [-1, 1], p_m the parent's polynomial on that half.
-std::vector<double> two_scale(int k) {
-    std::vector<double> out((size_t)4 * k * k);
+// H_b[i][m] = int leg_i(z) p_m((z + s) / 2) dz over [-1, 1], s = 2b - 1, p_m the
+// parent's Legendre function m, and G_b of level t 2^((t - 1) / 2) times the same of
+// the wavelets' polynomials on that half: child b's coefficients without the factor
+// 2^(-1/2) of every level, which is 2^(t/2) times what they stand for.  A line goes
+// through up to n of the H_b; so their diagonal is 1, 1/2, 1/4..., exactly, and
+// the rest is computed in long double and rounded once.  Relative L2 error of the
+// values against long double (blocks; pencils in double with the factors; like
+// this): 1D k=3 n=10 8.1e-16, 1.8e-15, 7.5e-16; 2D k=2 n=8 3.2e-16, 1.0e-15,
+// 3.3e-16; 2D k=4 n=6 1.4e-15, 2.0e-15, 1.1e-15; 3D k=3 n=7 1.15e-15, 1.31e-15,
+// 1.14e-15.  The wavelets are the blocks', rounded as they are.
+std::vector<double> two_scale(int k, int n) {
+    using Real = long double;
+    using Poly = std::vector<Real>;  // monomials in [-1, 1]
+    std::vector<Poly> leg(k, Poly(k, 0));
+    for (int m = 0; m < k; m++) {
+        if (m < 2) leg[m][m] = 1;
+        for (int i = 0; m >= 2 && i < k; i++)
+            leg[m][i] = ((2 * m - 1) * (i > 0 ? leg[m - 1][i - 1] : 0) - (m - 1) * leg[m - 2][i]) / m;
+    }
+    for (int m = 0; m < k; m++)
+        for (Real& c : leg[m]) c *= std::sqrt(Real(2 * m + 1) / 2);
+    std::vector<double> out((size_t)2 * (n + 1) * k * k);
     for (int b = 0; b < 2; b++)
         for (int g = 0; g < 2; g++)
             for (int m = 0; m < k; m++) {
-                const HierFn f = make_hier_fn(k, g, 1, m + 1);
-                const double* p = g && b ? f.right : f.left;
-                std::vector<double> q(k, 0.0);  // p((z + s) / 2) in z, by Horner
+                const HierFn f = make_hier_fn(k, 1, 1, m + 1);
+                const Poly wav(b ? f.right : f.left, (b ? f.right : f.left) + k);
+                const Poly& p = g ? wav : leg[m];
+                Poly q(k, 0);  // p((z + s) / 2) in z, by Horner
                 for (int i = k - 1; i >= 0; i--) {
-                    std::vector<double> t(k, 0.0);
+                    Poly t(k, 0);
                     for (int a = 0; a < k; a++) {
-                        t[a] += 0.5 * (2 * b - 1) * q[a];
-                        if (a + 1 < k) t[a + 1] += 0.5 * q[a];
+                        t[a] += Real(2 * b - 1) / 2 * q[a];
+                        if (a + 1 < k) t[a + 1] += q[a] / 2;
                     }
                     t[0] += p[i];
                     q = t;
                 }
                 for (int i = 0; i < k; i++) {
-                    const HierFn l = make_hier_fn(k, 0, 1, i + 1);
-                    double v = 0.0;
+                    Real v = 0;
                     for (int a = 0; a < k; a++)
                         for (int c = 0; c < k; c++)
-                            if ((a + c) % 2 == 0) v += l.left[a] * q[c] * 2.0 / (a + c + 1);
-                    out[(size_t)(2 * b + g) * k * k + i * k + m] = std::sqrt(0.5) * v;
+                            if ((a + c) % 2 == 0) v += leg[i][a] * q[c] * 2 / (a + c + 1);
+                    if (g == 0) out[(size_t)b * k * k + i * k + m] = (double)v;
+                    for (int t = 1; g == 1 && t <= n; t++)
+                        out[(size_t)(2 * t + b) * k * k + i * k + m] = (double)(std::sqrt(std::ldexp(Real(1), t - 1)) * v);
                 }
             }
     return out;
@@ -463,7 +483,7 @@ void build_pencils(EvalTables& T) {
             off.push_back((int32_t)ix.lev_off[ix.lookup_level(L)]);
             lm = l;
         }
-        int half = lm;  // log2 of the square of the scale
+        int half = 1;  // log2 of the square of the scale
         for (int d = 1; d < D; d++) {
             lev.push_back((int8_t)Lb[d]);
             half += std::max(1, Lb[d] - 1);
@@ -481,7 +501,7 @@ void build_pencils(EvalTables& T) {
     T.plevels = upload(lev, nullptr);
     T.item = upload(item, nullptr);
     T.plev_off = upload(off, nullptr);
-    T.two = upload(two_scale(k), nullptr);
+    T.two = upload(two_scale(k, n), nullptr);
     CK(cudaStreamSynchronize(nullptr));
     P.lmax = T.lmax.as<int32_t>();
     P.base = T.base.as<int64_t>();
