@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "sgdg_core.h"
 
@@ -278,35 +279,41 @@ LineTables line_tables(const DLF1D& op, int levels, bool square, bool prune) {
         // row's entries ascending, each times the entries of that row)
         marker.assign(m, -1);
         acc.assign(m, 0.0);
-        mag.assign(m, 0.0);
-        const int64_t base = (int64_t)T.col.size();
-        T.rowptr.push_back(base);
-        for (int r = 0; r < m; r++) {
-            cols.clear();
-            for (int64_t p = lp[r]; p < lp[r + 1]; p++) {
-                const int32_t j = lc[p];
-                const double a = lv[p];
-                for (int64_t q = lp[j]; q < lp[j + 1]; q++) {
-                    const int32_t c = lc[q];
-                    if (marker[c] != r) {
-                        marker[c] = r;
-                        acc[c] = a * lv[q];
-                        mag[c] = std::fabs(a * lv[q]);
-                        cols.push_back(c);
-                    } else {
-                        acc[c] += a * lv[q];
-                        mag[c] += std::fabs(a * lv[q]);
+        if (prune) mag.assign(m, 0.0);
+        T.rowptr.push_back((int64_t)T.col.size());
+        auto rows = [&](auto pruned) {
+            for (int r = 0; r < m; r++) {
+                cols.clear();
+                for (int64_t p = lp[r]; p < lp[r + 1]; p++) {
+                    const int32_t j = lc[p];
+                    const double a = lv[p];
+                    for (int64_t q = lp[j]; q < lp[j + 1]; q++) {
+                        const int32_t c = lc[q];
+                        const double t = a * lv[q];
+                        if (marker[c] != r) {
+                            marker[c] = r;
+                            acc[c] = t;
+                            if (pruned) mag[c] = std::fabs(t);
+                            cols.push_back(c);
+                        } else {
+                            acc[c] += t;
+                            if (pruned) mag[c] += std::fabs(t);
+                        }
                     }
                 }
+                std::sort(cols.begin(), cols.end());
+                for (int32_t c : cols) {
+                    if (pruned && !(std::fabs(acc[c]) > kPruneRel * mag[c])) continue;
+                    T.col.push_back(c);
+                    T.val.push_back(acc[c]);
+                }
+                T.rowptr.push_back((int64_t)T.col.size());
             }
-            std::sort(cols.begin(), cols.end());
-            for (int32_t c : cols) {
-                if (prune && !(std::fabs(acc[c]) > kPruneRel * mag[c])) continue;
-                T.col.push_back(c);
-                T.val.push_back(acc[c]);
-            }
-            T.rowptr.push_back((int64_t)T.col.size());
-        }
+        };
+        if (prune)
+            rows(std::true_type{});
+        else
+            rows(std::false_type{});
     }
     return T;
 }
