@@ -412,7 +412,8 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
 }
 
 // NV adjacent vectors of an interleaved set (element i of vector j at
-// y[i * stride + j]); a result that is not finite raises *nonfinite
+// y[i * stride + j]); for one vector a result that is not finite raises *nonfinite
+// (the sweeps of several are followed by one that checks)
 template <int NV>
 struct SweepOut {
     static constexpr bool kTogether = false;
@@ -423,7 +424,7 @@ struct SweepOut {
     __device__ __forceinline__ void fetch(int64_t, int, Fetched&) const {}
     __device__ __forceinline__ void one(int64_t row, int j, double s, const Fetched&) const {
         y[row * stride + j] = s;
-        if (nonfinite && not_finite(s)) *nonfinite = 1;
+        if (NV == 1 && nonfinite && not_finite(s)) *nonfinite = 1;
     }
     __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], const Fetched& f) const {
         double* p = y + row * stride;
@@ -458,7 +459,7 @@ __device__ __forceinline__ double point_product(const double* __restrict__ v, co
 // that short ones fill its end (8 steps of Vlasov 2x2v k=2 n=8 4885 -> 4511 us,
 // k=3 n=6 4288 -> 4112); a smaller one starts them all at once and is faster in
 // ascending order (k=2 n=7 2529 and 2343 us, n=6 1459 and 1279).
-constexpr unsigned kSweepResident = 152 * (768 / kSliceThreads);  // SMs; threads at 80 registers
+constexpr unsigned kSweepResident = kSMs * (768 / kSliceThreads);  // threads at 80 registers
 __device__ __forceinline__ int sweep_block(int n) {
     return gridDim.x * gridDim.y > kSweepResident ? n - 1 - (int)blockIdx.x : (int)blockIdx.x;
 }
@@ -717,9 +718,10 @@ cudaError_t launch_plain_interleave(int64_t len, int nv, int64_t nb, const doubl
     return cudaGetLastError();
 }
 
-// y = T x for P interleaved vectors (P = 1, or even)
+// y = T x for P interleaved vectors (P = 1, or even; nonfinite for P = 1 only)
 cudaError_t launch_sweep(const DevSliced& A, int P, const double* x, double* y, int* nonfinite, cudaStream_t st) {
     const unsigned nb = (unsigned)A.bin_block[kCsrBins];
+    if (P > 1 && nonfinite) return cudaErrorInvalidValue;
     if (nb == 0) return cudaSuccess;
     if (P % 4 == 0)
         launch_dependent(k_sweep<4>, dim3(nb, P / 4), kSliceThreads, st, A, x, y, P, nonfinite);
@@ -735,7 +737,7 @@ cudaError_t launch_apply(const DevSliced& P, const DevCSR& A, const double* x, d
                          cudaStream_t st) {
     if (P.bin_block[kCsrBins] == 0) return cudaSuccess;
     launch_dependent(k_apply, (unsigned)P.bin_block[kCsrBins], kSliceThreads, st, P, x, y, seen, call);
-    launch_dependent(k_apply_whole, 152u, 256, st, A, x, y, seen, call, left);
+    launch_dependent(k_apply_whole, (unsigned)kSMs, 256, st, A, x, y, seen, call, left);
     return cudaGetLastError();
 }
 

@@ -35,6 +35,8 @@ struct DevCSR {
     double* partial;          // kCsrMaxVec * nseg: segment sums, one block of nseg per vector
 };
 
+constexpr int kSMs = 152;  // of a GB300, for rules that are also evaluated without one
+
 // The stepping operators (csr_step.cu) in slices: a warp's 32 / 2^b rows of bin
 // b, the rows of a bin sorted by length, with slot u of lane l of slice s at
 // (base[s] + u) 32 + l: entry u 2^b + l % 2^b of row rows[s 32 + l].  A warp

@@ -43,7 +43,7 @@ static constexpr size_t kWaveLag = 3;       // steps between a group's consecuti
 // requests 7.9 and 8.7).  CTAs it reckons with: all that are resident on a GB300 (a
 // list is also built where there is no GPU to ask).
 constexpr double kListBytes = 96e6, kListWork = 4e6, kListItems = 300;
-constexpr int kListCtas = 456;
+constexpr int kListCtas = 3 * kSMs;
 static constexpr int kStageKey = 1 << 22;   // counter keys of a whole-step list: key + (stage - 1) * kStageKey
 
 // The wave's D_d D_d on a pencil of line length lmax: one sweep of the
