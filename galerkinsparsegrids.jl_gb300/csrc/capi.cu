@@ -971,6 +971,7 @@ static void plain_batch_steps(sgdg_op* op, int which, int64_t nsolves, double* y
     CK(cudaMemcpyAsync(keep.p, y, keep.bytes, cudaMemcpyDeviceToDevice, cs));
     const std::vector<int> bad = work->run(*A, nsolves, y, dt, nsteps, cs);
     work->recycle();
+    if (std::find(bad.begin(), bad.end(), 1) == bad.end()) return keep.recycle();
     const int64_t len = A->m;
     auto restore = [&](int64_t first, int64_t n) {
         CK(cudaMemcpyAsync(y + first * len, keep.as<double>() + first * len, sizeof(double) * (size_t)(n * len),

@@ -304,6 +304,7 @@ struct RkOut {
     double* y;
     int64_t m;
     int nv;
+    int first;  // flag of solve 0
     __device__ __forceinline__ void load(int64_t row, int j, Fetched& f) const {
         f.y = y[row + j * m];
         f.acc = rk.stage != 1 ? rk.acc[row * NV + j] : 0.0;
@@ -314,7 +315,7 @@ struct RkOut {
     __device__ __forceinline__ void one(int64_t row, int j, double s, Fetched& f) const {
         if (j >= nv) return;
         if constexpr (NV > 1) load(row, j, f);
-        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j, NV == 1 ? 0 : j);
+        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j, NV == 1 ? 0 : first + j);
     }
     __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], Fetched& f) const {
 #pragma unroll
@@ -354,9 +355,8 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
         y += o;
         rk.acc += o;
         rk.uout += o;
-        if (NV > 1 && rk.nonfinite) rk.nonfinite += g * NV;  // (one solve at a time for NV = 1)
     }
-    block_rows<NV>(A, rb, x, NV, RkOut<NV>{rk, y, A.m, g + 1 == q.count ? q.last : NV});
+    block_rows<NV>(A, rb, x, NV, RkOut<NV>{rk, y, A.m, g + 1 == q.count ? q.last : NV, (int)g * NV});
 }
 
 // One warp per segment of a long row, the sums in row_sum's order.  Segments are all
