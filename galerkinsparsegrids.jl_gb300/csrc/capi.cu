@@ -181,14 +181,15 @@ struct sgdg_op : LiveHandle, Spare {
     // pruned one (us per application, whole and pruned: Laplacian 2D k=3 n=7, 1.3
     // M entries, 8.3 and 8.9; 4D k=2 n=6, 1.6 M, 10.3 and 8.9; 3D k=3 n=6, 2.2 M,
     // 11.5 and 9.1; 3D k=3 n=7, 8.8 M, 28.3 and 9.0; below 9 the time is the
-    // caller's, two launches for one; building both takes the first application 14.7
-    // ms instead of 10.0 for the last of them, 5.7 instead of 3.4 for the 4D one), and where an element of x is not finite
-    // through the whole one after it (k_apply_whole).  Each call leaves its number
-    // in a word of its own among kApplyCalls: calls on other streams may still be
-    // in flight.  A captured call, whose number is the same in every replay, has two
-    // words for good (the second for k_apply_whole to clear the first) and keeps the
-    // pruned operator there; with a budget set, without the operator, or after
-    // kApplyCalls of them, it is captured with the whole one.
+    // caller's, two launches for one; building both takes the first application
+    // 14.7 ms instead of 10.0 for the last of them, 5.7 instead of 3.4 for the 4D
+    // one), and where an element of x is not finite through the whole one after it
+    // (k_apply_whole).  Each call leaves its number in a word of its own among
+    // kApplyCalls: calls on other streams may still be in flight.  A captured call,
+    // whose number is the same in every replay, has two words for good (the second
+    // for k_apply_whole to clear the first) and keeps the pruned operator there; with
+    // a budget set, without the operator, or after kApplyCalls of them, it is
+    // captured with the whole one.
     static constexpr int64_t kApplyPruned = 3 << 19;
     static constexpr int kApplyCalls = 1024;
     DevBuf apply_seen;  // the calls' words, then the pairs of captured calls
