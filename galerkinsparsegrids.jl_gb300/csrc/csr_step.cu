@@ -51,7 +51,7 @@ struct CsrRK {  // stage update of the RK4 epilogue: k = A uin, then rk_stage
     double dt, hdt, dt6;
     int stage;
     int write_u;     // stage 4 also stores the new state to uout (the next step's input when it is not y)
-    int* nonfinite;  // one per solve: set to 1 when a stage result of its is not finite (may be null)
+    int* nonfinite;  // one per solve: set to 1 when a stage result of its is not finite (not read with FLAGS = false)
 };
 
 // Programmatic dependent launch: waits until the launches this one depends on
@@ -146,6 +146,7 @@ __device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x)
 // RK4 stage update of one element: k its right-hand side, yy its state and aa its
 // accumulator (from y and acc[o]), which go back there and uout[o]; its solve's flag
 // is rk.nonfinite[j]
+template <bool FLAGS>
 __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double yy, double aa, double* y, int64_t o,
                                               int j) {
     double un;
@@ -155,7 +156,7 @@ __device__ __forceinline__ void csr_rk_update(const CsrRK& rk, double k, double 
     else
         rk.acc[o] = aa;
     if (rk.stage != 4 || rk.write_u) rk.uout[o] = un;
-    if (rk.nonfinite && not_finite(un)) rk.nonfinite[j] = 1;
+    if (FLAGS && not_finite(un)) rk.nonfinite[j] = 1;
 }
 
 // Block rb's rows, 2^bin lanes each: out.one(row, j, sum) by the lane that
@@ -294,7 +295,8 @@ __device__ __forceinline__ void block_rows(const DevCSR& A, int64_t rb, const do
 // One solve, whose time is latency, fetches its state and accumulator before the
 // sum (3D wave k=3 n=7 38.1 -> 35.8 us per step); sets, bound by the FP64 pipe,
 // after it (256 of them 4.49 ms, 4.59 with the registers held across the sum).
-template <int NV>
+// FLAGS: a result that is not finite raises its solve's flag.
+template <int NV, bool FLAGS>
 struct RkOut {
     static constexpr bool kTogether = false;
     struct Fetched {
@@ -315,7 +317,7 @@ struct RkOut {
     __device__ __forceinline__ void one(int64_t row, int j, double s, Fetched& f) const {
         if (j >= nv) return;
         if constexpr (NV > 1) load(row, j, f);
-        csr_rk_update(rk, s, f.y, f.acc, y + row + j * m, row * NV + j, NV == 1 ? 0 : first + j);
+        csr_rk_update<FLAGS>(rk, s, f.y, f.acc, y + row + j * m, row * NV + j, NV == 1 ? 0 : first + j);
     }
     __device__ __forceinline__ void all(int64_t row, const double (&s)[NV], Fetched& f) const {
 #pragma unroll
@@ -334,6 +336,10 @@ struct CsrSets {
     int group;
     int last;  // solves of the last set
 };
+
+// Only a pruned operator's steps are repeated where a value is not finite.
+template <class Mat>
+constexpr bool kFlags = std::is_same_v<Mat, DevSliced>;
 
 template <int NV, class Mat>
 __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
@@ -356,7 +362,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
         rk.acc += o;
         rk.uout += o;
     }
-    block_rows<NV>(A, rb, x, NV, RkOut<NV>{rk, y, A.m, g + 1 == q.count ? q.last : NV, (int)g * NV});
+    block_rows<NV>(A, rb, x, NV, RkOut<NV, kFlags<Mat>>{rk, y, A.m, g + 1 == q.count ? q.last : NV, (int)g * NV});
 }
 
 // One warp per segment of a long row, the sums in row_sum's order.  Segments are all
@@ -408,7 +414,7 @@ __global__ void k_rk_long_rows(DevCSR A, double* y, CsrRK rk) {
     for (int q = A.long_seg[i]; q < A.long_seg[i + 1]; q++) s += A.partial[q];
     const int64_t row = A.long_row[i];
     if (!SGDG_IN(row, A.m)) return;
-    csr_rk_update(rk, s, y[row], rk.stage == 1 ? 0.0 : rk.acc[row], y + row, row, 0);
+    csr_rk_update<false>(rk, s, y[row], rk.stage == 1 ? 0.0 : rk.acc[row], y + row, row, 0);
 }
 
 // NV adjacent vectors of an interleaved set (element i of vector j at
@@ -609,6 +615,7 @@ constexpr int block_threads = std::is_same_v<Mat, DevSliced> ? kSliceThreads : 2
 
 template <class Mat>
 static cudaError_t rk4_one(const Mat& A, const double* uin, double* y, const CsrRK& rk, cudaStream_t st) {
+    if (kFlags<Mat> && !rk.nonfinite) return cudaErrorInvalidValue;
     if (A.bin_block[kCsrBins] > 0)
         launch_dependent(k_csr_rk<1, Mat>, A.bin_block[kCsrBins], block_threads<Mat>, st, A, uin, y, rk, CsrSets{1, 1, 1});
     if constexpr (std::is_same_v<Mat, DevCSR>)
@@ -668,12 +675,13 @@ static void rk4_sets(const Mat& A, int64_t nb, double* y, double* acc, double* u
 // a row together: the stage inputs and accumulators are interleaved, so a
 // matrix entry is loaded once per set and meets a column's values in one
 // load.  nv is plain_set_size or 1; acc, u0 and u1 hold whole sets of A.m
-// numbers a solve, nonfinite (or null) one flag a solve, and with nv > 1 u0 holds the interleaved states on entry
-// (launch_plain_interleave) and on return.
+// numbers a solve, nonfinite one flag a solve (null with a whole operator), and with
+// nv > 1 u0 holds the interleaved states on entry (launch_plain_interleave) and on
+// return.
 template <class Mat>
 static cudaError_t plain_steps(const Mat& A, int nv, int64_t nb, double* y, double* acc, double* u0, double* u1,
                                double dt, int64_t nsteps, int* nonfinite, cudaStream_t st) {
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = kFlags<Mat> && !nonfinite ? cudaErrorInvalidValue : cudaSuccess;
     for (int64_t i = 0; i < nsteps && e == cudaSuccess; i++) {
         for (int stage = 1; stage <= 4 && e == cudaSuccess; stage++) {
             if (nv == 1) {
