@@ -365,12 +365,20 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 3)
     block_rows<NV>(A, rb, x, NV, RkOut<NV, kFlags<Mat>>{rk, y, A.m, g + 1 == q.count ? q.last : NV, (int)g * NV});
 }
 
-// One warp per segment of a long row, the sums in row_sum's order.  Segments are all
-// of one length, so the entries go in plain groups of four: 32 registers and 77 % of
-// the warps active keep the FP64 pipe 86 % busy (DRAM 64 %), where row_sum's next
-// entries, fetched ahead, cost registers and predicated additions (us for 20 steps of
-// the wave, row_sum and this: 1D k=8 n=9 4075 and 3496, 1D k=3 n=12 24480 and 23505).
+// One warp per segment of a long row, the sums in row_sum's order, in plain groups:
+// segments are of one length but for the rows' last ones, and row_sum's predicated
+// additions would take their turn on the FP64 pipe.  Groups of four, no look-ahead:
+// 32 registers and 77 % of the warps active keep that pipe 86 % busy (DRAM 64 %).
+// FEW: segments that are all resident at once are bound by their chain of loads
+// (entries, gather, sum), so eight are on their way and the next eight fetched
+// beside them.  us for 40 steps of the wave, row_sum, groups of four and FEW, with
+// the segments: 2D k=3 n=9 12456, 13264, 11803 (54); 2D k=2 n=10 12768, 13898, 12060
+// (4,560); 1D k=8 n=9 8053, 6954, 7548 (8,192); 2D k=4 n=9 5242, 4952, 5079 (32,736;
+// 3 steps of 3).
+constexpr int64_t kFewSegments = int64_t(kSMs) * 32;  // warps resident at FEW's 64 registers
+template <bool FEW>
 __global__ void __launch_bounds__(256) k_rk_segments(DevCSR A, const double* x) {
+    constexpr int G = FEW ? 8 : 4;
     const int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     int64_t p = 0, e = 0;
@@ -378,28 +386,47 @@ __global__ void __launch_bounds__(256) k_rk_segments(DevCSR A, const double* x) 
         p = __ldg(A.seg_begin + seg) + lane;
         e = __ldg(A.seg_end + seg);
     }
-    pdl_wait();
     auto entry = [&](int64_t at, int& c, double& v) {
         c = __ldg(A.col + at);
         v = __ldg(A.val + at);
         if (!SGDG_IN(c, A.m)) c = 0;
     };
-    double s[1] = {0.0};
-    for (; p + 96 < e; p += 128) {
-        int c[4];
-        double v[4], xv[4];
+    int c[G];
+    double v[G], s[1] = {0.0};
+    auto group = [&](int (&gc)[G], double (&gv)[G]) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) entry(p + 32 * u, c[u], v[u]);
+        for (int u = 0; u < G; u++) entry(p + 32 * u, gc[u], gv[u]);
+    };
+    bool more = p + 32 * (G - 1) < e;
+    if (more) group(c, v);
+    pdl_wait();
+    while (more) {
+        double xv[G];
 #pragma unroll
-        for (int u = 0; u < 4; u++) xv[u] = __ldca(x + c[u]);
+        for (int u = 0; u < G; u++) xv[u] = __ldca(x + c[u]);
+        p += 32 * G;
+        more = p + 32 * (G - 1) < e;
+        int nc[G];
+        double nv[G];
+        if (FEW && more) group(nc, nv);
 #pragma unroll
-        for (int u = 0; u < 4; u++) s[0] = fma(v[u], xv[u], s[0]);
+        for (int u = 0; u < G; u++) s[0] = fma(v[u], xv[u], s[0]);
+        if (!more) break;
+        if constexpr (FEW) {
+#pragma unroll
+            for (int u = 0; u < G; u++) {
+                c[u] = nc[u];
+                v[u] = nv[u];
+            }
+        } else {
+            group(c, v);
+        }
     }
     for (; p < e; p += 32) {
-        int c;
-        double v;
-        entry(p, c, v);
-        s[0] = fma(v, __ldca(x + c), s[0]);
+        int tc;
+        double tv;
+        entry(p, tc, tv);
+        s[0] = fma(tv, __ldca(x + tc), s[0]);
     }
     csr_reduce<32, 1>(s, lane);
     if (seg < A.nseg && lane == 0) A.partial[seg] = s[0];
@@ -620,7 +647,8 @@ static cudaError_t rk4_one(const Mat& A, const double* uin, double* y, const Csr
         launch_dependent(k_csr_rk<1, Mat>, A.bin_block[kCsrBins], block_threads<Mat>, st, A, uin, y, rk, CsrSets{1, 1, 1});
     if constexpr (std::is_same_v<Mat, DevCSR>)
         if (A.nlong > 0) {
-            launch_dependent(k_rk_segments, grid_for(A.nseg * 32), 256, st, A, uin);
+            launch_dependent(A.nseg <= kFewSegments ? k_rk_segments<true> : k_rk_segments<false>, grid_for(A.nseg * 32), 256, st,
+                             A, uin);
             launch_dependent(k_rk_long_rows, grid_for(A.nlong), 256, st, A, y, rk);
         }
     return cudaGetLastError();
